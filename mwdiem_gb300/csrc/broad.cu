@@ -29,6 +29,7 @@ namespace {
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+constexpr int64_t SCAN_RAW_MAX = 32 * SCAN_TILE;
 
 __device__ __forceinline__ int block_exclusive_scan(int v, int* sh, int* total)
 {
@@ -74,65 +75,18 @@ __global__ void scan_reduce_kernel(const int32_t* in, int64_t n, int32_t* block_
     if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
 }
 
-// out[i] = sum(in[0..i)), out[n] = total; in and out may alias.  Each block adds up the tile totals
-// of the blocks before it (at most a few thousand values), so no separate pass scans the totals.
-// exclusive scan of up to SCAN_SMALL_MAX elements by one block (one launch instead of two)
-constexpr int SCAN_SMALL_THREADS = 1024;
-constexpr int64_t SCAN_SMALL_MAX = 64 * SCAN_SMALL_THREADS;
-__global__ void __launch_bounds__(SCAN_SMALL_THREADS) scan_small_kernel(const int32_t* in, int64_t n, int32_t* out,
-                                                                        int64_t* total_out, int64_t cap,
-                                                                        uint32_t* status, uint32_t overflow_bit)
-{
-    pdl_wait();
-    pdl_launch_dependents();
-    __shared__ int sh[SCAN_SMALL_THREADS / 32];
-    const int per = (int)((n + SCAN_SMALL_THREADS - 1) / SCAN_SMALL_THREADS);
-    const int64_t base = (int64_t)threadIdx.x * per;
-    int sum = 0;
-    for (int k = 0; k < per; ++k)
-        if (base + k < n) sum += in[base + k];
-    // block scan of the per-thread sums (SCAN_SMALL_THREADS / 32 warps)
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int x = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) sh[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-        int w = sh[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        sh[lane] = w;
-    }
-    __syncthreads();
-    int ex = (wid ? sh[wid - 1] : 0) + x - sum;
-    for (int k = 0; k < per; ++k) {
-        if (base + k >= n) break;
-        const int v = in[base + k];
-        out[base + k] = ex;
-        ex += v;
-    }
-    if (threadIdx.x == 0) {
-        const int64_t t = sh[SCAN_SMALL_THREADS / 32 - 1];
-        out[n] = (int32_t)t;
-        if (total_out) *total_out = t < cap ? t : cap;
-        if (t > cap) set_status(status, overflow_bit);
-    }
-}
+// What scan_final_kernel scans, and where it finds what precedes a tile
+constexpr int SCAN_SUMS = 0;   // values; the tiles' totals are in block_sums
+constexpr int SCAN_WORDS = 1;  // the set bits of a bitmap (v = popc(word)), totals in block_sums; each word is
+                               // also copied to words_copy and zeroed in place (the next broad phase rebuilds it)
+constexpr int SCAN_RAW = 2;    // values; each block adds up all the values before its tile itself
 
-// The final pass of the scan: block b writes the exclusive prefix of its tile, offset by the totals of
-// tiles 0..b-1.  The tile's values are loaded first (two int4 per thread when vec: both arrays 16-byte
-// aligned), so that their latency overlaps the loads of the earlier tiles' totals, and one block pass
-// (a single barrier) both scans the thread sums and adds up those totals.
-// WORDS: the input is a bitmap whose set bits are counted (v = popc(word)); each word is also copied to
-// words_copy and zeroed in place (the bitmap is rebuilt by the next broad phase).
-template <bool WORDS>
+// The final pass of the scan: block b writes the exclusive prefix of its tile, offset by the sum of
+// tiles 0..b-1 (out[n] = total; in and out may alias, except with SCAN_RAW).  The tile's values are
+// loaded first (two int4 per thread when vec: both arrays 16-byte aligned), so that their latency
+// overlaps the loads of what precedes them, and one block pass (a single barrier) both scans the thread
+// sums and adds up the preceding ones.
+template <int MODE>
 __global__ void scan_final_kernel(const int32_t* in, int64_t n, const int32_t* block_sums, int32_t* out, int nb,
                                   int64_t* total_out, int64_t cap, uint32_t* status, uint32_t overflow_bit, int vec,
                                   int32_t* words_copy)
@@ -140,6 +94,7 @@ __global__ void scan_final_kernel(const int32_t* in, int64_t n, const int32_t* b
     static_assert(SCAN_ITEMS == 8, "two int4 per thread");
     pdl_wait();
     pdl_launch_dependents();
+    constexpr bool WORDS = MODE == SCAN_WORDS;
     constexpr int W = SCAN_THREADS / 32;
     __shared__ int sh_x[W], sh_p[W];
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
@@ -171,17 +126,32 @@ __global__ void scan_final_kernel(const int32_t* in, int64_t n, const int32_t* b
 #pragma unroll
         for (int k = 0; k < SCAN_ITEMS; ++k) v[k] = __popc((unsigned)v[k]);
     }
-    // the totals of the tiles before this one, eight independent loads in flight per thread (a
-    // 15M-cell table has 7,300 tiles); integer sums, so the order does not matter
+    // the totals of the tiles before this one (a 15M-cell table has 7,300 tiles), or all the values
+    // before it, four at a time; eight independent loads in flight per thread; integer sums, so the
+    // order does not matter
     constexpr int U = 8;
-    const int lim = (int)blockIdx.x;
     int acc[U] = {};
     int i = threadIdx.x;
-    for (; i + (U - 1) * SCAN_THREADS < lim; i += U * SCAN_THREADS) {
+    if (MODE == SCAN_RAW) {
+        const int lim = (int)blockIdx.x * (SCAN_TILE / 4);
+        const int4* q = reinterpret_cast<const int4*>(in);
+        for (; i < lim; i += U * SCAN_THREADS) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) acc[u] += block_sums[i + u * SCAN_THREADS];
+            for (int u = 0; u < U; ++u) {
+                const int j = i + u * SCAN_THREADS;
+                if (j >= lim) break;
+                const int4 x = vec ? q[j] : make_int4(in[4 * j], in[4 * j + 1], in[4 * j + 2], in[4 * j + 3]);
+                acc[u] += (x.x + x.y) + (x.z + x.w);
+            }
+        }
+    } else {
+        const int lim = (int)blockIdx.x;
+        for (; i + (U - 1) * SCAN_THREADS < lim; i += U * SCAN_THREADS) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) acc[u] += block_sums[i + u * SCAN_THREADS];
+        }
+        for (; i < lim; i += SCAN_THREADS) acc[0] += block_sums[i];
     }
-    for (; i < lim; i += SCAN_THREADS) acc[0] += block_sums[i];
     int part = 0;
 #pragma unroll
     for (int u = 0; u < U; ++u) part += acc[u];
@@ -327,11 +297,77 @@ __device__ __forceinline__ bool pyset_pair_lo_first(int lo, int hi, int base)
     return ia < i;
 }
 
-// cells up to SMALL_CELL members are ordered by one thread with the table in local memory; larger
-// cells go to a list handled by one warp each with the table in shared memory
-constexpr int SMALL_CELL = 32;
-constexpr int SMALL_TAB = 128;   // table size CPython reaches for <= 32 members
-constexpr int BIG_TAB = 512;     // ... for <= 306 members
+// The same order for a cell of 5 to 18 members by one warp, without a table in memory: which slots are
+// taken is a bit mask in a register (the table has 8 slots for the first five entries, 32 up to the
+// 18th), and a member's place in the listing is the number of taken slots below its own.  32-bit
+// arithmetic suffices: the hash has 32 bits and only the bits under the mask count.
+
+// the slot of hash h in the 8-slot table (no slot index admits linear probes)
+__device__ __forceinline__ unsigned pyset_slot8(unsigned occ, unsigned h)
+{
+    unsigned i = h & 7u, perturb = h;
+    while ((occ >> i) & 1u) {
+        perturb >>= 5;
+        i = (i * 5u + 1u + perturb) & 7u;
+    }
+    return i;
+}
+
+// the slot of hash h in the 32-slot table: the first free one of i .. i + 9 (of i alone where those
+// would pass the end), else the next probe
+__device__ __forceinline__ unsigned pyset_slot32(unsigned occ, unsigned h)
+{
+    unsigned i = h & 31u, perturb = h;
+    for (;;) {
+        const unsigned open = ~(occ >> i) & (i + 9u <= 31u ? 0x3ffu : 1u);
+        if (open) return i + (unsigned)__ffs(open) - 1u;
+        perturb >>= 5;
+        i = (i * 5u + 1u + perturb) & 31u;
+    }
+}
+
+// The place in the listing of the calling lane's member, for the k members (5 to 18) that lanes 0..k-1
+// of a full warp hold; rank: the member's place among the ids (-1 for the other lanes), h: its hash.
+// Only the occupancy mask is a serial chain; the exchanges between lanes are off it.
+__device__ __forceinline__ int pyset_warp_place(int k, int rank, unsigned h)
+{
+    const int lane = threadIdx.x & 31;
+    unsigned hs = 0;  // lane e: hash of the member of rank e
+    for (int e = 0; e < k; ++e) {
+        const unsigned x = __shfl_sync(0xffffffffu, h, __ffs(__ballot_sync(0xffffffffu, rank == e)) - 1);
+        if (lane == e) hs = x;
+    }
+    unsigned occ = 0, slot = 0;
+#pragma unroll
+    for (int e = 0; e < 5; ++e) {
+        const unsigned s = pyset_slot8(occ, __shfl_sync(0xffffffffu, hs, e));
+        occ |= 1u << s;
+        if (lane == e) slot = s;
+    }
+    // the fifth entry grows the table to 32 slots; the five move in the order of their slots
+    const int old = lane < 5 ? __popc(occ & ((1u << slot) - 1u)) : -1;
+    occ = 0;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        const int src = __ffs(__ballot_sync(0xffffffffu, old == q)) - 1;
+        const unsigned s = pyset_slot32(occ, __shfl_sync(0xffffffffu, hs, src));
+        occ |= 1u << s;
+        if (lane == src) slot = s;
+    }
+    for (int e = 5; e < k; ++e) {
+        const unsigned s = pyset_slot32(occ, __shfl_sync(0xffffffffu, hs, e));
+        occ |= 1u << s;
+        if (lane == e) slot = s;
+    }
+    const int listed = __popc(occ & ((1u << slot) - 1u));
+    return __shfl_sync(0xffffffffu, listed, rank < 0 ? 0 : rank);
+}
+
+// cells of up to 4 members are ordered by one thread, up to 18 by a warp of its block; larger cells go to a list
+// handled by one warp each with the table in shared memory
+constexpr int SMALL_CELL = 4;
+constexpr int WARP_CELL = 18;
+constexpr int BIG_TAB = 512;     // table size CPython reaches for <= 306 members
 constexpr int BIG_CELL = 306;
 
 // ---------------------------------------------------------------- broad-phase kernels
@@ -433,6 +469,7 @@ __global__ void assign_kernel(BroadArgs a)
     }
     const int r = a.row_lo + blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= a.row_hi) return;
+    if (!a.append && r - a.row_lo <= (a.row_hi - a.row_lo) / SCAN_TILE) a.scan_tmp[r - a.row_lo] = 0;  // pairs_kernel
     if (is_wall(a, r) || inactive(a, r)) {  // walls and rows waiting at an inlet have no cell
         a.cell_of[r] = -1;
         return;
@@ -457,12 +494,10 @@ __global__ void assign_kernel(BroadArgs a)
         return;
     }
     atomicAdd(a.cell_count + g, 1);
-    if (a.tile_sums) {
-        // one atomic per tile per warp (consecutive rows mostly share a tile)
-        const int tile = g / SCAN_TILE;
-        const unsigned peers = __match_any_sync(__activemask(), tile);
-        if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(a.tile_sums + tile, __popc(peers));
-    }
+    // one atomic per tile per warp (consecutive rows mostly share a tile)
+    const int tile = g / SCAN_TILE;
+    const unsigned peers = __match_any_sync(__activemask(), tile);
+    if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(a.tile_sums + tile, __popc(peers));
 }
 
 // sparse table: rows per occupied cell (by rank), with per-tile totals for the scan that follows
@@ -496,26 +531,78 @@ __device__ __forceinline__ void place(const BroadArgs& a, int i, int v, int g)
     }
 }
 
-// members of cell g (k of them, from scatter_out[s..s+k), written by other threads of this grid and
-// read past L1) ranked by id, then written in set order
-__device__ __forceinline__ void order_small_cell(const BroadArgs& a, int g, int s, int k)
+// The members of cell g (k of them, 2 to 4, from scatter_out[s..s+k), written by other threads of this
+// grid and read past L1) into set order, by one thread in registers: their table keeps its 8 slots,
+// which admit no linear probes.  The loads of the members, and then of their centres, go out together.
+// base: the first row of their scene.
+__device__ __forceinline__ void order_small_cell(const BroadArgs& a, int g, int s, int k, int base)
 {
     int m[SMALL_CELL];
-    for (int j = 0; j < k; ++j) {
-        int v = __ldcg(a.scatter_out + s + j);
-        int i = j;
-        while (i > 0 && m[i - 1] > v) {
-            m[i] = m[i - 1];
-            --i;
-        }
-        m[i] = v;
+#pragma unroll
+    for (int j = 0; j < SMALL_CELL; ++j) m[j] = j < k ? __ldcg(a.scatter_out + s + j) : 0x7fffffff;
+    auto order = [&](int i, int j) {
+        const int lo = min(m[i], m[j]), hi = max(m[i], m[j]);
+        m[i] = lo;
+        m[j] = hi;
+    };
+    order(0, 1);
+    order(2, 3);
+    order(0, 2);
+    order(1, 3);
+    order(1, 2);
+    double4 p[SMALL_CELL];
+#pragma unroll
+    for (int j = 0; j < SMALL_CELL; ++j)
+        if (a.sorted_pos && j < k) p[j] = reinterpret_cast<const double4*>(a.pos)[m[j]];
+    unsigned occ = 0, slot[SMALL_CELL];
+#pragma unroll
+    for (int j = 0; j < SMALL_CELL; ++j) {
+        if (j >= k) break;
+        slot[j] = pyset_slot8(occ, (unsigned)(m[j] - base));
+        occ |= 1u << slot[j];
     }
-    int o[SMALL_CELL];
-    int tab[SMALL_TAB], tmp[SMALL_TAB];
-    unsigned char used[SMALL_TAB], used2[SMALL_TAB];
-    const int base = a.info ? a.scenes[scene_of(a, m[0])].row_begin : 0;
-    pyset_order<SMALL_TAB>(m, k, o, tab, used, tmp, used2, base);
-    for (int j = 0; j < k; ++j) place(a, s + j, o[j], g);
+#pragma unroll
+    for (int j = 0; j < SMALL_CELL; ++j) {
+        if (j >= k) break;
+        const int o = s + __popc(occ & ((1u << slot[j]) - 1u));
+        a.sorted[o] = m[j];
+        if (a.sorted_pos) {
+            a.sorted_pos[o] = make_float4((float)p[j].x, (float)p[j].y, (float)p[j].z, (float)p[j].w);
+            a.sorted_cell[o] = g;
+        }
+    }
+}
+
+// a cell of 5 to 18 members for a warp of its block: k members from sorted position s, cell g, base the
+// first row of their scene
+struct WarpCell {
+    int g, s, k, base;
+};
+
+// the same for such cells, one after another by a full warp with one member per lane: list[i] for
+// i = first, first + step, ... < n.  The next cell's members are loaded while the present one is ordered.
+__device__ __forceinline__ void order_warp_cells(const BroadArgs& a, const WarpCell* list, int first, int step, int n)
+{
+    const int lane = threadIdx.x & 31;
+    auto member = [&](int i) { return i < n && lane < list[i].k ? __ldcg(a.scatter_out + list[i].s + lane) : 0x7fffffff; };
+    int next = member(first);
+    for (int i = first; i < n; i += step) {
+        const WarpCell c = list[i];
+        const int v = next;
+        double4 p = make_double4(0.0, 0.0, 0.0, 0.0);
+        if (lane < c.k && a.sorted_pos) p = reinterpret_cast<const double4*>(a.pos)[v];
+        next = member(i + step);
+        int rank = 0;
+        for (int j = 0; j < c.k; ++j) rank += __shfl_sync(0xffffffffu, v, j) < v;
+        const int o = c.s + pyset_warp_place(c.k, lane < c.k ? rank : -1, (unsigned)(v - c.base));
+        if (lane < c.k) {
+            a.sorted[o] = v;
+            if (a.sorted_pos) {
+                a.sorted_pos[o] = make_float4((float)p.x, (float)p.y, (float)p.z, (float)p.w);
+                a.sorted_cell[o] = c.g;
+            }
+        }
+    }
 }
 
 // The place pass: every row into its cell's range of the sorted list (the counting sort's scatter)
@@ -524,8 +611,10 @@ __device__ __forceinline__ void order_small_cell(const BroadArgs& a, int g, int 
 // cell claim slots with atomicSub on the cell's count (low 16 bits, counting down to zero), write
 // themselves into scatter_out, and then add 1 << 16 to the same word with an acquire-release atomic:
 // each member's add releases its write, and the member whose add finds k - 1 earlier ones (acquiring
-// all of them) orders the cell, in its own thread up to SMALL_CELL members, else by the first warp of its block with the
-// tables in shared memory; it sets the count back to zero.  (With PAIRS, of a two-member cell the
+// all of them) sets the count back to zero and orders the cell: in its own thread up to SMALL_CELL
+// members, by a warp of its block up to WARP_CELL, else by the block's first warp with the tables in
+// shared memory.  (On beds of 5,003 and 30,011 packed hulls, cells of up to 18 members, the pass takes 14
+// and 16.5 us; with one thread ordering up to 32 members, its table in local memory, it took 24 and 29.)  (With PAIRS, of a two-member cell the
 // first member to arrive leaves its id in the count word by an atomic exchange and the second,
 // finding it there, places both.)  Cells beyond BIG_CELL members are written in ascending ids, beyond
 // 65,535 (the packed count) in claim order; both are flagged MWD_ST_CELL_CROWDED.
@@ -540,9 +629,10 @@ __global__ void __launch_bounds__(PLACE_THREADS) place_kernel(BroadArgs a)
     pdl_wait();
     pdl_launch_dependents();
     __shared__ int s_crowd[PLACE_THREADS];
-    __shared__ int s_nc;
-    if (threadIdx.x == 0) s_nc = 0;
-    if (a.tile_sums) {  // read by the cell scan, which has finished: zero for the next broad phase
+    __shared__ WarpCell s_mid[PLACE_THREADS];
+    __shared__ int s_nc, s_nm;
+    if (threadIdx.x == 0) s_nc = s_nm = 0;
+    {  // read by the cell scan, which has finished: zero for the next broad phase
         int32_t* ts = a.sparse ? occ_tile_sums(a) : a.tile_sums;
         const int64_t nb = a.sparse ? (a.compact_len + SCAN_TILE - 1) / SCAN_TILE
                                     : (a.total_cells + SCAN_TILE - 1) / SCAN_TILE;
@@ -555,6 +645,7 @@ __global__ void __launch_bounds__(PLACE_THREADS) place_kernel(BroadArgs a)
         // the row's own centre, loaded beside its cell lookups (most rows are alone in their cell)
         double4 pr = make_double4(0.0, 0.0, 0.0, 0.0);
         if (a.sorted_pos) pr = reinterpret_cast<const double4*>(a.pos)[r];
+        const int scene = scene_of(a, r);
         const int g = a.cell_of[r];
         if (g >= 0) {
             // the cell's count word and range: by cell (dense table) or by its rank (sparse table)
@@ -587,6 +678,7 @@ __global__ void __launch_bounds__(PLACE_THREADS) place_kernel(BroadArgs a)
                 place(a, s + slot, r, g);
                 if (slot == 0) set_status(a.status, MWD_ST_CELL_CROWDED);
             } else {
+                const int base = a.info ? a.scenes[scene].row_begin : 0;  // its members share the scene
                 unsigned* w = reinterpret_cast<unsigned*>(cnt);
                 const int slot = (int)(atomicSub(w, 1u) & 0xffffu) - 1;
                 a.scatter_out[s + slot] = r;
@@ -596,13 +688,17 @@ __global__ void __launch_bounds__(PLACE_THREADS) place_kernel(BroadArgs a)
                 const unsigned before = prev >> 16;
                 if ((int)before == k - 1) {
                     *w = 0u;
-                    if (k <= SMALL_CELL) order_small_cell(a, g, s, k);
-                    else s_crowd[atomicAdd(&s_nc, 1)] = g;
+                    if (k <= SMALL_CELL) {
+                        order_small_cell(a, g, s, k, base);
+                    } else if (k <= WARP_CELL) {
+                        s_mid[atomicAdd(&s_nm, 1)] = {g, s, k, base};
+                    } else s_crowd[atomicAdd(&s_nc, 1)] = g;
                 }
             }
         }
     }
     __syncthreads();
+    order_warp_cells(a, s_mid, threadIdx.x / 32, PLACE_THREADS / 32, s_nm);
     const int nc = s_nc;
     if (nc == 0 || threadIdx.x >= 32) return;
     // the block's crowded cells, one at a time by its first warp: members ranked by id in parallel,
@@ -750,22 +846,21 @@ __device__ __forceinline__ void walk_pairs(const BroadArgs& a, int t, int r, int
         for (int j = rs[o]; j < re[o]; ++j) put(a.sorted[j], j);
 }
 
+// EMIT false: the candidates of each row, and (scan_tmp, zeroed by assign_kernel) of each tile of the
+// scan that follows; EMIT true: the pairs themselves, at the offsets that the scan left in pair_count
 template <bool EMIT>
 __global__ void pairs_kernel(BroadArgs a)
 {
     pdl_wait();
     pdl_launch_dependents();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n_sorted = n_sorted_rows(a);
-    if (t >= n_sorted) {
-        if (!EMIT && t < a.row_hi - a.row_lo) a.pair_count[t] = 0;
-        return;
-    }
-    const int r = a.sorted[t];
-    const int g = a.sorted_cell ? a.sorted_cell[t] : a.cell_of[r];
-    const int scene = scene_of(a, r);
+    const bool live = t < n_sorted_rows(a);
+    const int r = live ? a.sorted[t] : 0;
+    const int g = !live ? 0 : a.sorted_cell ? a.sorted_cell[t] : a.cell_of[r];
+    const int scene = live ? scene_of(a, r) : 0;
     const mwd_scene& sc = a.scenes[scene];
     if (EMIT) {
+        if (!live) return;
         int64_t out = a.pair_count[t];
         const int64_t cap = a.pair_cap;
         int2* pairs = reinterpret_cast<int2*>(a.pairs);
@@ -775,8 +870,10 @@ __global__ void pairs_kernel(BroadArgs a)
         });
     } else {
         int c = 0;
-        walk_pairs(a, t, r, g, sc, scene, nullptr, [&](int, int) { ++c; });
-        a.pair_count[t] = c;
+        if (live) walk_pairs(a, t, r, g, sc, scene, nullptr, [&](int, int) { ++c; });
+        if (t < a.row_hi - a.row_lo) a.pair_count[t] = c;
+        const int sum = __reduce_add_sync(0xffffffffu, c);
+        if ((threadIdx.x & 31) == 0 && sum) atomicAdd(a.scan_tmp + t / SCAN_TILE, sum);
     }
 }
 
@@ -955,17 +1052,19 @@ int64_t scan_tile_sums_offset(int64_t n) { return (n + SCAN_TILE - 1) / SCAN_TIL
 int launch_scan(const int32_t* in, int64_t n, int32_t* out, int32_t* tmp, int64_t* total_out, int64_t cap,
                 uint32_t* status, uint32_t overflow_bit, cudaStream_t s)
 {
-    if (n <= SCAN_SMALL_MAX) {
-        MWD_CUDA(launch_pdl(scan_small_kernel, 1, SCAN_SMALL_THREADS, 0, s, in, n, out, total_out, cap, status,
-                            overflow_bit));
-        return MWD_OK;
-    }
     const int nb = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
     const int nbl = nb > 0 ? nb : 1;
+    // Up to SCAN_RAW_MAX values in one launch: every block adds up the values before its tile itself (the
+    // last one at most 256 KB from L2): 3.4 us for 5,000 values, where one block for the whole scan took
+    // 12 us (17 us for 20,000).  Beyond, and in place, a pass over the tiles' totals first.
+    if (n <= SCAN_RAW_MAX && in != out) {
+        MWD_CUDA(launch_pdl(scan_final_kernel<SCAN_RAW>, nbl, SCAN_THREADS, 0, s, in, n, (const int32_t*)nullptr, out,
+                            nbl, total_out, cap, status, overflow_bit, aligned16(in, out), (int32_t*)nullptr));
+        return MWD_OK;
+    }
     MWD_CUDA(launch_pdl(scan_reduce_kernel, nbl, SCAN_THREADS, 0, s, in, n, tmp));
-    MWD_CUDA(launch_pdl(scan_final_kernel<false>, nbl, SCAN_THREADS, 0, s, in, n, tmp, out, nbl, total_out, cap,
-                        status, overflow_bit, aligned16(in, out), (int32_t*)nullptr));
-    MWD_CUDA(cudaGetLastError());
+    MWD_CUDA(launch_pdl(scan_final_kernel<SCAN_SUMS>, nbl, SCAN_THREADS, 0, s, in, n, (const int32_t*)tmp, out, nbl,
+                        total_out, cap, status, overflow_bit, aligned16(in, out), (int32_t*)nullptr));
     return MWD_OK;
 }
 
@@ -1022,21 +1121,20 @@ int launch_broad(const BroadArgs& a_in, cudaStream_t s)
         MWD_CUDA(cudaMemsetAsync(a.n_pairs, 0, sizeof(int64_t), s));
         return MWD_OK;
     }
+    if (!a.tile_sums) return MWD_ERR_INVALID;
     if (a.sparse) {
-        if (!a.tile_sums) return MWD_ERR_INVALID;
         const SparseLayout L = sparse_layout(rows, a.total_cells);
         a.n_words = (int32_t)L.n_words;
         a.words_pad = (int32_t)L.words_pad;
         a.compact_len = (int32_t)L.compact_len;
     }
     MWD_CUDA(launch_pdl(assign_kernel, blocks(rows, T), T, 0, s, a));
-    int rc = MWD_OK;
     if (a.sparse) {
         // the bitmap's scan (ranks of the occupied cells, a copy of the bits, the bits zeroed), the rows
         // per occupied cell, their scan
         const int nbw = (a.n_words + SCAN_TILE - 1) / SCAN_TILE;
         int32_t* copy = a.cell_start + a.words_pad;
-        MWD_CUDA(launch_pdl(scan_final_kernel<true>, nbw, SCAN_THREADS, 0, s, (const int32_t*)a.cell_count,
+        MWD_CUDA(launch_pdl(scan_final_kernel<SCAN_WORDS>, nbw, SCAN_THREADS, 0, s, (const int32_t*)a.cell_count,
                             (int64_t)a.n_words, (const int32_t*)a.tile_sums, a.cell_start, nbw, (int64_t*)nullptr,
                             (int64_t)INT64_MAX, (uint32_t*)nullptr, 0u,
                             aligned16(a.cell_count, a.cell_start) & aligned16(copy, copy), copy));
@@ -1044,22 +1142,19 @@ int launch_broad(const BroadArgs& a_in, cudaStream_t s)
         const int nbc = (a.compact_len + SCAN_TILE - 1) / SCAN_TILE;
         int32_t* cnt = a.cell_count + a.words_pad;
         int32_t* start = a.cell_start + 2 * a.words_pad;
-        MWD_CUDA(launch_pdl(scan_final_kernel<false>, nbc, SCAN_THREADS, 0, s, (const int32_t*)cnt,
+        MWD_CUDA(launch_pdl(scan_final_kernel<SCAN_SUMS>, nbc, SCAN_THREADS, 0, s, (const int32_t*)cnt,
                             (int64_t)a.compact_len, (const int32_t*)(a.tile_sums + nbw + 1), start, nbc,
                             (int64_t*)nullptr, (int64_t)INT64_MAX, (uint32_t*)nullptr, 0u, aligned16(cnt, start),
                             (int32_t*)nullptr));
-    } else if (a.tile_sums && a.total_cells > SCAN_SMALL_MAX) {
+    } else {
         // the tile totals were added up by assign_kernel: only the final pass of the scan remains (each
         // block adds up the totals of the tiles before it; turning them into prefixes in a separate
         // one-block pass first measured no faster with 7,300 tiles)
         const int nb = (int)((a.total_cells + SCAN_TILE - 1) / SCAN_TILE);
-        MWD_CUDA(launch_pdl(scan_final_kernel<false>, nb, SCAN_THREADS, 0, s, (const int32_t*)a.cell_count,
+        MWD_CUDA(launch_pdl(scan_final_kernel<SCAN_SUMS>, nb, SCAN_THREADS, 0, s, (const int32_t*)a.cell_count,
                             a.total_cells, (const int32_t*)a.tile_sums, a.cell_start, nb, (int64_t*)nullptr,
                             (int64_t)INT64_MAX, (uint32_t*)nullptr, 0u, aligned16(a.cell_count, a.cell_start),
                             (int32_t*)nullptr));
-    } else {
-        rc = launch_scan(a.cell_count, a.total_cells, a.cell_start, a.scan_tmp, nullptr, INT64_MAX, nullptr, 0, s);
-        if (rc) return rc;
     }
     // the two-member exchange path from two full waves of place blocks up (a 256-scene batch of 2M
     // rows: broad phase 0.221 -> 0.211 ms; a 20k-row pour is 1-2 us slower with it)
@@ -1079,12 +1174,12 @@ int launch_broad(const BroadArgs& a_in, cudaStream_t s)
         MWD_CUDA(cudaGetLastError());
         return MWD_OK;
     }
-    pairs_kernel<false><<<blocks(rows, T), T, 0, s>>>(a);
-    rc = launch_scan(a.pair_count, rows, a.pair_count, a.scan_tmp, a.n_pairs, a.pair_cap, a.status,
-                     MWD_ST_PAIR_OVERFLOW, s);
-    if (rc) return rc;
-    pairs_kernel<true><<<blocks(rows, T), T, 0, s>>>(a);
-    MWD_CUDA(cudaGetLastError());
+    MWD_CUDA(launch_pdl(pairs_kernel<false>, blocks(rows, T), T, 0, s, a));
+    const int nb = (int)((rows + SCAN_TILE - 1) / SCAN_TILE);
+    MWD_CUDA(launch_pdl(scan_final_kernel<SCAN_SUMS>, nb, SCAN_THREADS, 0, s, (const int32_t*)a.pair_count, rows,
+                        (const int32_t*)a.scan_tmp, a.pair_count, nb, a.n_pairs, a.pair_cap, a.status,
+                        (uint32_t)MWD_ST_PAIR_OVERFLOW, aligned16(a.pair_count, a.pair_count), (int32_t*)nullptr));
+    MWD_CUDA(launch_pdl(pairs_kernel<true>, blocks(rows, T), T, 0, s, a));
     return MWD_OK;
 }
 

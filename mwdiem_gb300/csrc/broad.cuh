@@ -32,7 +32,7 @@ struct BroadArgs {
     uint32_t* status;
     int64_t total_cells;
     int64_t pair_cap;
-    int32_t* tile_sums;          // optional: per-scan-tile cell counts, added to by assign_kernel, read by
+    int32_t* tile_sums;          // per-scan-tile cell counts, zero on entry, added to by assign_kernel, read by
                                  // the cell scan (no reduce pass) and zeroed by place_kernel
     int32_t walk_parts;          // append mode: threads per row (1, or 8: walls + own cell, 7 neighbours)
     // occupancy-compressed cell table (sparse = 1; needs tile_sums): a bit per cell of the dense

@@ -444,13 +444,13 @@ int mwd_linked_cell_hash(int32_t n_lo, int32_t n_hi, const int64_t* keys, int64_
     broad_table_ints(rows, R, sparse, &count_ints, &start_ints);
     Carver c;
     size_t o_scene = c.take<mwd_scene>(1);
-    size_t o_count = c.take<int32_t>(count_ints);
+    size_t o_tmp = c.take<int32_t>(scan_tmp_ints(m));  // ends with the per-tile cell counts: zeroed with
+    size_t o_count = c.take<int32_t>(count_ints);       // the cell counts that follow
     size_t o_start = c.take<int32_t>(start_ints);
     size_t o_cellof = c.take<int32_t>(n_hi);
     size_t o_scat = c.take<int32_t>(n_hi);
     size_t o_sorted = c.take<int32_t>(n_hi);
     size_t o_pc = c.take<int32_t>(rows + 1);
-    size_t o_tmp = c.take<int32_t>(scan_tmp_ints(m));
     rc = scratch(c.off, &base);
     if (rc) return rc;
     char* b = (char*)base;
@@ -461,12 +461,8 @@ int mwd_linked_cell_hash(int32_t n_lo, int32_t n_hi, const int64_t* keys, int64_
     sc.n_keys = R;
     sc.cell_base = 0;
     MWD_CUDA(cudaMemcpyAsync(b + o_scene, &sc, sizeof(sc), cudaMemcpyHostToDevice, s));
-    MWD_CUDA(cudaMemsetAsync(b + o_count, 0, count_ints * sizeof(int32_t), s));
-    int32_t* tile_sums = nullptr;
-    if (sparse) {  // the compressed table's per-tile counts, zero on entry
-        tile_sums = reinterpret_cast<int32_t*>(b + o_tmp) + scan_tile_sums_offset(m);
-        MWD_CUDA(cudaMemsetAsync(tile_sums, 0, (scan_tmp_ints(m) - scan_tile_sums_offset(m)) * sizeof(int32_t), s));
-    }
+    MWD_CUDA(cudaMemsetAsync(b + o_tmp, 0, o_count - o_tmp + count_ints * sizeof(int32_t), s));
+    int32_t* tile_sums = reinterpret_cast<int32_t*>(b + o_tmp) + scan_tile_sums_offset(m);
     BroadArgs a = {};
     a.row_lo = n_lo;
     a.row_hi = n_hi;

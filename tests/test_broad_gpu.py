@@ -119,3 +119,35 @@ def test_very_crowded_cell_flags_status():
     ref = oracle.linked_cell_hash(0, n, keys, 4, 4)
     assert int(st.item()) & _lib.ST_CELL_CROWDED
     assert set(map(frozenset, got.tolist())) == set(map(frozenset, ref.tolist()))
+
+
+@pytest.mark.parametrize("base", [0, 1_000_000])
+def test_cells_of_every_size_in_set_order(base):
+    # cells of 1 to 36 members, far apart, ids drawn at random: the orientation of every pair follows
+    # CPython's set order through each growth of the table (5th, 19th member) and past the warp limit (32)
+    from mwdiem_gb300 import LIBRARY_Coarse_contact_detection as CCD
+    rng = np.random.default_rng(31)
+    sizes = np.tile(np.arange(1, 37), 12)
+    cell = np.repeat(np.arange(len(sizes)) * 1000, sizes)
+    n = len(cell)
+    keys = np.zeros(base + n, np.int64)
+    keys[base:] = cell[rng.permutation(n)]
+    ref = oracle.linked_cell_hash(base, base + n, keys, 11, 11)
+    got = CCD.Linked_cell_hash(None, 11, 11, base, base + n, [], keys)
+    assert len(got) == len(ref) and pairset(got) == pairset(ref)
+
+
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 4096, 65535, 65536, 65537])
+def test_scan_tile_edges(n):
+    # rows, cells and wall tests at the edges of the scans' tiles and of the one-launch scan
+    from mwdiem_gb300 import LIBRARY_Coarse_contact_detection as CCD
+    rng = np.random.default_rng(n)
+    keys = rng.integers(0, n, size=n).astype(np.int64)
+    keys[:2] = 0, n - 1
+    ref = oracle.linked_cell_hash(0, n, keys, 13, 13)
+    got = CCD.Linked_cell_hash(None, 13, 13, 0, n, [], keys)
+    assert len(got) == len(ref) and pairset(got) == pairset(ref)
+    com = rng.uniform(-20, 20, size=(n + 1, 3))
+    wn, wc = np.array([[0.0, 0.6, 0.8]]), np.zeros((1, 3))
+    wall = CCD.wall_pairs(com, wn, wc, 1, 1, n + 1, 14.4).cpu().numpy()
+    assert np.array_equal(wall, oracle.wall_pairs(1, 1, n + 1, com, wn, wc, 14.4))
