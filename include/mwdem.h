@@ -48,7 +48,7 @@ enum {
 };
 
 #define MWD_EPA_FACE_CAP 128   /* EPA faces per pair, deleted ones included as in the reference (a pair
-                                  that needs more runs again with the deleted faces removed) */
+                                  that needs more drops the deleted faces) */
 #define MWD_EPA_COUNT_INTS 256 /* ints of mwd_work.epa_count */
 #define MWD_EPA_VERT_CAP 32    /* EPA polytope vertices per pair (4 + 25 iterations + 1) */
 #define MWD_HULL_CAP 64        /* hull vertices per side staged in shared memory */
@@ -300,9 +300,7 @@ typedef struct {
     uint64_t* work_counters; /* optional (3,), added to by the narrow phase: vertex dot products of the
                               support queries, EPA faces created, support queries (NULL: not counted) */
     int32_t* epa_count;    /* (MWD_EPA_COUNT_INTS,) 8-byte aligned, two-pass narrow phase: [0] pairs found in
-                              contact by the GJK pass, [2..3] the EPA pass's work queue (uint64), [4] and
-                              [8..] the records whose EPA face list overflowed (run again after the
-                              pass); [0..7] are zeroed by the broad phase of mwd_step, or by
+                              contact by the GJK pass, [2..3] the EPA pass's work queue (uint64); [0..7] are zeroed by the broad phase of mwd_step, or by
                               mwd_narrow_force when it runs alone */
     void* epa_rec;         /* (epa_cap, 80 B): their simplex; NULL selects the single-pass kernel */
     int64_t epa_cap;
@@ -369,9 +367,9 @@ int mwd_broadphase(const mwd_state* st, const mwd_scene* scenes_dev, const mwd_s
 
 /* Narrow phase + force over work->pairs[0 .. *work->n_pairs) into st->force/torque.
  * lanes: lanes per pair of the GJK pass (1 with the two-pass kernel, 4, 8, 16, 32), plus, in bits
- * 8-15, those of the EPA pass of the two-pass kernel (0: the same); bit 16 set: the EPA pass reads
- * the hulls in place from the vertex table instead of staging them in shared memory (less shared
- * memory, more resident pairs); bits 20-21 and 22-23: threads per block of the GJK and EPA passes
+ * 8-15, those of the EPA pass of the two-pass kernel (0, 4, 8, 16 or 32) and, in bit 16, whether it
+ * reads the hulls in place: both are accepted and without effect, the pass gives each pair a warp
+ * that reads the hulls in place; bits 20-21 and 22-23: threads per block of the GJK and EPA passes
  * of the two-pass kernel (0: 128, 1: 64, 2: 256). */
 #define MWD_LANES_EPA_IN_PLACE (1 << 16)
 #define MWD_LANES_GJK_BLOCK_SHIFT 20

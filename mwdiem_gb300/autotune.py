@@ -1,9 +1,8 @@
 """Autotuner for the device-resident step.
 
-Chooses the lanes per pair of the narrow phase's GJK pass (1, 4, 8 or 16) and EPA pass (8, 16 or 32),
-whether the EPA pass stages the two hulls in shared memory or reads them in place, and then the
-threads per block of each of the two passes (64, 128 or 256), by timing graph-captured steps of the
-actual scene and keeping the fastest.  The cell size is not a tuning knob: it decides the
+Chooses the lanes per pair of the narrow phase's GJK pass (1, 4, 8 or 16; the EPA pass gives each pair
+a warp) and then the threads per block of each of the two passes (64, 128 or 256), by timing
+graph-captured steps of the actual scene and keeping the fastest.  The cell size is not a tuning knob: it decides the
 reference's candidate set (an 8-cell forward stencil misses some neighbour pairs, and which ones
 depends on the cell size), so it stays what the scene defines (MWDiem.py:575-580).  The reference
 hard-codes its launch geometry (gpu_fine_contact_detection.py:28-29, gpu_Verlet.py:26-27).
@@ -47,13 +46,14 @@ def time_steps(sim, steps=5, reps=3, per=1, flush=None):
     return best[len(best) // 2]
 
 
-# lanes word: GJK-pass lanes | EPA-pass lanes << 8 | EPA hulls read in place (no staging) << 16 |
+# lanes word: GJK-pass lanes | EPA-pass lanes << 8 | EPA hulls read in place << 16 (these two without
+# effect: the EPA pass gives each pair a warp that reads the hulls in place) |
 # block-size codes of the two passes << 20 and << 22 (0: 128 threads, 1: 64, 2: 256)
 EPA_IN_PLACE = 1 << 16
 GJK_BLOCK_SHIFT = 20
 EPA_BLOCK_SHIFT = 22
 BLOCK_THREADS = {0: 128, 1: 64, 2: 256}
-DEFAULT_CANDIDATES = tuple(g | (e << 8) | f for g in (1, 4, 8, 16) for e in (8, 16, 32) for f in (0, EPA_IN_PLACE))
+DEFAULT_CANDIDATES = tuple(g | (32 << 8) | EPA_IN_PLACE for g in (1, 4, 8, 16))
 
 
 def block_size(lanes):
@@ -80,8 +80,7 @@ def describe(lanes):
 
 
 def tune_lanes(sim, candidates=DEFAULT_CANDIDATES, steps=5, blocks=True, flush=None):
-    """Time the scene with each lanes-per-pair setting (GJK-pass lanes | EPA-pass lanes << 8) on a
-    copy of its state, then the block sizes of the two passes at the fastest setting; set the fastest
+    """Time the scene with each lanes-per-pair setting of the GJK pass on a copy of its state, then the block sizes of the two passes at the fastest setting; set the fastest
     on `sim`, and return {setting: ms per step}.  The state of `sim` is restored afterwards.  `flush`:
     time every step with L2 overwritten first (time_steps)."""
     saved = {k: v.clone() for k, v in sim.t.items()}

@@ -464,7 +464,7 @@ __global__ void assign_kernel(BroadArgs a)
     pdl_launch_dependents();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (a.append) *a.n_pairs = 0;  // appended to by pairs_append_kernel
-        if (a.epa_count)  // the EPA record count, the EPA pass's work queue and retry count
+        if (a.epa_count)  // the EPA record count and the EPA pass's work queue
             for (int k = 0; k < 8; ++k) a.epa_count[k] = 0;
     }
     const int r = a.row_lo + blockIdx.x * blockDim.x + threadIdx.x;
@@ -614,9 +614,9 @@ __device__ __forceinline__ void order_warp_cells(const BroadArgs& a, const WarpC
 // all of them) sets the count back to zero and orders the cell: in its own thread up to SMALL_CELL
 // members, by a warp of its block up to WARP_CELL, else by the block's first warp with the tables in
 // shared memory.  (On beds of 5,003 and 30,011 packed hulls, cells of up to 18 members, the pass takes 14
-// and 16.5 us; with one thread ordering up to 32 members, its table in local memory, it took 24 and 29.)  (With PAIRS, of a two-member cell the
-// first member to arrive leaves its id in the count word by an atomic exchange and the second,
-// finding it there, places both.)  Cells beyond BIG_CELL members are written in ascending ids, beyond
+// and 16.5 us; with one thread ordering up to 32 members, its table in local memory, it took 24 and 29.)
+// (With PAIRS, of a two-member cell the first member to arrive leaves its id in the count word by an
+// atomic exchange and the second, finding it there, places both.)  Cells beyond BIG_CELL members are written in ascending ids, beyond
 // 65,535 (the packed count) in claim order; both are flagged MWD_ST_CELL_CROWDED.
 constexpr int PLACE_THREADS = 128;
 constexpr int PACKED_MAX = 0xffff;

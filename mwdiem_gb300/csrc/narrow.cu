@@ -8,18 +8,17 @@
 //  * a group of LPP lanes (4/8/16/32) works on one pair; a block holds 128/LPP groups and the grid
 //    strides over the pair list.  The device step runs two passes: GJK (gjk_pass_kernel, also one
 //    lane per pair) writes the pairs in contact with the simplex it stopped on to a list, and EPA
-//    with the force (epa_pass_kernel) continues from that list with its own lanes per pair;
-//  * a support query is a strided scan of the float4 hull vertices (staged in shared memory, or read
+//    with the force (epa_pass_kernel) continues from that list with a warp per pair;
+//  * a GJK support query is a strided scan of the float4 hull vertices (staged in shared memory, or read
 //    in place from the L1-cached vertex table) by the group's lanes, then a group argmax on (value
 //    desc, index asc), which reproduces the reference's strict-'>' first-index tie break;
 //  * the simplex logic runs redundantly (identically) on every lane of the group, so control flow
 //    stays group-uniform;
-//  * EPA keeps an append-only face list of MWD_EPA_FACE_CAP faces in shared memory, like the
-//    reference's T[50]/n[50]/dist[50] (which overflow past 50 faces); a pair that outgrows it runs
-//    again with the deleted faces removed from the list (epa_compacting); the face scan, the
-//    visibility test, the horizon edge count (the reference's 50x50 delpair matrix, replaced by
-//    counting over the deleted-face list) and the new faces are computed lane-parallel, with ballots
-//    to keep the reference's face order;
+//  * EPA keeps an append-only face list of MWD_EPA_FACE_CAP faces, four in each lane's registers, like
+//    the reference's T[50]/n[50]/dist[50] (which overflow past 50 faces); when it is full the removed
+//    faces are dropped from it; the face scan, the visibility test, the horizon edge count (the
+//    reference's 50x50 delpair matrix, replaced by marks per vertex pair) and the new faces are computed
+//    lane-parallel, with ballots to keep the reference's face order;
 //  * force/torque are accumulated with float atomics (skipped for wall rows in table mode, whose
 //    forces the reference discards, MWDiem.py:977-978).
 #include <float.h>
@@ -34,22 +33,7 @@ namespace {
 constexpr int FCAP = MWD_EPA_FACE_CAP;
 constexpr int VCAP = MWD_EPA_VERT_CAP;
 
-// per-group shared memory (the hull staging area follows, 2 * hull_cap float4)
-struct EpaMem {
-    float4 fn[FCAP];       // face normal xyz, distance
-    uint32_t ft[FCAP];     // T0 | T1 << 8 | T2 << 16 | (valid + 2) << 24
-    float4 pv[VCAP];       // polytope vertices
-    uint16_t pab[VCAP];    // support index on A | on B << 8
-    uint32_t del[FCAP];    // faces deleted in this iteration, in index order: vertices T0 T1 T2 | face << 24
-};
-
 __device__ __forceinline__ int ft_v(uint32_t t, int k) { return (t >> (8 * k)) & 0xff; }
-__device__ __forceinline__ int ft_valid(uint32_t t) { return (int)(t >> 24) - 2; }
-__device__ __forceinline__ uint32_t ft_make(int a, int b, int c, int valid)
-{
-    return (uint32_t)a | ((uint32_t)b << 8) | ((uint32_t)c << 16) | ((uint32_t)(valid + 2) << 24);
-}
-
 template <int LPP>
 struct Group {
     int lane;
@@ -68,9 +52,8 @@ struct Group {
 // group reductions below run on these keys with redux.sync.
 __device__ __forceinline__ unsigned fkey(float f)
 {
-    f = (f == 0.f) ? 0.f : f;
-    const unsigned b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+    const unsigned b = __float_as_uint(f + 0.f);
+    return b ^ ((unsigned)((int)b >> 31) | 0x80000000u);
 }
 
 // Group-wide (largest value, then smallest index) of the lanes' (v, i), v not NaN: the sequential
@@ -91,12 +74,6 @@ __device__ __forceinline__ unsigned long long* epa_queue(const NarrowArgs& a)
 {
     return reinterpret_cast<unsigned long long*>(a.epa_count + 2);
 }
-
-// EPA records whose face list overflowed, run again by epa_retry_kernel after the EPA pass: their
-// count at int [4] of the block epa_count points to, the record indices from int [8]
-constexpr int EPA_RETRY_CAP = MWD_EPA_COUNT_INTS - 8;
-__device__ __forceinline__ int* epa_retry_count(const NarrowArgs& a) { return a.epa_count + 4; }
-__device__ __forceinline__ int32_t* epa_retry_list(const NarrowArgs& a) { return a.epa_count + 8; }
 
 // The next `amount` items of a queue for the calling group: its first lane takes them with one atomic.
 template <int LPP>
@@ -259,22 +236,20 @@ __device__ __forceinline__ bool is_flat(f3 S1, f3 S2, f3 S3, f3 S4)
     return false;
 }
 
-// The EPA's convergence test (.cu:439), (double)x * 1.00001 > (double)p && (double)x * 0.99999 <
-// (double)p, decided in FP32 unless p lies within 2^-22 |x| of one of the two bounds.  The float
-// products x * 1.00001f, x * 0.99999f are within 7.5e-8 |x| of the double ones and the shifted
-// bounds round by at most 6e-8 |x| more (1.4e-7 |x| < 2^-22 |x| in all), so outside that band the
-// float answer is the double one; inside it (and for |x| outside [1e-30, 1e37], NaN, or 0) the
-// double test runs.
-__device__ __forceinline__ bool epa_converged(float x, float p)
+// The EPA's stop tests (.cu:437-439): x > p, or (double)x * 1.00001 > (double)p && (double)x * 0.99999 <
+// (double)p.  For x > 0 the two together are (double)x * 1.00001 > (double)p, decided in FP32 unless p
+// lies within 2^-22 x of the bound: the float product x * 1.00001f is within 7.5e-8 x of the double one
+// and the shifted bounds round by at most 6e-8 x more (1.4e-7 x < 2^-22 x in all), so outside that band
+// the float answer is the double one; inside it (and for x outside [1e-30, 1e37], NaN, or 0) the
+// reference's tests run.
+__device__ __forceinline__ bool epa_stops(float x, float p)
 {
-    const float ax = fabsf(x);
-    if (ax > 1e-30f && ax < 1e37f) {
-        const float hi = x * 1.00001f, lo = x * 0.99999f;
-        const float tol = ax * 2.384185791015625e-7f;
-        if (p < hi - tol && p > lo + tol) return true;
-        if (p > hi + tol || p < lo - tol) return false;
+    if (x > 1e-30f && x < 1e37f) {
+        const float hi = x * 1.00001f, tol = x * 2.384185791015625e-7f;
+        if (p < hi - tol) return true;
+        if (p > hi + tol) return false;
     }
-    return (double)x * 1.00001 > (double)p && (double)x * 0.99999 < (double)p;
+    return x > p || ((double)x * 1.00001 > (double)p && (double)x * 0.99999 < (double)p);
 }
 
 // ---------------------------------------------------------------- the reference's double results in FP32
@@ -401,52 +376,6 @@ __device__ __forceinline__ int coulomb_compare(float Ftn, float Fnn, const mwd_m
     return X > P ? 1 : (X <= P ? 0 : -1);
 }
 
-// AddTriangle (.cu:270-325): normal and distance of the face (e0, e1, e2), its winding (t1, t2) and
-// validity (1, or -2 with distance 1e30 when the origin's projection falls outside it)
-__device__ __forceinline__ float4 face_geom(const EpaMem& m, int e0, int e1, int e2, int& t1, int& t2, int& valid)
-{
-    f3 a = xyz(m.pv[e0]), b = xyz(m.pv[e1]), c = xyz(m.pv[e2]);
-    f3 n = cross(b - a, c - b);
-    float len = sqrtf(n.x * n.x + n.y * n.y + n.z * n.z);
-    n = n / len;
-    float dist = dot(n, a);
-    t1 = e1;
-    t2 = e2;
-    if (dist < 0.f) {
-        t2 = e1;
-        t1 = e2;
-        dist = dist * (-1.f);
-        n = n * (-1.f);
-    }
-    f3 A = xyz(m.pv[e0]), B = xyz(m.pv[t1]), C = xyz(m.pv[t2]);
-    bool inside = false;
-    if (dot(cross(B - A, n), A * (-1.f)) < 0.f)
-        if (dot(cross(C - B, n), B * (-1.f)) < 0.f)
-            if (dot(cross(A - C, n), C * (-1.f)) < 0.f) inside = true;
-    valid = 1;
-    if (!inside) {
-        valid = -2;
-        dist = 1e30f;
-    }
-    return f4(n, dist);
-}
-
-// AddTriangle into slot f of the face list, one face per calling lane
-__device__ __forceinline__ void add_face(EpaMem& m, int e0, int e1, int e2, int f)
-{
-    int t1, t2, valid;
-    m.fn[f] = face_geom(m, e0, e1, e2, t1, t2, valid);
-    m.ft[f] = ft_make(e0, t1, t2, valid);
-}
-
-// "x < best" of the reference's array_min_finder (.cu:41-53), NaN never wins
-__device__ __forceinline__ bool min_better(float v, int i, float bv, int bi)
-{
-    if (v != v) return false;
-    if (bv != bv) return true;
-    return v < bv || (v == bv && i < bi);
-}
-
 struct EpaResult {
     float depth;
     f3 n, cpA, cpB;
@@ -454,193 +383,13 @@ struct EpaResult {
     uint32_t status;
 };
 
-// EPA (.cu:328-603) with the reference's append-only face list: deleted faces stay in it at distance
-// 3e20 (.cu:541-542).  A pair whose list would outgrow FCAP stops with MWD_ST_EPA_OVERFLOW and is run
-// again by epa_compacting.
-template <int LPP>
-__device__ void epa(const Group<LPP>& g, EpaMem& m, const float4* hA, int nA, const float4* hB, int nB,
-                    f3 S1, int a1, int b1, f3 S2, int a2, int b2, f3 S3, int a3, int b3, f3 S4, int a4, int b4,
-                    EpaResult& r, Work3& wk)
-{
-    r.status = 0;
-    g.sync();
-    if (g.lane == 0) {
-        m.pv[0] = f4(S1, 0.f); m.pv[1] = f4(S2, 0.f); m.pv[2] = f4(S3, 0.f); m.pv[3] = f4(S4, 0.f);
-        m.pab[0] = (uint16_t)(a1 | (b1 << 8)); m.pab[1] = (uint16_t)(a2 | (b2 << 8));
-        m.pab[2] = (uint16_t)(a3 | (b3 << 8)); m.pab[3] = (uint16_t)(a4 | (b4 << 8));
-    }
-    g.sync();
-    if (g.lane < 4) {
-        // faces (0,1,2), (1,2,3), (2,0,3), (0,1,3), packed as 4-bit vertex numbers (no local array)
-        const unsigned long long e = 0x310302321210ull >> (12 * g.lane);
-        add_face(m, (int)(e & 0xf), (int)((e >> 4) & 0xf), (int)((e >> 8) & 0xf), g.lane);
-    }
-    g.sync();
-    wk.faces += 4;
-    int nt = 4, nv = 4, counter = 0, indmin = 0;
-    float xmin_old = 1e29f;
-    float proj = 2 * xmin_old + 1;
-    float xmin_new = 0.f;
-    while (xmin_old < proj) {
-        // first index of the minimum distance
-        float bv = __int_as_float(0x7fffffff);
-        int bi = 0x7fffffff;
-        for (int f = g.lane; f < nt; f += LPP) {
-            float v = m.fn[f].w;
-            if (min_better(v, f, bv, bi)) { bv = v; bi = f; }
-        }
-        {
-            // group minimum (NaN never wins), then the first face index holding it
-            const unsigned k = (bv != bv) ? 0xffffffffu : fkey(bv);
-            const unsigned km = __reduce_min_sync(g.mask, k);
-            bi = (int)__reduce_min_sync(g.mask, k == km ? (unsigned)bi : 0xffffffffu);
-        }
-        float d0 = m.fn[0].w;
-        indmin = (d0 != d0) ? 0 : bi;
-        float4 fm = m.fn[indmin];
-        xmin_new = fm.w;
-        xmin_old = xmin_new;
-        f3 n = xyz(fm);
-        f3 s;
-        int sa, sb;
-        support<LPP>(g, hA, nA, hB, nB, n, s, sa, sb, wk);
-        proj = dot(n, s);
-        if (xmin_old > proj || epa_converged(xmin_old, proj)) break;
-        if (counter > 49) { r.status |= MWD_ST_EPA_NOCONV; break; }
-        counter = counter + 1;
-        if (nv >= VCAP) { r.status |= MWD_ST_EPA_OVERFLOW; break; }
-        g.sync();
-        if (g.lane == 0) {
-            m.pv[nv] = f4(s, 0.f);
-            m.pab[nv] = (uint16_t)(sa | (sb << 8));
-        }
-        nv++;
-        // visible faces -> deleted, collected in index order
-        int ndel = 0;
-        for (int base = 0; base < nt; base += LPP) {
-            int f = base + g.lane;
-            bool dead = false;
-            uint32_t t = 0;
-            if (f < nt) {
-                t = m.ft[f];
-                int vl = ft_valid(t);
-                if ((vl == 1 || vl == -2) && dot(s - xyz(m.pv[ft_v(t, 0)]), xyz(m.fn[f])) >= 0.f) {
-                    dead = true;
-                    m.ft[f] = (t & 0x00ffffffu) | ((uint32_t)(-1 + 2) << 24);
-                }
-            }
-            unsigned b = g.ballot(dead);
-            if (dead) m.del[ndel + __popc(b & g.lt_mask())] = (t & 0x00ffffffu) | ((uint32_t)f << 24);
-            ndel += __popc(b);
-        }
-        g.sync();
-        // horizon edges of the deleted faces, in face order then edge order (0,1),(1,2),(2,0);
-        // an edge is kept when fewer than two delpair increments land on it (.cu:482-544), i.e. when
-        // its unordered vertex pair occurs once among the deleted faces' edges (a face's vertex indices
-        // are distinct).  When all those edges fit the group's lanes at once, one match over the lanes'
-        // vertex pairs counts them; otherwise each lane counts its edge against the deleted list.
-        int nnew = 0;
-        bool overflow = false;
-        const bool one_trip = 3 * ndel <= LPP;
-        for (int base = 0; base < 3 * ndel; base += LPP) {
-            int c = base + g.lane;
-            bool keep = false;
-            int e0 = 0, e1 = 0;
-            unsigned pair_code = 0x10000u + (unsigned)g.lane;  // distinct for lanes without an edge
-            if (c < 3 * ndel) {
-                uint32_t t = m.del[c / 3];
-                int k = c % 3;
-                e0 = ft_v(t, k);
-                e1 = ft_v(t, k == 2 ? 0 : k + 1);
-                pair_code = (unsigned)(min(e0, e1) * 256 + max(e0, e1));
-                if (!one_trip) {
-                    int cnt = 0;
-                    for (int j = 0; j < ndel; ++j) {
-                        uint32_t u = m.del[j];
-                        int x = ft_v(u, 0), y = ft_v(u, 1), z = ft_v(u, 2);
-                        cnt += (e0 == y && e1 == x) + (e0 == x && e1 == y) + (e0 == z && e1 == y) +
-                               (e0 == y && e1 == z) + (e0 == x && e1 == z) + (e0 == z && e1 == x);
-                    }
-                    keep = cnt < 2;
-                }
-            }
-            if (one_trip) {
-                // every lane of the group takes part in the match (lanes without an edge hold a code no
-                // other lane holds)
-                const unsigned same = __match_any_sync(g.mask, pair_code);
-                keep = c < 3 * ndel && __popc(same) == 1;
-            }
-            unsigned b = g.ballot(keep);
-            if (keep) {
-                int f = nt + nnew + __popc(b & g.lt_mask());
-                if (f < FCAP) add_face(m, e0, e1, nv - 1, f);
-            }
-            nnew += __popc(b);
-        }
-        if (nt + nnew > FCAP) overflow = true;
-        g.sync();
-        for (int k = g.lane; k < ndel; k += LPP) {
-            int f = (int)(m.del[k] >> 24);
-            m.ft[f] = (m.ft[f] & 0x00ffffffu) | ((uint32_t)(0 + 2) << 24);
-            m.fn[f].w = 3e20f;
-        }
-        g.sync();
-        if (overflow) { r.status |= MWD_ST_EPA_OVERFLOW; break; }
-        nt += nnew;
-        wk.faces += (uint32_t)nnew;
-        counter = counter + 1;
-    }
-    g.sync();
-    r.depth = xmin_new;
-    // the contact point and everything after it (the force) are needed by one lane only: the others
-    // skip them, which keeps their FP64 operations (below and in contact_force) off the FP64 pipe
-    if (g.lane != 0) return;
-    uint32_t t = m.ft[indmin];
-    int a = ft_v(t, 0), b = ft_v(t, 1), c = ft_v(t, 2);
-    f3 n = xyz(m.fn[indmin]);
-    f3 Pr = n * r.depth;
-    f3 Va = xyz(m.pv[a]), Vb = xyz(m.pv[b]), Vc = xyz(m.pv[c]);
-    f3 v0 = Vb - Va, v1 = Vc - Va, v2 = Pr - Va;
-    if (dot(cross(v0, v1), n) < 0.f) {
-        v0 = Vc - Va;
-        v1 = Vb - Va;
-    }
-    float v00 = dot(v0, v0), v01 = dot(v0, v1), v11 = dot(v1, v1), v20 = dot(v2, v0), v21 = dot(v2, v1);
-    float den = v00 * v11 - v01 * v01;
-    float bv = (v11 * v20 - v01 * v21) / den;
-    float bw = (v00 * v21 - v01 * v20) / den;
-    float bu = one_minus_two(bw, bv);
-    int pa = m.pab[a], pb = m.pab[b], pc = m.pab[c];
-    r.fa[0] = pa & 0xff; r.fa[1] = pb & 0xff; r.fa[2] = pc & 0xff;
-    r.fb[0] = pa >> 8; r.fb[1] = pb >> 8; r.fb[2] = pc >> 8;
-    r.cpA = (xyz(hA[r.fa[0]]) * bu + xyz(hA[r.fa[1]]) * bv) + xyz(hA[r.fa[2]]) * bw;
-    r.cpB = (xyz(hB[r.fb[0]]) * bu + xyz(hB[r.fb[1]]) * bv) + xyz(hB[r.fb[2]]) * bw;
-    r.n = n;
-}
-
-// The EPA of a pair whose face list outgrew FCAP, run again from the same simplex: the same decisions
-// and arithmetic with the deleted faces removed from the list (the survivors keep their order) instead
-// of kept at 3e20.  Of the removed faces only the earliest created can still win the minimum search
-// (.cu:41-53: all are at 3e20, the first index wins): it is kept in the list's last slot, FCAP - 1, with
-// every face's creation index (its index in the reference's arrays) packed into its vertex word:
-// T0 | T1 << 5 | T2 << 10 | (valid + 2) << 15 | creation << 17.  At most 2 * 30 - 4 = 56 faces are
-// alive within the reference's iteration limit, so this list does not overflow.  Rarely needed: the
-// two-pass narrow phase runs the records that overflowed again in a kernel of their own after its EPA
-// pass, the single-pass kernel calls it out of line right after the overflow (epa_run).
-__device__ __forceinline__ int fc_v(uint32_t t, int k) { return (t >> (5 * k)) & 31; }
-__device__ __forceinline__ uint32_t fc_created(uint32_t t) { return t >> 17; }
-__device__ __forceinline__ uint32_t fc_make(int a, int b, int c, int valid, uint32_t created)
-{
-    return (uint32_t)a | ((uint32_t)b << 5) | ((uint32_t)c << 10) | ((uint32_t)(valid + 2) << 15) | (created << 17);
-}
-
 // contact points of the final face (.cu:548-600): barycentric coordinates of n * depth on the face
-// (winding swapped when its normal points the other way), applied to the support vertices of A and B
-__device__ __forceinline__ void epa_contact(const EpaMem& m, const float4* hA, const float4* hB, f3 n, int a, int b,
-                                            int c, EpaResult& r)
+// Va, Vb, Vc (winding swapped when its normal points the other way), applied to the support vertices of
+// A and B (pa, pb, pc: index on A | index on B << 8)
+__device__ __forceinline__ void epa_contact(f3 Va, f3 Vb, f3 Vc, int pa, int pb, int pc, const float4* hA,
+                                            const float4* hB, f3 n, EpaResult& r)
 {
     f3 Pr = n * r.depth;
-    f3 Va = xyz(m.pv[a]), Vb = xyz(m.pv[b]), Vc = xyz(m.pv[c]);
     f3 v0 = Vb - Va, v1 = Vc - Va, v2 = Pr - Va;
     if (dot(cross(v0, v1), n) < 0.f) {
         v0 = Vc - Va;
@@ -651,7 +400,6 @@ __device__ __forceinline__ void epa_contact(const EpaMem& m, const float4* hA, c
     float bv = (v11 * v20 - v01 * v21) / den;
     float bw = (v00 * v21 - v01 * v20) / den;
     float bu = one_minus_two(bw, bv);
-    int pa = m.pab[a], pb = m.pab[b], pc = m.pab[c];
     r.fa[0] = pa & 0xff; r.fa[1] = pb & 0xff; r.fa[2] = pc & 0xff;
     r.fb[0] = pa >> 8; r.fb[1] = pb >> 8; r.fb[2] = pc >> 8;
     r.cpA = (xyz(hA[r.fa[0]]) * bu + xyz(hA[r.fa[1]]) * bv) + xyz(hA[r.fa[2]]) * bw;
@@ -659,196 +407,350 @@ __device__ __forceinline__ void epa_contact(const EpaMem& m, const float4* hA, c
     r.n = n;
 }
 
-template <int LPP>
-__device__ __forceinline__ EpaResult epa_compacting(const Group<LPP>& g, EpaMem* mp, const float4* hA, int nA,
-                                                    const float4* hB, int nB, f3 S1, int a1, int b1, f3 S2, int a2,
-                                                    int b2, f3 S3, int a3, int b3, f3 S4, int a4, int b4, Work3* wkp)
+// ------------------------------------------------------------------ EPA by one warp
+//
+// One pair per warp, laid out for the length of an iteration's dependent chain, which sets the time of
+// a step with a few thousand contacts (its longest EPA runs 25 iterations): each lane keeps its
+// hull vertices and its faces of the append-only list (face f in lane f % 32, slot f / 32) in
+// registers, so a support query, the minimum search and the visibility test read no memory; the new
+// faces are computed in the lanes that will hold them.  Shared memory holds what is looked up by index:
+// the polytope's vertices and a copy of the faces.  The forces wait until the warp has up to 32 of them,
+// one per lane.
+//
+// Against groups of 8, 16 or 32 lanes with the polytope in shared memory, which it replaces: an iteration
+// alone on its scheduler 3,300 cycles (of about 560 instructions, mostly waiting for their fetch);
+// the pass on 3,001 random pairs 122 -> 50 us (8 lanes before), on four steps of 5,003 packed hulls
+// 122 -> 56 us each (8 lanes and the rerun of the overflowing pairs), on 30,011 packed hulls 83 -> 70 us
+// (32 lanes), on 2M random pairs 9.05 -> 7.6 ms (16 lanes), where it issues on 71% of the cycles.
+
+// the two hulls over a warp: lanes 0-15 hold A's vertices, lanes 16-31 B's, `per` consecutive ones each
+// (NaN past the end: such a product never wins)
+struct WarpHulls {
+    const float4 *hA, *hB;
+    int nA, nB, per;
+    float x[4], y[4], z[4];
+    __device__ __forceinline__ void load(const float4* a, int na, const float4* b, int nb)
+    {
+        hA = a;
+        hB = b;
+        nA = na;
+        nB = nb;
+        per = (max(na, nb) + 15) >> 4;
+        const int lane = threadIdx.x & 31;
+        const float4* h = lane < 16 ? a : b;
+        const int n = lane < 16 ? na : nb, first = (lane & 15) * per;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float4 v = make_float4(__int_as_float(0x7fffffff), 0.f, 0.f, 0.f);
+            if (j < per && first + j < n) v = h[first + j];
+            x[j] = v.x;
+            y[j] = v.y;
+            z[j] = v.z;
+        }
+    }
+};
+static_assert(MWD_HULL_CAP <= 64, "four vertices per lane");
+
+// support() by a warp: each half's largest product, then the smallest index among the lanes that hold it
+__device__ __forceinline__ void support_warp(const WarpHulls& h, f3 d, f3& s, int& ia, int& ib)
 {
-    constexpr int SLOT = FCAP - 1;   // the earliest-created removed face
-    constexpr int LIVE = FCAP - 1;   // capacity of the live list
-    constexpr uint32_t NONE = 0xffffffffu;
-    EpaMem& m = *mp;
-    Work3 wk = *wkp;
-    EpaResult r;
+    const int lane = threadIdx.x & 31;
+    const bool onB = lane >= 16;
+    const f3 e = onB ? d * (-1.f) : d;
+    float best = -1e30f;
+    int at = -1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j < h.per) {
+            const float t = e.x * h.x[j] + e.y * h.y[j] + e.z * h.z[j];
+            if (t > best) { best = t; at = j; }
+        }
+    }
+    const unsigned k = fkey(best);
+    const unsigned kA = __reduce_max_sync(0xffffffffu, onB ? 0u : k);
+    const unsigned kB = __reduce_max_sync(0xffffffffu, onB ? k : 0u);
+    const unsigned idx = at < 0 ? 0u : (unsigned)((lane & 15) * h.per + at);
+    ia = (int)__reduce_min_sync(0xffffffffu, !onB && k == kA ? idx : 0xffffu);
+    ib = (int)__reduce_min_sync(0xffffffffu, onB && k == kB ? idx : 0xffffu);
+    const float4 a = h.hA[ia], b = h.hB[ib];
+    s = mk3(a.x - b.x, a.y - b.y, a.z - b.z);
+}
+
+constexpr uint32_t FACE_LIVE = 0x80000000u;
+constexpr int FACE_SLOTS = FCAP / 32;
+
+struct WarpEpaMem {
+    float4 fn[FCAP];      // face normal xyz, distance (3e20 once removed)
+    float4 pv[VCAP];      // polytope vertices
+    uint32_t ft[FCAP];    // vertices T0 | T1 << 8 | T2 << 16, FACE_LIVE
+    uint32_t del[FCAP];   // faces removed in this iteration, in index order
+    uint16_t edge[FCAP];  // horizon edges, first vertex | second << 8
+    uint16_t mark[VCAP * VCAP];  // by unordered vertex pair: the removed faces' edge that has it
+    uint16_t pab[VCAP];   // support index on A | on B << 8
+};
+
+// AddTriangle (.cu:270-325) for the face a, b, c: its normal and distance (1e30 when the origin's
+// projection falls outside it); flip: its winding is a, c, b
+__device__ __forceinline__ float4 face_plane(f3 a, f3 b, f3 c, bool& flip)
+{
+    f3 n = cross(b - a, c - b);
+    n = n / sqrtf(n.x * n.x + n.y * n.y + n.z * n.z);
+    float dist = dot(n, a);
+    flip = dist < 0.f;
+    if (flip) {
+        const f3 t = b;
+        b = c;
+        c = t;
+        dist = dist * (-1.f);
+        n = n * (-1.f);
+    }
+    // (the reference's dot(., -a) < 0: the negated product is exact)
+    const float ia = dot(cross(b - a, n), a), ib = dot(cross(c - b, n), b), ic = dot(cross(a - c, n), c);
+    return f4(n, ia > 0.f && ib > 0.f && ic > 0.f ? dist : 1e30f);
+}
+
+struct WarpEpaOut {
+    float4 face;      // the final face's normal; w: depth
+    uint32_t t;       // its vertices in the polytope
+    uint32_t status;
+    int faces, queries;  // faces created, support queries
+};
+
+// EPA (.cu:328-603).  The list is append-only like the reference's: a removed face stays at distance
+// 3e20 (.cu:541-542), where the first of them can still win the minimum search (.cu:41-53).  When the
+// list is full the removed faces are dropped from it, the first one excepted, in order.
+__device__ __forceinline__ void epa_warp(WarpEpaMem& m, const WarpHulls& h, f3 S1, int a1, int b1, f3 S2, int a2,
+                                         int b2, f3 S3, int a3, int b3, f3 S4, int a4, int b4, WarpEpaOut& r)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    const int lane_face = lane / 3, lane_edge = lane % 3;  // of the first 32 edges of the removed faces
+    constexpr unsigned ALL = 0xffffffffu;
+    const float nan = __int_as_float(0x7fffffff);
     r.status = 0;
-    g.sync();
-    if (g.lane == 0) {
+    __syncwarp();
+    if (lane == 0) {
         m.pv[0] = f4(S1, 0.f); m.pv[1] = f4(S2, 0.f); m.pv[2] = f4(S3, 0.f); m.pv[3] = f4(S4, 0.f);
         m.pab[0] = (uint16_t)(a1 | (b1 << 8)); m.pab[1] = (uint16_t)(a2 | (b2 << 8));
         m.pab[2] = (uint16_t)(a3 | (b3 << 8)); m.pab[3] = (uint16_t)(a4 | (b4 << 8));
     }
-    g.sync();
-    if (g.lane < 4) {
-        const unsigned long long e = 0x310302321210ull >> (12 * g.lane);
-        const int e0 = (int)(e & 0xf), e1 = (int)((e >> 4) & 0xf), e2 = (int)((e >> 8) & 0xf);
-        int t1, t2, valid;
-        m.fn[g.lane] = face_geom(m, e0, e1, e2, t1, t2, valid);
-        m.ft[g.lane] = fc_make(e0, t1, t2, valid, (uint32_t)g.lane);
+    // this lane's faces: normal, distance (NaN: no face), first vertex, vertex numbers
+    f3 fn[FACE_SLOTS], f0[FACE_SLOTS];
+    float fd[FACE_SLOTS];
+    uint32_t ft[FACE_SLOTS];
+#pragma unroll
+    for (int s = 0; s < FACE_SLOTS; ++s) {
+        fn[s] = f0[s] = mk3(0.f, 0.f, 0.f);
+        fd[s] = nan;
+        ft[s] = 0;
     }
-    g.sync();
-    wk.faces += 4;
+    // face f of (0,1,2), (1,2,3), (2,0,3), (0,1,3) in lane f
+    if (lane < 4) {
+        const f3 a = lane == 1 ? S2 : lane == 2 ? S3 : S1;
+        const f3 b = lane == 1 ? S3 : lane == 2 ? S1 : S2;
+        const f3 c = lane == 0 ? S3 : S4;
+        const uint32_t e = lane == 0 ? 0x020100u : lane == 1 ? 0x030201u : lane == 2 ? 0x030002u : 0x030100u;
+        bool flip;
+        const float4 p = face_plane(a, b, c, flip);
+        fn[0] = xyz(p);
+        fd[0] = p.w;
+        f0[0] = a;
+        ft[0] = (flip ? (e & 0xffu) | ((e >> 8) & 0xff00u) | ((e & 0xff00u) << 8) : e) | FACE_LIVE;
+        m.fn[lane] = p;
+        m.ft[lane] = ft[0];
+    }
+    __syncwarp();
     int nt = 4, nv = 4, counter = 0;
-    uint32_t created = 4;
-    uint32_t del_c = NONE;  // creation index of the face in the slot (NONE: none removed yet)
-    const int lane0 = (int)(threadIdx.x & 31) - g.lane;
+    r.faces = 4;
+    r.queries = 0;
     float xmin_old = 1e29f;
     float proj = 2 * xmin_old + 1;
-    float xmin_new = 0.f;
-    float4 fm = make_float4(0.f, 0.f, 0.f, 0.f);  // the face chosen last, and its vertex word
+    float4 fm = make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t tm = 0;
     while (xmin_old < proj) {
-        float bv = __int_as_float(0x7fffffff);
-        int bi = 0x7fffffff;
-        for (int f = g.lane; f < nt; f += LPP) {
-            float v = m.fn[f].w;
-            if (min_better(v, f, bv, bi)) { bv = v; bi = f; }
+        // first index of the minimum distance (NaN never wins, except in face 0, where the search starts)
+        float bv = fd[0];
+        int bs = 0;
+#pragma unroll
+        for (int s = 1; s < FACE_SLOTS; ++s) {
+            if (32 * s < nt && (fd[s] < bv || bv != bv)) { bv = fd[s]; bs = s; }
         }
-        {
-            const unsigned k = (bv != bv) ? 0xffffffffu : fkey(bv);
-            const unsigned km = __reduce_min_sync(g.mask, k);
-            bi = (int)__reduce_min_sync(g.mask, k == km ? (unsigned)bi : 0xffffffffu);
-        }
-        // the removed faces (all at 3e20) are represented by the earliest created of them
-        bool use_slot = false;
-        if (del_c != NONE) {
-            if (bi == 0x7fffffff) use_slot = true;
-            else {
-                const float lv = m.fn[bi].w;
-                use_slot = lv > 3e20f || (lv == 3e20f && del_c < fc_created(m.ft[bi]));
-            }
-        }
-        // the search starts from face 0's distance: a NaN there keeps face 0
-        if (nt > 0 && fc_created(m.ft[0]) == 0 && m.fn[0].w != m.fn[0].w) {
-            use_slot = false;
-            bi = 0;
-        }
-        fm = use_slot ? m.fn[SLOT] : m.fn[bi];
-        tm = use_slot ? m.ft[SLOT] : m.ft[bi];
-        xmin_new = fm.w;
-        xmin_old = xmin_new;
-        f3 n = xyz(fm);
-        f3 s;
+        unsigned k = bv != bv ? 0xffffffffu : fkey(bv);
+        if (lane == 0 && fd[0] != fd[0]) { k = 0u; bs = 0; }
+        const unsigned km = __reduce_min_sync(ALL, k);
+        const int bi = (int)__reduce_min_sync(ALL, k == km ? (unsigned)(32 * bs + lane) : 0x7fffffffu);
+        fm = m.fn[bi];
+        tm = m.ft[bi];
+        xmin_old = fm.w;
+        const f3 n = xyz(fm);
+        f3 sp;
         int sa, sb;
-        support<LPP>(g, hA, nA, hB, nB, n, s, sa, sb, wk);
-        proj = dot(n, s);
-        if (xmin_old > proj || epa_converged(xmin_old, proj)) break;
+        support_warp(h, n, sp, sa, sb);
+        r.queries += 1;
+        proj = dot(n, sp);
+        if (epa_stops(xmin_old, proj)) break;
         if (counter > 49) { r.status |= MWD_ST_EPA_NOCONV; break; }
         counter = counter + 1;
         if (nv >= VCAP) { r.status |= MWD_ST_EPA_OVERFLOW; break; }
-        g.sync();
-        if (g.lane == 0) {
-            m.pv[nv] = f4(s, 0.f);
+        if (lane == 0) {
+            m.pv[nv] = f4(sp, 0.f);
             m.pab[nv] = (uint16_t)(sa | (sb << 8));
         }
         nv++;
-        // faces the new vertex sees are deleted, collected in list order; the others move down
-        int ndel = 0, nkeep = 0;
-        for (int base = 0; base < nt; base += LPP) {
-            const int f = base + g.lane;
-            bool dead = false, live = false;
-            float4 fv = make_float4(0.f, 0.f, 0.f, 0.f);
-            uint32_t t = 0;
-            if (f < nt) {
-                fv = m.fn[f];
-                t = m.ft[f];
-                dead = dot(s - xyz(m.pv[fc_v(t, 0)]), xyz(fv)) >= 0.f;
-                live = !dead;
-            }
-            const unsigned bd = g.ballot(dead), bl = g.ballot(live);
-            g.sync();
-            if (dead)
-                m.del[ndel + __popc(bd & g.lt_mask())] = (uint32_t)fc_v(t, 0) | ((uint32_t)fc_v(t, 1) << 8) |
-                                                         ((uint32_t)fc_v(t, 2) << 16);
-            if (live) {
-                const int o = nkeep + __popc(bl & g.lt_mask());
-                if (o != f) {
-                    m.fn[o] = fv;
-                    m.ft[o] = t;
+        // faces that the new vertex sees are removed, collected in index order
+        int ndel = 0;
+#pragma unroll
+        for (int s = 0; s < FACE_SLOTS; ++s) {
+            if (32 * s < nt) {
+                const bool dead = (ft[s] & FACE_LIVE) && dot(sp - f0[s], fn[s]) >= 0.f;
+                const unsigned b = __ballot_sync(ALL, dead);
+                if (dead) {
+                    m.del[ndel + __popc(b & lt)] = ft[s];
+                    ft[s] &= ~FACE_LIVE;
+                    fd[s] = 3e20f;
+                    m.fn[32 * s + lane].w = 3e20f;
                 }
+                ndel += __popc(b);
             }
-            if (bd && ndel == 0) {
-                // the first face deleted in this iteration is the earliest created of them
-                const int fl = __ffs(bd) - 1;
-                const uint32_t c0 = (uint32_t)__shfl_sync(g.mask, (int)fc_created(t), lane0 + fl);
-                if (c0 < del_c) {
-                    if (g.lane == fl) {
-                        m.fn[SLOT] = make_float4(fv.x, fv.y, fv.z, 3e20f);
-                        m.ft[SLOT] = (t & ~((uint32_t)3 << 15)) | ((uint32_t)(0 + 2) << 15);
-                    }
-                    del_c = c0;
-                }
-            }
-            ndel += __popc(bd);
-            nkeep += __popc(bl);
         }
-        g.sync();
-        // horizon edges, as in epa (.cu:482-544); the new faces follow the survivors
+        __syncwarp();
+        // horizon edges of the removed faces, in face order then edge order (0,1),(1,2),(2,0); an edge is
+        // kept when fewer than two delpair increments land on it (.cu:482-544), i.e. when its unordered
+        // vertex pair occurs once among the removed faces' edges (a face's vertices are distinct).  Every
+        // edge marks its pair with its number; one that finds another's number there spoils the mark; an
+        // edge that still finds its own is alone.  (A match over the warp takes 390 cycles on this GPU;
+        // comparing the lanes' pairs by exchanges took a quarter of the EPA's instructions.)
         int nnew = 0;
-        for (int base = 0; base < 3 * ndel; base += LPP) {
-            int c = base + g.lane;
-            bool keep = false;
-            int e0 = 0, e1 = 0;
-            if (c < 3 * ndel) {
-                uint32_t t = m.del[c / 3];
-                int k = c % 3;
-                e0 = ft_v(t, k);
-                e1 = ft_v(t, k == 2 ? 0 : k + 1);
-                int cnt = 0;
-                for (int j = 0; j < ndel; ++j) {
-                    uint32_t u = m.del[j];
-                    int x = ft_v(u, 0), y = ft_v(u, 1), z = ft_v(u, 2);
-                    cnt += (e0 == y && e1 == x) + (e0 == x && e1 == y) + (e0 == z && e1 == y) +
-                           (e0 == y && e1 == z) + (e0 == x && e1 == z) + (e0 == z && e1 == x);
-                }
-                keep = cnt < 2;
+        const int edges = 3 * ndel;
+        auto edge_of = [&](int c, int& e0, int& e1) {
+            const int f = c < 32 ? lane_face : c / 3;
+            const int j = c < 32 ? lane_edge : c - 3 * f;
+            const uint32_t t = m.del[f];
+            e0 = (int)((t >> (8 * j)) & 0xffu);
+            e1 = (int)((t >> (j == 2 ? 0 : 8 * j + 8)) & 0xffu);
+            return min(e0, e1) * VCAP + max(e0, e1);
+        };
+        if (edges <= 32) {
+            const bool has = lane < edges;
+            int e0 = 0, e1 = 0, code = 0;
+            if (has) {
+                code = edge_of(lane, e0, e1);
+                m.mark[code] = (uint16_t)lane;
             }
-            unsigned b = g.ballot(keep);
-            if (keep) {
-                const int q = nnew + __popc(b & g.lt_mask());
-                const int f = nkeep + q;
-                if (f < LIVE) {
-                    int t1, t2, valid;
-                    m.fn[f] = face_geom(m, e0, e1, nv - 1, t1, t2, valid);
-                    m.ft[f] = fc_make(e0, t1, t2, valid, created + (uint32_t)q);
-                }
+            __syncwarp();
+            if (has && m.mark[code] != lane) m.mark[code] = 0xffffu;
+            __syncwarp();
+            const bool keep = has && m.mark[code] == lane;
+            const unsigned b = __ballot_sync(ALL, keep);
+            if (keep) m.edge[__popc(b & lt)] = (uint16_t)(e0 | (e1 << 8));
+            nnew = __popc(b);
+        } else {
+            int e0, e1;
+            for (int c = lane; c < edges; c += 32) m.mark[edge_of(c, e0, e1)] = (uint16_t)c;
+            __syncwarp();
+            for (int c = lane; c < edges; c += 32) {
+                const int code = edge_of(c, e0, e1);
+                if (m.mark[code] != c) m.mark[code] = 0xffffu;
             }
-            nnew += __popc(b);
+            __syncwarp();
+            for (int base = 0; base < edges; base += 32) {
+                const int c = base + lane;
+                const bool keep = c < edges && m.mark[edge_of(c, e0, e1)] == c;
+                const unsigned b = __ballot_sync(ALL, keep);
+                const int q = nnew + __popc(b & lt);
+                if (keep && q < FCAP) m.edge[q] = (uint16_t)(e0 | (e1 << 8));
+                nnew += __popc(b);
+            }
         }
-        g.sync();
-        if (nkeep + nnew > LIVE) { r.status |= MWD_ST_EPA_OVERFLOW; break; }
-        nt = nkeep + nnew;
-        created += (uint32_t)nnew;
-        wk.faces += (uint32_t)nnew;
+        __syncwarp();
+        if (nt + nnew > FCAP) {
+            // the list is full (about one deep overlap in 120,000 of random hulls, some contacts of every
+            // step of packed hulls or cubes): drop the removed faces, the first one excepted.  At most
+            // 2 * 30 - 4 = 56 faces of a closed polytope are alive within the reference's iteration limit.
+            int kept = 0;
+            bool first = true;
+#pragma unroll
+            for (int s = 0; s < FACE_SLOTS; ++s) {
+                const bool in = 32 * s + lane < nt;
+                const unsigned gone = __ballot_sync(ALL, in && !(ft[s] & FACE_LIVE));
+                const bool keep = in && ((ft[s] & FACE_LIVE) || (first && lane == __ffs(gone) - 1));
+                if (gone) first = false;
+                const unsigned b = __ballot_sync(ALL, keep);
+                if (keep) {
+                    const int o = kept + __popc(b & lt);
+                    m.fn[o] = f4(fn[s], fd[s]);
+                    m.ft[o] = ft[s];
+                }
+                kept += __popc(b);
+            }
+            __syncwarp();
+            nt = kept;
+#pragma unroll
+            for (int s = 0; s < FACE_SLOTS; ++s) {
+                fd[s] = nan;
+                ft[s] = 0;
+                if (32 * s + lane < nt) {
+                    const float4 p = m.fn[32 * s + lane];
+                    ft[s] = m.ft[32 * s + lane];
+                    fn[s] = xyz(p);
+                    fd[s] = p.w;
+                    f0[s] = xyz(m.pv[ft_v(ft[s], 0)]);
+                }
+            }
+            __syncwarp();
+            if (nt + nnew > FCAP) { r.status |= MWD_ST_EPA_OVERFLOW; break; }
+        }
+        // the new faces (edge q, new vertex) at list positions nt + q, each in the lane that holds it
+        for (int q0 = 0; q0 < nnew; q0 += 32) {
+            const int q = q0 + ((lane - nt - q0) & 31);
+            const int pos = q < nnew ? nt + q : -1;
+            f3 a = mk3(0.f, 0.f, 0.f);
+            float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+            uint32_t t = 0;
+            if (pos >= 0) {
+                const uint32_t e = m.edge[q];
+                const uint32_t e0 = e & 0xffu, e1 = e >> 8, e2 = (uint32_t)(nv - 1);
+                a = xyz(m.pv[e0]);
+                bool flip;
+                p = face_plane(a, xyz(m.pv[e1]), sp, flip);
+                t = e0 | (flip ? (e2 << 8) | (e1 << 16) : (e1 << 8) | (e2 << 16)) | FACE_LIVE;
+                m.fn[pos] = p;
+                m.ft[pos] = t;
+            }
+            const int s0 = (nt + q0) >> 5;  // the 32 positions lie in slots s0 and s0 + 1
+#pragma unroll
+            for (int s = 0; s < FACE_SLOTS; ++s) {
+                if (s != s0 && s != s0 + 1) continue;
+                const bool here = (pos >> 5) == s;  // selects, so that the arrays stay in registers
+                fn[s].x = here ? p.x : fn[s].x;
+                fn[s].y = here ? p.y : fn[s].y;
+                fn[s].z = here ? p.z : fn[s].z;
+                fd[s] = here ? p.w : fd[s];
+                f0[s].x = here ? a.x : f0[s].x;
+                f0[s].y = here ? a.y : f0[s].y;
+                f0[s].z = here ? a.z : f0[s].z;
+                ft[s] = here ? t : ft[s];
+            }
+        }
+        nt += nnew;
+        r.faces += nnew;
         counter = counter + 1;
+        __syncwarp();
     }
-    g.sync();
-    r.depth = xmin_new;
-    *wkp = wk;
-    if (g.lane == 0) epa_contact(m, hA, hB, xyz(fm), fc_v(tm, 0), fc_v(tm, 1), fc_v(tm, 2), r);
-    return r;
+    r.face = make_float4(fm.x, fm.y, fm.z, fm.w);
+    r.t = tm;
 }
 
-template <int LPP>
-__device__ __noinline__ EpaResult epa_compacting_call(const Group<LPP> g, EpaMem* mp, const float4* hA, int nA,
-                                                      const float4* hB, int nB, f3 S1, int a1, int b1, f3 S2, int a2,
-                                                      int b2, f3 S3, int a3, int b3, f3 S4, int a4, int b4, Work3* wkp)
+// CorrectFlat (.cu:256-268) and EPA from the simplex GJK stopped on (ia, ib: its support indices, 8 bits each)
+__device__ __forceinline__ void epa_from_simplex(WarpEpaMem& m, const WarpHulls& h, f3 S1, f3 S2, f3 S3, f3 S4,
+                                                 uint32_t ia, uint32_t ib, WarpEpaOut& r)
 {
-    return epa_compacting<LPP>(g, mp, hA, nA, hB, nB, S1, a1, b1, S2, a2, b2, S3, a3, b3, S4, a4, b4, wkp);
-}
-
-// EPA of one pair in the single-pass kernel: the append-only list, and for the rare pair that outgrows
-// it, the compacting one (its work counted once: the first attempt's is dropped)
-template <int LPP>
-__device__ __forceinline__ void epa_run(const Group<LPP>& g, EpaMem& m, const float4* hA, int nA, const float4* hB,
-                                        int nB, f3 S1, int a1, int b1, f3 S2, int a2, int b2, f3 S3, int a3, int b3,
-                                        f3 S4, int a4, int b4, EpaResult& r, Work3& wk)
-{
-    const Work3 w0 = wk;
-    epa<LPP>(g, m, hA, nA, hB, nB, S1, a1, b1, S2, a2, b2, S3, a3, b3, S4, a4, b4, r, wk);
-    if (r.status & MWD_ST_EPA_OVERFLOW) {
-        wk = w0;
-        r = epa_compacting_call<LPP>(g, &m, hA, nA, hB, nB, S1, a1, b1, S2, a2, b2, S3, a3, b3, S4, a4, b4, &wk);
-    }
+    int a4 = ia >> 24, b4 = ib >> 24;
+    const bool flat = is_flat(S1, S2, S3, S4);
+    if (flat) support_warp(h, cross(S1, S2), S4, a4, b4);
+    epa_warp(m, h, S1, ia & 0xff, ib & 0xff, S2, (ia >> 8) & 0xff, (ib >> 8) & 0xff, S3, (ia >> 16) & 0xff,
+             (ib >> 16) & 0xff, S4, a4, b4, r);
+    r.queries += flat ? 1 : 0;
 }
 
 struct ForceResult {
@@ -1054,182 +956,6 @@ __device__ __forceinline__ void accumulate(const NarrowArgs& a, const PairView& 
     }
 }
 
-template <int LPP, int MODE>
-__device__ void process_pair(const NarrowArgs& a, int64_t P, const Group<LPP>& g, EpaMem& em, float4* hA, float4* hB)
-{
-    PairView p;
-    const bool ok = load_pair<MODE>(a, P, p, hA, hB, g.lane, LPP);
-    g.sync();
-    const bool leader = g.lane == 0;
-    if (!ok) {
-        if (leader) {
-            set_status(a.status, MWD_ST_BAD_SHAPE);
-            if (a.collision) a.collision[P] = -1;
-        }
-        return;
-    }
-    const mwd_material& M = MODE == 0 ? a.mat[p.wall] : a.scenes[a.st.info[p.idA] >> 1].mat[p.wall];
-
-    Work3 wk = {0u, 0u, 0u};
-    f3 S1, S2, S3, S4, d3, d4;
-    int a1, b1, a2, b2, a3, b3, a4 = 0, b4 = 0, todel = 0, coll = -1;
-    bool early = false, resolved = false;
-    f3 d1 = p.cB - p.cA;
-    support<LPP>(g, hA, p.nA, hB, p.nB, d1, S1, a1, b1, wk);
-    if (dot(d1, S1) < 0.f) early = true;
-    if (!early) {
-        f3 d2 = d1 * (-1.f);
-        support<LPP>(g, hA, p.nA, hB, p.nB, d2, S2, a2, b2, wk);
-        if (dot(d2, S2) < 0.f) early = true;
-    }
-    if (!early) {
-        seg_test(S1, S2, coll, d3);
-        if (coll == 0) early = true;
-    }
-    if (!early) {
-        support<LPP>(g, hA, p.nA, hB, p.nB, d3, S3, a3, b3, wk);
-        if (dot(d3, S3) < 0.f) early = true;
-    }
-    if (!early) {
-        tri_test(S1, S2, S3, coll, d4);
-        if (coll == 0) early = true;
-    }
-    ForceResult fo;
-    fo.F = fo.TA = fo.TB = mk3(0.f, 0.f, 0.f);
-    fo.dt = p.dt;
-    EpaResult er;
-    er.status = 0;
-    uint32_t st = 0;
-    if (!early) {
-        int zz = 0;
-        while (zz < 50) {
-            support<LPP>(g, hA, p.nA, hB, p.nB, d4, S4, a4, b4, wk);
-            if (dot(d4, S4) < 0.f) { early = true; break; }
-            bool hit = false;
-            if (S4.x == 0.f && S4.y == 0.f && S4.z == 0.f) hit = true;
-            else {
-                tet_test(S1, S2, S3, S4, coll, d4, todel);
-                if (coll == 0) { early = true; break; }
-                if (coll == 1) hit = true;
-            }
-            if (hit) {
-                if (is_flat(S1, S2, S3, S4)) {
-                    d4 = cross(S1, S2);
-                    support<LPP>(g, hA, p.nA, hB, p.nB, d4, S4, a4, b4, wk);
-                }
-                epa_run<LPP>(g, em, hA, p.nA, hB, p.nB, S1, a1, b1, S2, a2, b2, S3, a3, b3, S4, a4, b4, er, wk);
-                if (leader) {
-                    float imA, imB;
-                    pair_inv_mass<MODE>(a, p, M, imA, imB);
-                    contact_force(p.cA, p.cB, er.depth, er.n, er.cpA, er.cpB, M, p.vA, p.vB, p.wA, p.wB, p.dt,
-                                  p.qA, p.dtn, p.IsA, p.IsB, imA, imB, fo);
-                }
-                st |= er.status;
-                resolved = true;
-                break;
-            }
-            f3 n1, n2, n3;
-            int na1, nb1, na2, nb2, na3, nb3;
-            if (todel == 1) { n1 = S2; na1 = a2; nb1 = b2; n2 = S3; na2 = a3; nb2 = b3; n3 = S4; na3 = a4; nb3 = b4; }
-            else if (todel == 2) { n1 = S3; na1 = a3; nb1 = b3; n2 = S1; na2 = a1; nb2 = b1; n3 = S4; na3 = a4; nb3 = b4; }
-            else { n1 = S1; na1 = a1; nb1 = b1; n2 = S2; na2 = a2; nb2 = b2; n3 = S4; na3 = a4; nb3 = b4; }
-            S1 = n1; a1 = na1; b1 = nb1; S2 = n2; a2 = na2; b2 = nb2; S3 = n3; a3 = na3; b3 = nb3;
-            zz = zz + 1;
-        }
-        if (!early && !resolved) st |= MWD_ST_GJK_NOCONV;
-    }
-    if (!leader) return;
-    set_status(a.status, st);
-    if (a.work_counters) {
-        atomicAdd(a.work_counters + 0, (unsigned long long)wk.dots);
-        atomicAdd(a.work_counters + 1, (unsigned long long)wk.faces);
-        atomicAdd(a.work_counters + 2, (unsigned long long)wk.queries);
-    }
-    if (early) {
-        if (a.collision) a.collision[P] = 0;
-        write_hist<MODE>(a, P, mk3(0.f, 0.f, 0.f), 0.f);
-    } else {
-        if (a.collision) a.collision[P] = resolved ? 1 : -1;
-        if (resolved) write_hist<MODE>(a, P, fo.dt, 1.f);
-        accumulate<MODE>(a, p, fo);
-    }
-    if (a.diag) {
-        float* dg = a.diag + 10 * P;
-        if (resolved) {
-            dg[0] = er.depth;
-            dg[1] = er.n.x; dg[2] = er.n.y; dg[3] = er.n.z;
-            dg[4] = er.cpA.x; dg[5] = er.cpA.y; dg[6] = er.cpA.z;
-            dg[7] = er.cpB.x; dg[8] = er.cpB.y; dg[9] = er.cpB.z;
-        } else {
-            for (int k = 0; k < 10; ++k) dg[k] = 0.f;
-        }
-    }
-    if (a.face_ids) {
-        int* fid = a.face_ids + 6 * P;
-        for (int k = 0; k < 3; ++k) {
-            fid[k] = resolved ? er.fa[k] : -1;
-            fid[3 + k] = resolved ? er.fb[k] : -1;
-        }
-    }
-}
-
-template <int LPP, int MODE>
-__global__ void __launch_bounds__(NARROW_THREADS) narrow_kernel(NarrowArgs a)
-{
-    extern __shared__ float4 smem[];
-    constexpr int GPB = NARROW_THREADS / LPP;
-    const int grp = threadIdx.x / LPP;
-    Group<LPP> g;
-    g.lane = threadIdx.x % LPP;
-    g.mask = LPP == 32 ? 0xffffffffu : (((1u << LPP) - 1u) << ((threadIdx.x & 31) / LPP * LPP));
-    EpaMem* em = reinterpret_cast<EpaMem*>(smem) + grp;
-    float4* hull = reinterpret_cast<float4*>(reinterpret_cast<EpaMem*>(smem) + GPB) + (size_t)grp * 2 * a.hull_cap;
-    float4* hA = hull;
-    float4* hB = hull + a.hull_cap;
-    int64_t n = a.n_pairs;
-    if (MODE == 1) {
-        int64_t m = *a.n_pairs_dev;
-        n = m < a.pair_cap ? m : a.pair_cap;
-    }
-    if (MODE == 1) {
-        // sphere pre-test (spheres_apart), LPP candidate pairs at a time (one per lane); pairs it
-        // settles get the reference's outcome (collision 0, no force) without running GJK
-        const double4* pos = reinterpret_cast<const double4*>(a.st.pos);
-        const int2* pairs = reinterpret_cast<const int2*>(a.pairs);
-        const int64_t stride = (int64_t)gridDim.x * GPB * LPP;
-        for (int64_t base = ((int64_t)blockIdx.x * GPB + grp) * LPP; base < n; base += stride) {
-            const int64_t Pl = base + g.lane;
-            bool live = false;
-            if (Pl < n) {
-                const int2 pr = pairs[Pl];
-                live = !spheres_apart(pos[pr.x], pos[pr.y]);
-                if (!live && a.collision) a.collision[Pl] = 0;
-            }
-            unsigned m = g.ballot(live);
-            while (m) {
-                const int l = __ffs(m) - 1;
-                m &= m - 1;
-                process_pair<LPP, MODE>(a, base + l, g, *em, hA, hB);
-                g.sync();
-            }
-        }
-        return;
-    }
-    for (int64_t P = (int64_t)blockIdx.x * GPB + grp; P < n; P += (int64_t)gridDim.x * GPB) {
-        process_pair<LPP, MODE>(a, P, g, *em, hA, hB);
-        g.sync();
-    }
-}
-
-// ------------------------------------------------------------------ two-pass narrow phase (table mode)
-//
-// Pass 1 (gjk_pass_kernel) runs the sphere pre-test and GJK on every candidate pair with the hulls
-// read straight from the world-vertex table (no shared memory, few registers, many resident warps);
-// separated and undecided pairs are finished there.  Pairs GJK finds in contact append the simplex
-// it stopped on to a compact list.  Pass 2 (epa_pass_kernel) continues exactly where pass 1
-// stopped -- CorrectFlat, EPA, force -- for the listed pairs only, with the shared-memory polytope.
-// The operation sequence per pair is the single-pass kernel's.
-
 // GJK up to the decision (.cu:996-1288): 0 separated, 1 in contact (simplex in rec), -1 undecided
 // after 50 tetrahedron iterations.
 template <int LPP>
@@ -1278,6 +1004,161 @@ __device__ int gjk_decide(const Group<LPP>& g, const float4* hA, int nA, const f
     }
     return -1;
 }
+
+// ------------------------------------------------------------------ single-pass narrow phase
+// GJK by the groups of a warp, each on its own pair, then EPA by the whole warp on one after another of
+// the pairs they found in contact; the lane that leads a pair's group evaluates its force.
+template <int LPP, int MODE>
+__device__ __forceinline__ void narrow_pairs(const NarrowArgs& a, int64_t P, bool in, const Group<LPP>& g,
+                                             WarpEpaMem& em, float4* hA, float4* hB)
+{
+    const int lane = threadIdx.x & 31;
+    PairView p;
+    Work3 wk = {0u, 0u, 0u};
+    SimplexRec rec;
+    int out = 0;  // 0 separated, 1 in contact, -1 undecided
+    bool ok = false;
+    if (in) {
+        ok = load_pair<MODE>(a, P, p, hA, hB, g.lane, LPP);
+        g.sync();
+        if (ok) out = gjk_decide<LPP>(g, hA, p.nA, hB, p.nB, p.cA, p.cB, rec, wk);
+    }
+    __syncwarp();
+    EpaResult er;
+    er.status = 0;
+    for (unsigned hits = __ballot_sync(0xffffffffu, out == 1 && g.lane == 0); hits; hits &= hits - 1) {
+        const int src = __ffs(hits) - 1;
+        if (lane == src) {
+            for (int k = 0; k < 4; ++k) em.pv[k] = rec.S[k];
+            em.ft[0] = rec.ia;
+            em.ft[1] = rec.ib;
+        }
+        const float4* ha = hA + (src / LPP - lane / LPP) * 2 * a.hull_cap;  // the group's staged hulls
+        WarpHulls h;
+        h.load(ha, __shfl_sync(0xffffffffu, p.nA, src), ha + a.hull_cap, __shfl_sync(0xffffffffu, p.nB, src));
+        __syncwarp();
+        const f3 S1 = xyz(em.pv[0]), S2 = xyz(em.pv[1]), S3 = xyz(em.pv[2]);
+        f3 S4 = xyz(em.pv[3]);
+        const uint32_t ia = em.ft[0], ib = em.ft[1];
+        WarpEpaOut o;
+        epa_from_simplex(em, h, S1, S2, S3, S4, ia, ib, o);
+        if (lane == src) {
+            wk.queries += (uint32_t)o.queries;
+            wk.faces += (uint32_t)o.faces;
+            wk.dots += (uint32_t)o.queries * (uint32_t)(p.nA + p.nB);
+            const int ta = ft_v(o.t, 0), tb = ft_v(o.t, 1), tc = ft_v(o.t, 2);
+            er.status = o.status;
+            er.depth = o.face.w;
+            epa_contact(xyz(em.pv[ta]), xyz(em.pv[tb]), xyz(em.pv[tc]), em.pab[ta], em.pab[tb], em.pab[tc], hA, hB,
+                        xyz(o.face), er);
+        }
+        __syncwarp();
+    }
+    if (!in || g.lane != 0) return;
+    if (!ok) {
+        set_status(a.status, MWD_ST_BAD_SHAPE);
+        if (a.collision) a.collision[P] = -1;
+        return;
+    }
+    const bool resolved = out == 1;
+    ForceResult fo;
+    fo.F = fo.TA = fo.TB = mk3(0.f, 0.f, 0.f);
+    fo.dt = p.dt;
+    if (resolved) {
+        const mwd_material& M = MODE == 0 ? a.mat[p.wall] : a.scenes[a.st.info[p.idA] >> 1].mat[p.wall];
+        float imA, imB;
+        pair_inv_mass<MODE>(a, p, M, imA, imB);
+        contact_force(p.cA, p.cB, er.depth, er.n, er.cpA, er.cpB, M, p.vA, p.vB, p.wA, p.wB, p.dt, p.qA, p.dtn, p.IsA,
+                      p.IsB, imA, imB, fo);
+    }
+    set_status(a.status, out == -1 ? (uint32_t)MWD_ST_GJK_NOCONV : er.status);
+    if (a.work_counters) {
+        atomicAdd(a.work_counters + 0, (unsigned long long)wk.dots);
+        atomicAdd(a.work_counters + 1, (unsigned long long)wk.faces);
+        atomicAdd(a.work_counters + 2, (unsigned long long)wk.queries);
+    }
+    if (a.collision) a.collision[P] = out;
+    if (out == 0) {
+        write_hist<MODE>(a, P, mk3(0.f, 0.f, 0.f), 0.f);
+    } else {
+        if (resolved) write_hist<MODE>(a, P, fo.dt, 1.f);
+        accumulate<MODE>(a, p, fo);
+    }
+    if (a.diag) {
+        float* dg = a.diag + 10 * P;
+        if (resolved) {
+            dg[0] = er.depth;
+            dg[1] = er.n.x; dg[2] = er.n.y; dg[3] = er.n.z;
+            dg[4] = er.cpA.x; dg[5] = er.cpA.y; dg[6] = er.cpA.z;
+            dg[7] = er.cpB.x; dg[8] = er.cpB.y; dg[9] = er.cpB.z;
+        } else {
+            for (int k = 0; k < 10; ++k) dg[k] = 0.f;
+        }
+    }
+    if (a.face_ids) {
+        int* fid = a.face_ids + 6 * P;
+        for (int k = 0; k < 3; ++k) {
+            fid[k] = resolved ? er.fa[k] : -1;
+            fid[3 + k] = resolved ? er.fb[k] : -1;
+        }
+    }
+}
+
+template <int LPP, int MODE>
+__global__ void __launch_bounds__(NARROW_THREADS) narrow_kernel(NarrowArgs a)
+{
+    extern __shared__ float4 smem[];
+    constexpr int GPB = NARROW_THREADS / LPP;
+    const int grp = threadIdx.x / LPP;
+    Group<LPP> g;
+    g.lane = threadIdx.x % LPP;
+    g.mask = LPP == 32 ? 0xffffffffu : (((1u << LPP) - 1u) << ((threadIdx.x & 31) / LPP * LPP));
+    WarpEpaMem& em = reinterpret_cast<WarpEpaMem*>(smem)[threadIdx.x / 32];
+    float4* hA = reinterpret_cast<float4*>(reinterpret_cast<WarpEpaMem*>(smem) + NARROW_THREADS / 32) +
+                 (size_t)grp * 2 * a.hull_cap;
+    float4* hB = hA + a.hull_cap;
+    int64_t n = a.n_pairs;
+    if (MODE == 1) {
+        int64_t m = *a.n_pairs_dev;
+        n = m < a.pair_cap ? m : a.pair_cap;
+        // sphere pre-test (spheres_apart), LPP candidate pairs at a time per group (one per lane); pairs it
+        // settles get the reference's outcome (collision 0, no force) without running GJK
+        const double4* pos = reinterpret_cast<const double4*>(a.st.pos);
+        const int2* pairs = reinterpret_cast<const int2*>(a.pairs);
+        const int64_t stride = (int64_t)gridDim.x * GPB * LPP;
+        for (int64_t b0 = (int64_t)blockIdx.x * GPB * LPP; b0 < n; b0 += stride) {
+            const int64_t base = b0 + (int64_t)grp * LPP;
+            const int64_t Pl = base + g.lane;
+            bool live = false;
+            if (Pl < n) {
+                const int2 pr = pairs[Pl];
+                live = !spheres_apart(pos[pr.x], pos[pr.y]);
+                if (!live && a.collision) a.collision[Pl] = 0;
+            }
+            unsigned m = g.ballot(live);
+            while (__any_sync(0xffffffffu, m != 0)) {
+                const int l = __ffs(m) - 1;
+                narrow_pairs<LPP, MODE>(a, base + l, m != 0, g, em, hA, hB);
+                m &= m - 1;
+                __syncwarp();
+            }
+        }
+    } else {
+        for (int64_t base = (int64_t)blockIdx.x * GPB; base < n; base += (int64_t)gridDim.x * GPB) {
+            narrow_pairs<LPP, MODE>(a, base + grp, base + grp < n, g, em, hA, hB);
+            __syncwarp();
+        }
+    }
+}
+
+// ------------------------------------------------------------------ two-pass narrow phase (table mode)
+//
+// Pass 1 (gjk_pass_kernel) runs the sphere pre-test and GJK on every candidate pair with the hulls
+// read straight from the world-vertex table (no shared memory, few registers, many resident warps);
+// separated and undecided pairs are finished there.  Pairs GJK finds in contact append the simplex
+// it stopped on to a compact list.  Pass 2 (epa_pass_kernel) continues exactly where pass 1
+// stopped -- CorrectFlat, EPA, force -- for the listed pairs only, with the shared-memory polytope.
+// The operation sequence per pair is the single-pass kernel's.
 
 // GJK on pair P by the group; lane 0 records the outcome (status, contact flag, and for a pair in
 // contact its simplex in the EPA list, whose slot it also appends to *list when list is given)
@@ -1454,168 +1335,154 @@ __global__ void hist_flip_kernel(NarrowArgs a)
     if (threadIdx.x == 0 && blockIdx.x == 0) *a.hist_parity ^= 1;
 }
 
-// CorrectFlat, EPA, force and the outputs for EPA record i, by one group (em: its polytope; hull: its
-// staging area when the hulls are staged).  RETRY: the record's face list overflowed in the EPA pass,
-// run it with the compacting EPA.
-template <int LPP, bool RETRY>
-__device__ __forceinline__ void epa_record(const NarrowArgs& a, const Group<LPP>& g, EpaMem* em, float4* hull,
-                                           int64_t i)
-{
-    const float4* wv = reinterpret_cast<const float4*>(a.st.world_verts);
-    const SimplexRec* recs = reinterpret_cast<const SimplexRec*>(a.epa_rec);
-    const SimplexRec rec = recs[i];
-    const int64_t P = rec.P;
-    // Only the hulls before the EPA: the pair's other inputs are loaded after it, by the lane that
-    // evaluates the force, so that the EPA loop holds fewer registers.  The hulls are staged in shared
-    // memory, or read in place from the (L1-cached) vertex table.  (GJK recorded the pair, so both
-    // hulls fit the staging area.)
-    const int2 pr = reinterpret_cast<const int2*>(a.pairs)[P];
-    const int oa = a.st.vert_off[pr.x], ob = a.st.vert_off[pr.y];
-    const int nA = a.st.vert_off[pr.x + 1] - oa, nB = a.st.vert_off[pr.y + 1] - ob;
-    const float4* hA = hull;
-    const float4* hB = hull + a.hull_cap;
-    if (a.epa_global) {
-        hA = wv + oa;
-        hB = wv + ob;
-    } else {
-        for (int k = g.lane; k < nA; k += LPP) hull[k] = wv[oa + k];
-        for (int k = g.lane; k < nB; k += LPP) hull[a.hull_cap + k] = wv[ob + k];
-    }
-    g.sync();
-    Work3 wk = {0u, 0u, 0u};
-    f3 S1 = xyz(rec.S[0]), S2 = xyz(rec.S[1]), S3 = xyz(rec.S[2]), S4 = xyz(rec.S[3]);
-    int a1 = rec.ia & 0xff, a2 = (rec.ia >> 8) & 0xff, a3 = (rec.ia >> 16) & 0xff, a4 = rec.ia >> 24;
-    int b1 = rec.ib & 0xff, b2 = (rec.ib >> 8) & 0xff, b3 = (rec.ib >> 16) & 0xff, b4 = rec.ib >> 24;
-    if (is_flat(S1, S2, S3, S4)) {
-        f3 d4 = cross(S1, S2);
-        support<LPP>(g, hA, nA, hB, nB, d4, S4, a4, b4, wk);
-    }
-    EpaResult er;
-    if (!RETRY)
-        epa<LPP>(g, *em, hA, nA, hB, nB, S1, a1, b1, S2, a2, b2, S3, a3, b3, S4, a4, b4, er, wk);
-    else
-        er = epa_compacting<LPP>(g, em, hA, nA, hB, nB, S1, a1, b1, S2, a2, b2, S3, a3, b3, S4, a4, b4, &wk);
-    if (g.lane == 0) {
-        bool retry = false;
-        if (!RETRY && (er.status & MWD_ST_EPA_OVERFLOW)) {
-            // the face list outgrew FCAP: the record runs again with the compacting EPA after this
-            // pass (the list of such records permitting; otherwise the truncated result stands, flagged)
-            const int slot = atomicAdd(epa_retry_count(a), 1);
-            if (slot < EPA_RETRY_CAP) {
-                epa_retry_list(a)[slot] = (int32_t)i;
-                retry = true;
-            }
-        }
-        if (!retry) {
-            PairView p;
-            load_pair<1>(a, P, p, nullptr, nullptr, 0, 1, false);
-            if (a.hist_keys) {
-                p.dt = hist_get(a, p.idA, p.idB);
-                p.dtn = sqrtf(p.dt.x * p.dt.x + p.dt.y * p.dt.y + p.dt.z * p.dt.z);
-            }
-            const mwd_material& M = a.scenes[a.st.info[p.idA] >> 1].mat[p.wall];
-            ForceResult fo;
-            float imA, imB;
-            pair_inv_mass<1>(a, p, M, imA, imB);
-            contact_force(p.cA, p.cB, er.depth, er.n, er.cpA, er.cpB, M, p.vA, p.vB, p.wA, p.wB, p.dt, p.qA, p.dtn,
-                          p.IsA, p.IsB, imA, imB, fo);
-            set_status(a.status, er.status);
-            if (a.hist_keys) hist_put(a, p.idA, p.idB, fo.dt);
-            if (a.det_out) {
-                float4* o = a.det_out + 3 * i;
-                o[0] = f4(fo.F, 0.f);
-                o[1] = f4(fo.TA, 0.f);
-                o[2] = f4(fo.TB, 0.f);
-            } else {
-                accumulate<1>(a, p, fo);
-            }
-            if (a.face_ids) {
-                int* fid = a.face_ids + 6 * P;
-                for (int k = 0; k < 3; ++k) {
-                    fid[k] = er.fa[k];
-                    fid[3 + k] = er.fb[k];
-                }
-            }
-            if (a.work_counters) {
-                atomicAdd(a.work_counters + 0, (unsigned long long)wk.dots);
-                atomicAdd(a.work_counters + 1, (unsigned long long)wk.faces);
-                atomicAdd(a.work_counters + 2, (unsigned long long)wk.queries);
-            }
-        }
-    }
-    g.sync();
-}
-
 // the EPA queue's smallest claim, and the fraction of the remaining records per group a claim takes
 constexpr int EPA_CLAIM = 2;
 constexpr int EPA_GUIDE = 4;
 
+// A finished EPA whose force is still to be evaluated: the final face's normal and depth, its three
+// polytope vertices with their support indices, and the record
+struct EpaDone {
+    float4 nd;       // normal, depth
+    float4 a, b, c;  // vertices; w: support indices of a and b, of c and the status bits, the record
+};
+
+// The forces of up to 32 finished records, one per lane
+__device__ __forceinline__ void epa_flush(const NarrowArgs& a, const EpaDone* done, int n)
+{
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    if (lane < n) {
+        const EpaDone e = done[lane];
+        const uint32_t pab = __float_as_uint(e.a.w), pcs = __float_as_uint(e.b.w);
+        const int64_t i = (int64_t)__float_as_uint(e.c.w);
+        const int64_t P = reinterpret_cast<const SimplexRec*>(a.epa_rec)[i].P;
+        PairView p;
+        load_pair<1>(a, P, p, nullptr, nullptr, 0, 1, false);
+        const float4* wv = reinterpret_cast<const float4*>(a.st.world_verts);
+        EpaResult er;
+        er.depth = e.nd.w;
+        epa_contact(xyz(e.a), xyz(e.b), xyz(e.c), (int)(pab & 0xffffu), (int)(pab >> 16), (int)(pcs & 0xffffu),
+                    wv + a.st.vert_off[p.idA], wv + a.st.vert_off[p.idB], xyz(e.nd), er);
+        if (a.hist_keys) {
+            p.dt = hist_get(a, p.idA, p.idB);
+            p.dtn = sqrtf(p.dt.x * p.dt.x + p.dt.y * p.dt.y + p.dt.z * p.dt.z);
+        }
+        const mwd_material& M = a.scenes[a.st.info[p.idA] >> 1].mat[p.wall];
+        ForceResult fo;
+        float imA, imB;
+        pair_inv_mass<1>(a, p, M, imA, imB);
+        contact_force(p.cA, p.cB, er.depth, er.n, er.cpA, er.cpB, M, p.vA, p.vB, p.wA, p.wB, p.dt, p.qA, p.dtn,
+                      p.IsA, p.IsB, imA, imB, fo);
+        set_status(a.status, pcs >> 16);
+        if (a.hist_keys) hist_put(a, p.idA, p.idB, fo.dt);
+        if (a.det_out) {
+            float4* o = a.det_out + 3 * i;
+            o[0] = f4(fo.F, 0.f);
+            o[1] = f4(fo.TA, 0.f);
+            o[2] = f4(fo.TB, 0.f);
+        } else {
+            accumulate<1>(a, p, fo);
+        }
+        if (a.face_ids) {
+            int* fid = a.face_ids + 6 * P;
+            for (int k = 0; k < 3; ++k) {
+                fid[k] = er.fa[k];
+                fid[3 + k] = er.fb[k];
+            }
+        }
+    }
+    __syncwarp();
+}
+
 // BT threads per block, registers capped so that 640 threads per SM stay resident (5 blocks of 128)
-template <int LPP, int BT>
+template <int BT>
 __global__ void __launch_bounds__(BT, 640 / BT) epa_pass_kernel(NarrowArgs a)
 {
     pdl_wait();
     pdl_launch_dependents();
     extern __shared__ float4 smem[];
-    constexpr int GPB = BT / LPP;
-    const int grp = threadIdx.x / LPP;
-    Group<LPP> g;
-    g.lane = threadIdx.x % LPP;
-    g.mask = LPP == 32 ? 0xffffffffu : (((1u << LPP) - 1u) << ((threadIdx.x & 31) / LPP * LPP));
-    EpaMem* em = reinterpret_cast<EpaMem*>(smem) + grp;
-    float4* hull = reinterpret_cast<float4*>(reinterpret_cast<EpaMem*>(smem) + GPB) + (size_t)grp * 2 * a.hull_cap;
+    constexpr int W = BT / 32;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+    WarpEpaMem& em = reinterpret_cast<WarpEpaMem*>(smem)[warp];
+    EpaDone* done = reinterpret_cast<EpaDone*>(reinterpret_cast<WarpEpaMem*>(smem) + W) + 32 * warp;
+    const float4* wv = reinterpret_cast<const float4*>(a.st.world_verts);
+    const SimplexRec* recs = reinterpret_cast<const SimplexRec*>(a.epa_rec);
+    Group<32> g;
+    g.lane = lane;
+    g.mask = 0xffffffffu;
     const int cnt = *a.epa_count;
     const int m = (int64_t)cnt < a.epa_cap ? cnt : (int)a.epa_cap;
-    // Persistent over a work queue (guided self-scheduling): every group first takes a fixed share of
+    // Persistent over a work queue (guided self-scheduling): every warp first takes a fixed share of
     // the records, interleaved with the others' (all of them when there are no more records than
-    // groups: no atomic at all); the rest are claimed from the queue in pieces of a quarter of what is
-    // left per group, so that the groups that finish early take over the work of the others and the
+    // warps: no atomic at all); the rest are claimed from the queue in pieces of a quarter of what is
+    // left per warp, so that the warps that finish early take over the work of the others and the
     // pass ends with its last record rather than with the unluckiest fixed share.  (Record counts are
     // int32.)
-    const int G = (int)gridDim.x * GPB;
+    const int G = (int)gridDim.x * W;
     const int share = m <= G ? 1 : (m / (2 * G) > 1 ? m / (2 * G) : 1);
     const int fixed = m <= G ? m : G * share;
     unsigned long long* next = epa_queue(a);
     // records i, i + step, ... below e: first the fixed share (step G), then each claimed piece (step 1)
-    int i = (int)blockIdx.x * GPB + grp, step = G, e = fixed;
-    int seen = 0;  // queue position after this group's last claim
+    int i = (int)blockIdx.x * W + warp, step = G, e = fixed;
+    int seen = 0;  // queue position after this warp's last claim
+    int nd = 0;    // finished records whose forces are still to be evaluated
+    Work3 wk = {0u, 0u, 0u};
+    unsigned long long dots = 0;
     for (;;) {
         if (i >= e) {
             if (fixed >= m) break;
             int size = (m - fixed - seen) / (EPA_GUIDE * G);
             if (size < EPA_CLAIM) size = EPA_CLAIM;
-            const int64_t b = (int64_t)fixed + claim<LPP>(g, next, size);
+            const int64_t b = (int64_t)fixed + claim<32>(g, next, size);
             if (b >= m) break;
             i = (int)b;
             step = 1;
             e = b + size < m ? (int)b + size : m;
             seen = i - fixed + size;
         }
-        epa_record<LPP, false>(a, g, em, hull, i);
+        const SimplexRec rec = recs[i];
+        const int2 pr = reinterpret_cast<const int2*>(a.pairs)[rec.P];
+        const int oa = a.st.vert_off[pr.x], ob = a.st.vert_off[pr.y];
+        WarpHulls h;
+        h.load(wv + oa, a.st.vert_off[pr.x + 1] - oa, wv + ob, a.st.vert_off[pr.y + 1] - ob);
+        WarpEpaOut o;
+        epa_from_simplex(em, h, xyz(rec.S[0]), xyz(rec.S[1]), xyz(rec.S[2]), xyz(rec.S[3]), rec.ia, rec.ib, o);
+        wk.queries += (uint32_t)o.queries;
+        wk.faces += (uint32_t)o.faces;
+        dots += (unsigned long long)o.queries * (unsigned)(h.nA + h.nB);
+        if (lane == 0) {
+            const int ta = ft_v(o.t, 0), tb = ft_v(o.t, 1), tc = ft_v(o.t, 2);
+            EpaDone& d = done[nd];
+            d.nd = o.face;
+            d.a = f4(xyz(em.pv[ta]), __uint_as_float((uint32_t)em.pab[ta] | ((uint32_t)em.pab[tb] << 16)));
+            d.b = f4(xyz(em.pv[tb]), __uint_as_float((uint32_t)em.pab[tc] | (o.status << 16)));
+            d.c = f4(xyz(em.pv[tc]), __uint_as_float((uint32_t)i));
+        }
+        if (++nd == 32) {
+            epa_flush(a, done, nd);
+            nd = 0;
+        }
         i += step;
+    }
+    if (nd) epa_flush(a, done, nd);
+    if (a.work_counters && lane == 0 && wk.queries) {
+        atomicAdd(a.work_counters + 0, dots);
+        atomicAdd(a.work_counters + 1, (unsigned long long)wk.faces);
+        atomicAdd(a.work_counters + 2, (unsigned long long)wk.queries);
     }
 }
 
-// The records whose face list overflowed in the EPA pass, run again with the compacting EPA (a
-// separate kernel, so that the EPA pass itself carries none of that code; it finds an empty list almost
-// always and ends at once)
-template <int LPP, int BT>
-__global__ void __launch_bounds__(BT, 1) epa_retry_kernel(NarrowArgs a)
+template <int BT>
+int launch_epa_bt(const NarrowArgs& a, cudaStream_t s)
 {
-    pdl_wait();
-    pdl_launch_dependents();
-    extern __shared__ float4 smem[];
-    constexpr int GPB = BT / LPP;
-    const int grp = threadIdx.x / LPP;
-    Group<LPP> g;
-    g.lane = threadIdx.x % LPP;
-    g.mask = LPP == 32 ? 0xffffffffu : (((1u << LPP) - 1u) << ((threadIdx.x & 31) / LPP * LPP));
-    EpaMem* em = reinterpret_cast<EpaMem*>(smem) + grp;
-    float4* hull = reinterpret_cast<float4*>(reinterpret_cast<EpaMem*>(smem) + GPB) + (size_t)grp * 2 * a.hull_cap;
-    const int c = *epa_retry_count(a);
-    const int nr = c < EPA_RETRY_CAP ? c : EPA_RETRY_CAP;
-    for (int k = (int)blockIdx.x * GPB + grp; k < nr; k += (int)gridDim.x * GPB)
-        epa_record<LPP, true>(a, g, em, hull, epa_retry_list(a)[k]);
+    constexpr int W = BT / 32;
+    static LaunchSetup setup;
+    int per_sm = 0;
+    const size_t shm = (size_t)W * (sizeof(WarpEpaMem) + 32 * sizeof(EpaDone));
+    int rc = launch_setup(setup, epa_pass_kernel<BT>, BT, shm, 200 * 1024, &per_sm);
+    if (rc) return rc;
+    MWD_CUDA(launch_pdl(epa_pass_kernel<BT>, (unsigned)(num_sms() * per_sm), BT, shm, s, a));
+    return MWD_OK;
 }
 
 // threads per block of a block-size code of the lanes word (0: 128, 1: 64, 2: 256)
@@ -1640,30 +1507,11 @@ int launch_gjk(const NarrowArgs& a, int code, cudaStream_t s)
     return launch_gjk_bt<LPP, 128>(a, s);
 }
 
-template <int LPP, int BT>
-int launch_epa_bt(const NarrowArgs& a, cudaStream_t s)
-{
-    constexpr int GPB = BT / LPP;
-    static LaunchSetup setup;
-    int per_sm = 0;
-    const size_t shm = (size_t)GPB * sizeof(EpaMem) + (a.epa_global ? 0 : (size_t)GPB * 2 * a.hull_cap * sizeof(float4));
-    int rc = launch_setup(setup, epa_pass_kernel<LPP, BT>, BT, shm, 200 * 1024, &per_sm);
-    if (rc) return rc;
-    MWD_CUDA(launch_pdl(epa_pass_kernel<LPP, BT>, (unsigned)(num_sms() * per_sm), BT, shm, s, a));
-    static LaunchSetup retry_setup;
-    int retry_per_sm = 0;
-    rc = launch_setup(retry_setup, epa_retry_kernel<LPP, BT>, BT, shm, 200 * 1024, &retry_per_sm);
-    if (rc) return rc;
-    MWD_CUDA(launch_pdl(epa_retry_kernel<LPP, BT>, (unsigned)num_sms(), BT, shm, s, a));
-    return MWD_OK;
-}
-
-template <int LPP>
 int launch_epa(const NarrowArgs& a, int code, cudaStream_t s)
 {
-    if (code == 1) return launch_epa_bt<LPP, 64>(a, s);
-    if (code == 2) return launch_epa_bt<LPP, 256>(a, s);
-    return launch_epa_bt<LPP, 128>(a, s);
+    if (code == 1) return launch_epa_bt<64>(a, s);
+    if (code == 2) return launch_epa_bt<256>(a, s);
+    return launch_epa_bt<128>(a, s);
 }
 
 // Resolve the reference's overlapping stride-1 history writes (.cu:1018-1021, :1158-1161): the
@@ -1686,7 +1534,7 @@ template <int LPP, int MODE>
 int launch_lpp(const NarrowArgs& a, int64_t n_hint, cudaStream_t s)
 {
     constexpr int GPB = NARROW_THREADS / LPP;
-    size_t shm = (size_t)GPB * sizeof(EpaMem) + (size_t)GPB * 2 * a.hull_cap * sizeof(float4);
+    size_t shm = (size_t)(NARROW_THREADS / 32) * sizeof(WarpEpaMem) + (size_t)GPB * 2 * a.hull_cap * sizeof(float4);
     static LaunchSetup setup;
     int per_sm = 0;
     int rc = launch_setup(setup, narrow_kernel<LPP, MODE>, NARROW_THREADS, shm, 200 * 1024, &per_sm);
@@ -1700,12 +1548,6 @@ int launch_lpp(const NarrowArgs& a, int64_t n_hint, cudaStream_t s)
 }
 
 }  // namespace
-
-size_t narrow_smem_bytes(int lpp, int hull_cap)
-{
-    int gpb = NARROW_THREADS / lpp;
-    return (size_t)gpb * sizeof(EpaMem) + (size_t)gpb * 2 * hull_cap * sizeof(float4);
-}
 
 int launch_narrow(const NarrowArgs& a, int mode, int lanes, int64_t n_hint, cudaStream_t s)
 {
@@ -1728,9 +1570,8 @@ int launch_narrow(const NarrowArgs& a, int mode, int lanes, int64_t n_hint, cuda
     return MWD_ERR_INVALID;
 }
 
-// lanes = GJK-pass lanes per pair | EPA-pass lanes per pair << 8 (EPA lanes 0: same as GJK) | the two
-// passes' block-size codes (MWD_LANES_*_BLOCK_SHIFT); whether the EPA pass reads the hulls in place
-// comes in NarrowArgs (epa_global)
+// lanes = GJK-pass lanes per pair | EPA-pass lanes per pair << 8 (checked; the EPA pass gives each pair
+// a warp) | the two passes' block-size codes (MWD_LANES_*_BLOCK_SHIFT)
 int launch_narrow_two_pass(const NarrowArgs& a, int lanes, cudaStream_t s)
 {
     const int gl = lanes & 0xff;
@@ -1758,12 +1599,7 @@ int launch_narrow_two_pass(const NarrowArgs& a, int lanes, cudaStream_t s)
         default: rc = launch_gjk<32>(a, gb, s); break;
     }
     if (rc) return rc;
-    switch (el) {
-        case 4: rc = launch_epa<4>(a, eb, s); break;
-        case 8: rc = launch_epa<8>(a, eb, s); break;
-        case 16: rc = launch_epa<16>(a, eb, s); break;
-        default: rc = launch_epa<32>(a, eb, s); break;
-    }
+    rc = launch_epa(a, eb, s);
     if (rc) return rc;
     if (a.hist_keys) MWD_CUDA(launch_pdl(hist_flip_kernel, 1, 32, 0, s, a));
     return MWD_OK;

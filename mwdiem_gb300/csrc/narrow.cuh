@@ -52,8 +52,6 @@ struct NarrowArgs {
     int32_t pre_culled;     // the pair list holds only pairs whose bounding spheres overlap
     int32_t epa_zeroed;     // 1: epa_count was zeroed by an earlier kernel of the stream (the broad phase)
     float4* det_out;        // deterministic mode: (epa_cap, 3) F, TA, TB per EPA record instead of atomics
-    int32_t epa_global;     // 1: the EPA pass reads the hulls from global memory (L1) instead of staging them
-    int32_t pad3;
     // persistent tangential history (two-pass mode): tables read at *hist_parity, written at the other
     unsigned long long* hist_keys;
     float4* hist_vals;
@@ -64,6 +62,5 @@ struct NarrowArgs {
 int launch_narrow(const NarrowArgs& a, int mode, int lanes, int64_t n_hint, cudaStream_t s);
 int launch_narrow_two_pass(const NarrowArgs& a, int lanes, cudaStream_t s);
 int launch_hist_resolve(float* hist, const float* stage, const uint8_t* wrote, int64_t n, cudaStream_t s);
-size_t narrow_smem_bytes(int lpp, int hull_cap);
 
 }  // namespace mwd

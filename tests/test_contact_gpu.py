@@ -238,3 +238,22 @@ def test_epa_beyond_128_faces_in_the_two_pass_narrow_phase(lanes):
     want = (int((nsup * (local["A_nv"].astype(np.int64) + local["B_nv"])).sum()),
             int(o["counters"][:, 9][o["collision"] == 1].astype(np.int64).sum()), int(nsup.sum()))
     assert got == want
+
+
+@pytest.mark.parametrize("nv", [4, 8, 16, 17, 32, 33, 48, 49, 64])
+@pytest.mark.parametrize("n_pairs", [1, 33])
+def test_epa_warp_hull_sizes(nv, n_pairs):
+    # hulls at the edges of the warp's vertex shares (16 lanes per hull, one to four vertices each), deep
+    # overlaps, alone and as one more than a warp's worth of pairs
+    from mwdiem_gb300.pairbench import PairScene
+    inp, N = make_pairs(n_pairs, seed=100 + nv, V=64, n_min=nv, n_max=nv, dist=(0.3, 1.0), pool=8)
+    p = dict(CONTACT_PARAMS, num_vertices_max=64)
+    local = dict(inp, A_id=(2 * np.arange(n_pairs)).astype(np.int32), B_id=(2 * np.arange(n_pairs) + 1).astype(np.int32))
+    o = oracle.contact(local, p, 2 * n_pairs, "f32")
+    assert (o["collision"] == 1).any()
+    ps = PairScene.from_arrays(inp, p)
+    ps.narrow()
+    torch.cuda.synchronize()
+    assert np.array_equal(ps.w["collision"].cpu().numpy(), o["collision"])
+    assert bits_equal(ps.t["force"][:, :3].cpu().numpy(), o["force"])
+    assert bits_equal(ps.t["torque"][:, :3].cpu().numpy(), o["torque"])
