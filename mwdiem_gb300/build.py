@@ -1,9 +1,10 @@
 """Build ``libmwdem.so`` in-tree (``mwdiem_gb300/_build/``) with nvcc for sm_103a.
 
-Every translation unit is compiled with ``--fmad=false`` and IEEE division/square root: the narrow
+The translation units are compiled with ``--fmad=false`` and IEEE division/square root: the narrow
 phase reproduces the reference kernel's rounding operation by operation, and the host parts of the
 library (which derive the contact-law constants) are compiled with ``-ffp-contract=off`` for the
-same reason.  Translation units compile in parallel.
+same reason.  The differentiable step (``adjoint.cu``) reproduces no operation sequence: there a product
+and a sum become one FP64 instruction.  Translation units compile in parallel.
 """
 from __future__ import annotations
 
@@ -21,6 +22,7 @@ LIB = BUILD / "libmwdem.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVFLAGS = ["-O3", "-lineinfo", "--fmad=false", "-prec-div=true", "-prec-sqrt=true", "-std=c++17",
            "-Xcompiler", "-fPIC,-ffp-contract=off", "-diag-suppress", "1444", f"-I{INCLUDE}"]
+FUSED = ("adjoint.cu",)  # sources whose products and sums may be fused
 SOURCES = ["narrow.cu", "integrate.cu", "broad.cu", "capi.cu", "probe.cu", "noalloc.cu", "adjoint.cu", "reduce.cu", "inlet.cu"]
 
 
@@ -50,7 +52,8 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
     def one(src):
         obj = BUILD / (Path(src).stem + ".o")
-        cmd = [cc, *ARCH, *NVFLAGS, "-c", str(CSRC / src), "-o", str(obj)]
+        flags = [f for f in NVFLAGS if not (src in FUSED and f == "--fmad=false")]
+        cmd = [cc, *ARCH, *flags, "-c", str(CSRC / src), "-o", str(obj)]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
         r = subprocess.run(cmd, capture_output=True, text=True)

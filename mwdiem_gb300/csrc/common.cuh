@@ -1,7 +1,7 @@
 // Shared device helpers for libmwdem (sm_103a).
 //
-// Every translation unit of the library is compiled with --fmad=false and IEEE division/sqrt
-// (no -use_fast_math): the narrow phase must round exactly like the reference kernel's
+// The translation units of the library are compiled with --fmad=false (adjoint.cu excepted) and IEEE
+// division/sqrt (no -use_fast_math): the narrow phase must round exactly like the reference kernel's
 // operation sequence, which the oracle evaluates on the CPU without FMA contraction.
 #pragma once
 
