@@ -158,6 +158,23 @@ __device__ __forceinline__ void support_pair(const Group<LPP>& g, const float4* 
     S2 = mk3(p2.x - q2.x, p2.y - q2.y, p2.z - q2.z);
 }
 
+// two hulls read in place (or staged) by a group of lanes
+template <int LPP>
+struct GroupHulls {
+    const Group<LPP>& g;
+    const float4 *hA, *hB;
+    int nA, nB;
+    __device__ __forceinline__ void query(f3 d, f3& s, int& ia, int& ib) const
+    {
+        Work3 wk;
+        support<LPP>(g, hA, nA, hB, nB, d, s, ia, ib, wk);
+    }
+    __device__ __forceinline__ void both(f3 d, f3& S1, int& a1, int& b1, f3& S2, int& a2, int& b2) const
+    {
+        support_pair<LPP>(g, hA, nA, hB, nB, d, S1, a1, b1, S2, a2, b2);
+    }
+};
+
 // ---- simplex tests, identical on every lane (.cu:103-268) ----
 __device__ __forceinline__ void seg_test(f3 P1, f3 P2, int& coll, f3& d)
 {
@@ -215,6 +232,53 @@ __device__ __forceinline__ void tet_test(f3 P1, f3 P2, f3 P3, f3 P4, int& coll, 
     else if (dot(n3, P4) < 0.f) { d = n3; todel = 1; }
     else if (dot(n4, P4) < 0.f) { d = n4; todel = 2; }
     else coll = 1;
+}
+
+// the outcome of seg_test and of tri_test, without their direction (which tet_test does not use)
+__device__ __forceinline__ int seg_outcome(f3 P1, f3 P2)
+{
+    const f3 e = P2 - P1;
+    const f3 t = cross(e, P2);
+    return dot(e, P2) < 0.f ? 0 : (t.x == 0.f && t.y == 0.f && t.z == 0.f) ? 1 : -1;
+}
+__device__ __forceinline__ int tri_outcome(f3 P1, f3 P2, f3 P3)
+{
+    const int c2 = seg_outcome(P2, P3), c3 = seg_outcome(P1, P3);
+    const f3 e13 = P1 - P3;
+    const f3 e32 = P3 - P2;
+    const f3 n = cross(e32, e13);
+    const bool beside = dot(cross(e32, n), P2) < 0.f || dot(cross(e13, n), P3) < 0.f;
+    if (c2 == 1 || c3 == 1) return 1;
+    if (c2 == 0 && c3 == 0) return 0;
+    return !beside && dot(P3, n) == 0.f ? 1 : -1;
+}
+
+// tet_test by a group of at least four lanes: lane f = 0, 1, 2 tests the face (P1,P2,P4), (P2,P3,P4),
+// (P3,P1,P4) -- tri_test's outcome and the side the origin lies on -- and ballots combine them.  (On every
+// lane in turn, the three faces are about 400 instructions, and GJK's slow pairs run 50 such tests.)
+template <int LPP>
+__device__ __forceinline__ void tet_test_lanes(const Group<LPP>& g, f3 P1, f3 P2, f3 P3, f3 P4, int& coll, f3& d,
+                                               int& todel)
+{
+    static_assert(LPP >= 4, "a lane per face");
+    const int f = g.lane & 3;
+    const f3 a = f == 0 ? P1 : f == 1 ? P2 : P3;
+    const f3 b = f == 0 ? P2 : f == 1 ? P3 : P1;
+    const int c = tri_outcome(a, b, P4);
+    const f3 n = cross(b - a, P4 - a);
+    const unsigned inside = g.ballot(c == 1) & 7u, zero = g.ballot(c == 0) & 7u;
+    const unsigned beyond = g.ballot(dot(n, P4) < 0.f) & 7u;
+    todel = 0;
+    coll = -1;
+    if (inside) { coll = 1; return; }
+    if (__popc(zero) >= 2) { coll = 0; return; }  // c1 + c2 + c3 > -2
+    if (!beyond) { coll = 1; return; }
+    const int first = __ffs(beyond) - 1;
+    todel = first == 0 ? 3 : first;
+    const int src = (int)(threadIdx.x & 31) - g.lane + first;
+    d.x = __shfl_sync(g.mask, n.x, src);
+    d.y = __shfl_sync(g.mask, n.y, src);
+    d.z = __shfl_sync(g.mask, n.z, src);
 }
 
 // (double)v < 1e-6 && (double)v > -1e-6 for a float v, without FP64: a float compares with the
@@ -429,6 +493,8 @@ struct WarpHulls {
     const float4 *hA, *hB;
     int nA, nB, per;
     float x[4], y[4], z[4];
+    __device__ __forceinline__ void query(f3 d, f3& s, int& ia, int& ib) const;
+    __device__ __forceinline__ void both(f3 d, f3& S1, int& a1, int& b1, f3& S2, int& a2, int& b2) const;
     __device__ __forceinline__ void load(const float4* a, int na, const float4* b, int nb)
     {
         hA = a;
@@ -452,28 +518,55 @@ struct WarpHulls {
 static_assert(MWD_HULL_CAP <= 64, "four vertices per lane");
 
 // support() by a warp: each half's largest product, then the smallest index among the lanes that hold it
-__device__ __forceinline__ void support_warp(const WarpHulls& h, f3 d, f3& s, int& ia, int& ib)
+__device__ __forceinline__ void warp_winners(float best, unsigned idx, int& ia, int& ib)
+{
+    const bool onB = (threadIdx.x & 16) != 0;
+    const unsigned k = fkey(best);
+    const unsigned kA = __reduce_max_sync(0xffffffffu, onB ? 0u : k);
+    const unsigned kB = __reduce_max_sync(0xffffffffu, onB ? k : 0u);
+    ia = (int)__reduce_min_sync(0xffffffffu, !onB && k == kA ? idx : 0xffffu);
+    ib = (int)__reduce_min_sync(0xffffffffu, onB && k == kB ? idx : 0xffffu);
+}
+
+__device__ __forceinline__ void WarpHulls::query(f3 d, f3& s, int& ia, int& ib) const
 {
     const int lane = threadIdx.x & 31;
-    const bool onB = lane >= 16;
-    const f3 e = onB ? d * (-1.f) : d;
+    const f3 e = lane >= 16 ? d * (-1.f) : d;
     float best = -1e30f;
     int at = -1;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        if (j < h.per) {
-            const float t = e.x * h.x[j] + e.y * h.y[j] + e.z * h.z[j];
+        if (j < per) {
+            const float t = e.x * x[j] + e.y * y[j] + e.z * z[j];
             if (t > best) { best = t; at = j; }
         }
     }
-    const unsigned k = fkey(best);
-    const unsigned kA = __reduce_max_sync(0xffffffffu, onB ? 0u : k);
-    const unsigned kB = __reduce_max_sync(0xffffffffu, onB ? k : 0u);
-    const unsigned idx = at < 0 ? 0u : (unsigned)((lane & 15) * h.per + at);
-    ia = (int)__reduce_min_sync(0xffffffffu, !onB && k == kA ? idx : 0xffffu);
-    ib = (int)__reduce_min_sync(0xffffffffu, onB && k == kB ? idx : 0xffffu);
-    const float4 a = h.hA[ia], b = h.hB[ib];
+    warp_winners(best, at < 0 ? 0u : (unsigned)((lane & 15) * per + at), ia, ib);
+    const float4 a = hA[ia], b = hB[ib];
     s = mk3(a.x - b.x, a.y - b.y, a.z - b.z);
+}
+
+// support_pair() by a warp: the second query's products are the first one's negated (exactly)
+__device__ __forceinline__ void WarpHulls::both(f3 d, f3& S1, int& a1, int& b1, f3& S2, int& a2, int& b2) const
+{
+    const int lane = threadIdx.x & 31;
+    const f3 e = lane >= 16 ? d * (-1.f) : d;
+    float best = -1e30f, opp = -1e30f;
+    int at = -1, oat = -1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j < per) {
+            const float t = e.x * x[j] + e.y * y[j] + e.z * z[j];
+            if (t > best) { best = t; at = j; }
+            if (-t > opp) { opp = -t; oat = j; }
+        }
+    }
+    const unsigned first = (unsigned)((lane & 15) * per);
+    warp_winners(best, at < 0 ? 0u : first + (unsigned)at, a1, b1);
+    warp_winners(opp, oat < 0 ? 0u : first + (unsigned)oat, a2, b2);
+    const float4 p1 = hA[a1], q1 = hB[b1], p2 = hA[a2], q2 = hB[b2];
+    S1 = mk3(p1.x - q1.x, p1.y - q1.y, p1.z - q1.z);
+    S2 = mk3(p2.x - q2.x, p2.y - q2.y, p2.z - q2.z);
 }
 
 constexpr uint32_t FACE_LIVE = 0x80000000u;
@@ -585,7 +678,7 @@ __device__ __forceinline__ void epa_warp(WarpEpaMem& m, const WarpHulls& h, f3 S
         const f3 n = xyz(fm);
         f3 sp;
         int sa, sb;
-        support_warp(h, n, sp, sa, sb);
+        h.query(n, sp, sa, sb);
         r.queries += 1;
         proj = dot(n, sp);
         if (epa_stops(xmin_old, proj)) break;
@@ -747,7 +840,7 @@ __device__ __forceinline__ void epa_from_simplex(WarpEpaMem& m, const WarpHulls&
 {
     int a4 = ia >> 24, b4 = ib >> 24;
     const bool flat = is_flat(S1, S2, S3, S4);
-    if (flat) support_warp(h, cross(S1, S2), S4, a4, b4);
+    if (flat) h.query(cross(S1, S2), S4, a4, b4);
     epa_warp(m, h, S1, ia & 0xff, ib & 0xff, S2, (ia >> 8) & 0xff, (ib >> 8) & 0xff, S3, (ia >> 16) & 0xff,
              (ib >> 16) & 0xff, S4, a4, b4, r);
     r.queries += flat ? 1 : 0;
@@ -958,34 +1051,39 @@ __device__ __forceinline__ void accumulate(const NarrowArgs& a, const PairView& 
 
 // GJK up to the decision (.cu:996-1288): 0 separated, 1 in contact (simplex in rec), -1 undecided
 // after 50 tetrahedron iterations.
-template <int LPP>
-__device__ int gjk_decide(const Group<LPP>& g, const float4* hA, int nA, const float4* hB, int nB, f3 cA, f3 cB,
-                          SimplexRec& rec, Work3& wk)
+// h: the hulls, with the support queries of the group or warp that holds them
+template <int LPP, class Hulls>
+__device__ __forceinline__ int gjk_decide(const Group<LPP>& g, const Hulls& h, f3 cA, f3 cB, SimplexRec& rec, Work3& wk)
 {
+    auto counted = [&]() {
+        wk.dots += (uint32_t)(h.nA + h.nB);
+        wk.queries += 1;
+    };
     f3 S1, S2, S3, S4, d3, d4;
     int a1, b1, a2, b2, a3, b3, a4 = 0, b4 = 0, todel = 0, coll = -1;
     f3 d1 = cB - cA;
     f3 d2 = d1 * (-1.f);
-    support_pair<LPP>(g, hA, nA, hB, nB, d1, S1, a1, b1, S2, a2, b2);
-    wk.dots += (uint32_t)(nA + nB);
-    wk.queries += 1;
+    h.both(d1, S1, a1, b1, S2, a2, b2);
+    counted();
     if (dot(d1, S1) < 0.f) return 0;
-    wk.dots += (uint32_t)(nA + nB);
-    wk.queries += 1;
+    counted();
     if (dot(d2, S2) < 0.f) return 0;
     seg_test(S1, S2, coll, d3);
     if (coll == 0) return 0;
-    support<LPP>(g, hA, nA, hB, nB, d3, S3, a3, b3, wk);
+    h.query(d3, S3, a3, b3);
+    counted();
     if (dot(d3, S3) < 0.f) return 0;
     tri_test(S1, S2, S3, coll, d4);
     if (coll == 0) return 0;
     for (int zz = 0; zz < 50; ++zz) {
-        support<LPP>(g, hA, nA, hB, nB, d4, S4, a4, b4, wk);
+        h.query(d4, S4, a4, b4);
+        counted();
         if (dot(d4, S4) < 0.f) return 0;
         bool hit = false;
         if (S4.x == 0.f && S4.y == 0.f && S4.z == 0.f) hit = true;
         else {
-            tet_test(S1, S2, S3, S4, coll, d4, todel);
+            if constexpr (LPP >= 4) tet_test_lanes<LPP>(g, S1, S2, S3, S4, coll, d4, todel);
+            else tet_test(S1, S2, S3, S4, coll, d4, todel);
             if (coll == 0) return 0;
             if (coll == 1) hit = true;
         }
@@ -1021,7 +1119,7 @@ __device__ __forceinline__ void narrow_pairs(const NarrowArgs& a, int64_t P, boo
     if (in) {
         ok = load_pair<MODE>(a, P, p, hA, hB, g.lane, LPP);
         g.sync();
-        if (ok) out = gjk_decide<LPP>(g, hA, p.nA, hB, p.nB, p.cA, p.cB, rec, wk);
+        if (ok) out = gjk_decide<LPP>(g, GroupHulls<LPP>{g, hA, hB, p.nA, p.nB}, p.cA, p.cB, rec, wk);
     }
     __syncwarp();
     EpaResult er;
@@ -1157,13 +1255,13 @@ __global__ void __launch_bounds__(NARROW_THREADS) narrow_kernel(NarrowArgs a)
 // read straight from the world-vertex table (no shared memory, few registers, many resident warps);
 // separated and undecided pairs are finished there.  Pairs GJK finds in contact append the simplex
 // it stopped on to a compact list.  Pass 2 (epa_pass_kernel) continues exactly where pass 1
-// stopped -- CorrectFlat, EPA, force -- for the listed pairs only, with the shared-memory polytope.
+// stopped -- CorrectFlat, EPA, force -- for the listed pairs only, a warp each.
 // The operation sequence per pair is the single-pass kernel's.
 
-// GJK on pair P by the group; lane 0 records the outcome (status, contact flag, and for a pair in
-// contact its simplex in the EPA list, whose slot it also appends to *list when list is given)
+// GJK on pair P by the group (a full warp holds the hulls in registers); lane 0 records the outcome
+// (status, contact flag, and for a pair in contact its simplex in the EPA list)
 template <int LPP>
-__device__ __forceinline__ void gjk_pair(const NarrowArgs& a, const Group<LPP>& g, int64_t P, int* list, int* list_n)
+__device__ __forceinline__ void gjk_pair(const NarrowArgs& a, const Group<LPP>& g, int64_t P)
 {
     const double4* pos = reinterpret_cast<const double4*>(a.st.pos);
     const int2* pairs = reinterpret_cast<const int2*>(a.pairs);
@@ -1179,7 +1277,15 @@ __device__ __forceinline__ void gjk_pair(const NarrowArgs& a, const Group<LPP>& 
     SimplexRec rec;
     int out = 0;
     const bool ok = nA <= a.hull_cap && nB <= a.hull_cap;
-    if (ok) out = gjk_decide<LPP>(g, wv + oa, nA, wv + ob, nB, cA, cB, rec, wk);
+    if (ok) {
+        if constexpr (LPP == 32) {
+            WarpHulls h;
+            h.load(wv + oa, nA, wv + ob, nB);
+            out = gjk_decide<LPP>(g, h, cA, cB, rec, wk);
+        } else {
+            out = gjk_decide<LPP>(g, GroupHulls<LPP>{g, wv + oa, wv + ob, nA, nB}, cA, cB, rec, wk);
+        }
+    }
     if (g.lane == 0) {
         if (!ok) {
             set_status(a.status, MWD_ST_BAD_SHAPE);
@@ -1189,7 +1295,6 @@ __device__ __forceinline__ void gjk_pair(const NarrowArgs& a, const Group<LPP>& 
             if (slot < a.epa_cap) {
                 rec.P = P;
                 recs[slot] = rec;
-                if (list) list[atomicAdd(list_n, 1)] = slot;
             } else {
                 set_status(a.status, MWD_ST_PAIR_OVERFLOW);
             }
@@ -1207,15 +1312,11 @@ __device__ __forceinline__ void gjk_pair(const NarrowArgs& a, const Group<LPP>& 
     g.sync();
 }
 
-// GJK on the candidates [base, base + chunk), clipped to hi, by one group (chunk = gjk_chunk(a, LPP)).
-// pre_culled: the broad phase already dropped the pairs whose spheres are apart, so each chunk is one
-// pair and it runs GJK; otherwise the chunk's LPP candidates are sphere-tested at once (one per lane)
-// and the survivors run GJK one after another.
-__device__ __forceinline__ int gjk_chunk(const NarrowArgs& a, int lpp) { return a.pre_culled ? 1 : lpp; }
-
+// GJK on the candidates [base, hi) (LPP at most) by one group.  pre_culled: the broad phase already dropped
+// the pairs whose spheres are apart, and there is one candidate, which runs GJK; otherwise the candidates
+// are sphere-tested at once (one per lane) and the survivors run GJK one after another.
 template <int LPP>
-__device__ __forceinline__ void gjk_candidates(const NarrowArgs& a, const Group<LPP>& g, int64_t base, int64_t hi,
-                                               int* list, int* list_n)
+__device__ __forceinline__ void gjk_candidates(const NarrowArgs& a, const Group<LPP>& g, int64_t base, int64_t hi)
 {
     unsigned msk;
     if (a.pre_culled) {
@@ -1235,8 +1336,23 @@ __device__ __forceinline__ void gjk_candidates(const NarrowArgs& a, const Group<
     while (msk) {
         const int l = __ffs(msk) - 1;
         msk &= msk - 1;
-        gjk_pair<LPP>(a, g, base + l, list, list_n);
+        gjk_pair<LPP>(a, g, base + l);
     }
+}
+
+template <int LPP, int BT>
+__device__ __forceinline__ void gjk_stride(const NarrowArgs& a, int64_t n)
+{
+    constexpr int GPB = BT / LPP;
+    const int grp = threadIdx.x / LPP;
+    Group<LPP> g;
+    g.lane = threadIdx.x % LPP;
+    g.mask = LPP == 32 ? 0xffffffffu : (((1u << LPP) - 1u) << ((threadIdx.x & 31) / LPP * LPP));
+    // candidates a group takes at a time: one when they are pre-culled or no more than the groups
+    const int chunk = a.pre_culled || n <= (int64_t)gridDim.x * GPB ? 1 : LPP;
+    const int64_t stride = (int64_t)gridDim.x * GPB * chunk;
+    for (int64_t base = ((int64_t)blockIdx.x * GPB + grp) * chunk; base < n; base += stride)
+        gjk_candidates<LPP>(a, g, base, base + chunk < n ? base + chunk : n);
 }
 
 // BT threads per block (64, 128 or 256: the autotuner's block-size knob), registers capped so that
@@ -1247,17 +1363,11 @@ __global__ void __launch_bounds__(BT, (LPP == 1 ? 896 : 768) / BT) gjk_pass_kern
 {
     pdl_wait();
     pdl_launch_dependents();
-    constexpr int GPB = BT / LPP;
-    const int grp = threadIdx.x / LPP;
-    Group<LPP> g;
-    g.lane = threadIdx.x % LPP;
-    g.mask = LPP == 32 ? 0xffffffffu : (((1u << LPP) - 1u) << ((threadIdx.x & 31) / LPP * LPP));
     const int64_t m = *a.n_pairs_dev;
     const int64_t n = m < a.pair_cap ? m : a.pair_cap;
-    const int chunk = gjk_chunk(a, LPP);
-    const int64_t stride = (int64_t)gridDim.x * GPB * chunk;
-    for (int64_t base = ((int64_t)blockIdx.x * GPB + grp) * chunk; base < n; base += stride)
-        gjk_candidates<LPP>(a, g, base, n, nullptr, nullptr);
+    // as many warps as pairs: a warp for each, whatever LPP
+    if (LPP < 32 && n <= (int64_t)gridDim.x * (BT / 32)) gjk_stride<32, BT>(a, n);
+    else gjk_stride<LPP, BT>(a, n);
 }
 
 // ------------------------------------------------------------------ persistent tangential history
