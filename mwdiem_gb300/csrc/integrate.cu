@@ -1,9 +1,9 @@
 // Quaternion leapfrog integrator (gpu_Verlet.cu:85-431), two variants:
 //
 //  * verlet_ref_kernel -- FP64 over the reference's own arrays (the drop-in for gpu_Verlet.Verlet_GPU).
-//    Same operation sequence as the reference; the per-vertex rotation of the world-frame vertex
-//    table (gpu_Verlet.cu:279-323) is done block-cooperatively so the (N,V,3) array is read and
-//    written with coalesced accesses instead of one thread walking V vertices.
+//    The reference's formulas with products and sums fused; the per-vertex rotation of the world-frame
+//    vertex table (gpu_Verlet.cu:279-323) is done by all lanes of the rows' warp, so the (N,V,3) array is
+//    read and written with coalesced accesses instead of one thread walking V vertices.
 //
 //  * integrate_kernel -- FP32 state in float4 structure-of-arrays with FP64 centres (the
 //    device-resident step).  Instead of rotating every world vertex by q each step (which compounds
@@ -33,45 +33,36 @@ __device__ __forceinline__ d3 dm(double x, double y, double z)
 __device__ __forceinline__ d3 operator+(d3 a, d3 b) { return dm(a.x + b.x, a.y + b.y, a.z + b.z); }
 __device__ __forceinline__ d3 operator-(d3 a, d3 b) { return dm(a.x - b.x, a.y - b.y, a.z - b.z); }
 __device__ __forceinline__ d3 operator*(d3 a, double s) { return dm(a.x * s, a.y * s, a.z * s); }
-__device__ __forceinline__ d3 operator/(d3 a, double s) { return dm(a.x / s, a.y / s, a.z / s); }
-__device__ __forceinline__ double ddot(d3 a, d3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ d3 dcross(d3 a, d3 b) { return dm(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x); }
+// a s + b
+__device__ __forceinline__ d3 dfma(d3 a, double s, d3 b) { return dm(fma(a.x, s, b.x), fma(a.y, s, b.y), fma(a.z, s, b.z)); }
+__device__ __forceinline__ double ddot(d3 a, d3 b) { return fma(a.x, b.x, fma(a.y, b.y, a.z * b.z)); }
+__device__ __forceinline__ d3 dcross(d3 a, d3 b)
+{
+    return dm(fma(a.y, b.z, -(a.z * b.y)), fma(a.z, b.x, -(a.x * b.z)), fma(a.x, b.y, -(a.y * b.x)));
+}
 __device__ __forceinline__ d3 dld(const double* p) { return dm(p[0], p[1], p[2]); }
 __device__ __forceinline__ void dst(double* p, d3 v) { p[0] = v.x; p[1] = v.y; p[2] = v.z; }
 
 struct dq {
     double w, x, y, z;
 };
-// Hamilton product, operand order of gpu_Verlet.cu:43-54
+// Hamilton product (gpu_Verlet.cu:43-54)
 __device__ __forceinline__ dq dqmul(dq a, dq b)
 {
-    d3 u = dm(a.x, a.y, a.z), v = dm(b.x, b.y, b.z);
-    d3 s = (v * a.w + u * b.w) + dcross(u, v);
     dq r;
-    r.w = a.w * b.w - ddot(u, v);
-    r.x = s.x;
-    r.y = s.y;
-    r.z = s.z;
+    r.w = fma(a.w, b.w, -ddot(dm(a.x, a.y, a.z), dm(b.x, b.y, b.z)));
+    r.x = fma(a.w, b.x, fma(a.x, b.w, fma(a.y, b.z, -(a.z * b.y))));
+    r.y = fma(a.w, b.y, fma(a.y, b.w, fma(a.z, b.x, -(a.x * b.z))));
+    r.z = fma(a.w, b.z, fma(a.z, b.w, fma(a.x, b.y, -(a.y * b.x))));
     return r;
 }
-__device__ __forceinline__ dq dqinv(dq q)
+// vector part of q (0, v) q* (sign 1) or q* (0, v) q (sign -1), q of any length:
+// (w^2 - u.u) v + 2 (u.v) u + sign 2 w (u x v)
+__device__ __forceinline__ d3 dqturn(dq q, d3 v, double sign)
 {
-    dq r;
-    r.w = q.w;
-    r.x = q.x * (-1);
-    r.y = q.y * (-1);
-    r.z = q.z * (-1);
-    return r;
-}
-__device__ __forceinline__ d3 dqtrip(dq q1, d3 v, dq q2)
-{
-    dq vq;
-    vq.w = 0;
-    vq.x = v.x;
-    vq.y = v.y;
-    vq.z = v.z;
-    dq m = dqmul(q1, dqmul(vq, q2));
-    return dm(m.x, m.y, m.z);
+    const d3 u = dm(q.x, q.y, q.z);
+    const d3 r = dfma(u, 2 * ddot(u, v), v * fma(q.w, q.w, -ddot(u, u)));
+    return dfma(dcross(u, v), sign * 2 * q.w, r);
 }
 __device__ __forceinline__ dq dqld(const double* p)
 {
@@ -91,79 +82,85 @@ __device__ __forceinline__ void dqst(double* p, dq q)
 }
 __device__ __forceinline__ d3 matvec(const double* M, d3 v)
 {
-    return dm(M[0] * v.x + M[1] * v.y + M[2] * v.z, M[3] * v.x + M[4] * v.y + M[5] * v.z, M[6] * v.x + M[7] * v.y + M[8] * v.z);
+    return dm(ddot(dld(M), v), ddot(dld(M + 3), v), ddot(dld(M + 6), v));
+}
+// [cos(|w| s), sin(|w| s) w / |w|]
+__device__ __forceinline__ dq dqincrement(d3 w, double s)
+{
+    const double wn = sqrt(ddot(w, w));
+    double sn, cs;
+    sincos(wn * s, &sn, &cs);
+    const double k = wn != 0 ? sn / wn : 0.0;
+    dq r;
+    r.w = cs;
+    r.x = w.x * k;
+    r.y = w.y * k;
+    r.z = w.z * k;
+    return r;
 }
 
-constexpr int RB = 128;  // rows per block
-
-__global__ void __launch_bounds__(RB) verlet_ref_kernel(VerletRefArgs a)
+// One warp per block, `rows` of its lanes with a row each; then all lanes turn the rows' vertices.  Bound
+// by FP64 instructions, each of which holds its scheduler for 64 cycles on this GPU however many of its
+// lanes work: so products and sums are fused, the turn of a vertex is a product with a matrix that its
+// row's lane forms (15 instructions with the shifts; the quaternion products were 65), and the host picks `rows` so that
+// the warps fill whole rounds of the schedulers.  20,005 rows of 32 vertices: 189 us before.
+constexpr int VR = 32;
+__global__ void __launch_bounds__(VR) verlet_ref_kernel(VerletRefArgs a, int rows)
 {
-    __shared__ dq s_q[RB];
-    __shared__ d3 s_c[RB];
-    __shared__ d3 s_dx[RB];
-    __shared__ int s_mode[RB];  // 0 inactive, 1 active, 2 active + fly-away reset
-    const int P = blockIdx.x * RB + threadIdx.x;
+    __shared__ double s_m[VR][9];  // turn about the old centre
+    __shared__ d3 s_c[VR], s_t[VR];  // old centre, and where it goes
+    __shared__ bool s_on[VR];
+    const int lane = threadIdx.x;
+    const int p0 = blockIdx.x * rows;
+    const int P = p0 + lane;
     const double dt = a.p.dt;
-    int mode = 0;
-    if (P < a.N && P >= a.p.n_min && P < a.p.n_max) {
+    const bool on = lane < rows && P < a.N && P >= a.p.n_min && P < a.p.n_max;
+    if (on) {
         d3 vel12 = dld(a.v12 + 3 * P), om12bf = dld(a.w12bf + 3 * P), ombf = dld(a.wbf + 3 * P);
         d3 om = dld(a.w + 3 * P), c = dld(a.com + 3 * P);
-        d3 f = dld(a.F + 3 * P), t = dld(a.T + 3 * P);
+        const d3 f = dld(a.F + 3 * P), t = dld(a.T + 3 * P);
         const double m = a.mass[P];
-        const double* Mi = a.Iinv + 9 * P;
-        const double* Mm = a.I + 9 * P;
         dq qq = dqld(a.q + 4 * P), qh = dqld(a.q12 + 4 * P);
         d3 dxa = dld(a.dxall + 3 * P);
 
-        d3 v32 = vel12 + ((f * 1) / m) * dt;
-        dq qi = dqinv(qq);
-        d3 tbf = dqtrip(qi, t, qq);
-        d3 p1 = matvec(Mm, ombf);
-        d3 p2 = tbf - dcross(ombf, p1);
-        d3 alpha = matvec(Mi, p2);
-        d3 om32bf = om12bf + alpha * dt;
-        double wn = sqrt(om.x * om.x + om.y * om.y + om.z * om.z);
-        d3 h = dm(0, 0, 0);
-        if (wn != 0) h = (om / wn) * sin(wn * dt / 2);
-        dq rq;
-        rq.w = cos(wn * dt / 2);
-        rq.x = h.x;
-        rq.y = h.y;
-        rq.z = h.z;
-        dq q32 = dqmul(rq, qh);
-        vel12 = v32;
-        qh = q32;
-        om12bf = om32bf;
-        d3 dx = vel12 * dt;
+        // F / m, each quotient corrected by its exact remainder (extreme operands divide)
+        const double im = 1 / m;
+        const bool plain = fabs(m) > 1e-150 && fabs(m) < 1e150;
+        auto over_m = [&](double x) {
+            const double y = x * im;
+            if (plain && (x == 0 || (fabs(x) > 1e-120 && fabs(x) < 1e150))) return x == 0 ? y : fma(fma(-m, y, x), im, y);
+            return x / m;
+        };
+        const d3 acc = dm(over_m(f.x), over_m(f.y), over_m(f.z));
+        const d3 tbf = dqturn(qq, t, -1);
+        const d3 p1 = matvec(a.I + 9 * P, ombf);
+        const d3 p2 = tbf - dcross(ombf, p1);
+        const d3 alpha = matvec(a.Iinv + 9 * P, p2);
+        vel12 = dfma(acc, dt, vel12);
+        qh = dqmul(dqincrement(om, dt / 2), qh);
+        om12bf = dfma(alpha, dt, om12bf);
+        const d3 dx = vel12 * dt;
         dxa = dxa + dx;
-        d3 om34bf = om12bf + ((alpha * dt) * 1) / 4;
-        d3 om34 = dqtrip(qh, om34bf, dqinv(qh));
-        double wn34 = sqrt(om34.x * om34.x + om34.y * om34.y + om34.z * om34.z);
-        d3 h2 = dm(0, 0, 0);
-        if (wn34 != 0) h2 = (om34 / wn34) * sin(wn34 * dt / 4);
-        dq rq2;
-        rq2.w = cos(wn34 * dt / 4);
-        rq2.x = h2.x;
-        rq2.y = h2.y;
-        rq2.z = h2.z;
-        dq qold = qq;
-        qq = dqmul(rq2, qh);
-        dq qa = dqmul(qq, qold);
-        ombf = om12bf + ((alpha * dt) * 1) / 2;
-        om = dqtrip(qq, ombf, dqinv(qq));
-        d3 vel = vel12 + (f * dt) / m;
+        const d3 om34 = dqturn(qh, dfma(alpha, dt / 4, om12bf), 1);
+        const dq qold = qq;
+        qq = dqmul(dqincrement(om34, dt / 4), qh);
+        const dq qa = dqmul(qq, qold);
+        ombf = dfma(alpha, dt / 2, om12bf);
+        om = dqturn(qq, ombf, 1);
+        d3 vel = dfma(acc, dt, vel12);
         const d3 c_old = c;
         c = c + dx;
-        mode = 1;
+        d3 to = c;
         const double* box = a.p.box;
         if (c.x > box[0] || c.x < box[1] || c.y > box[2] || c.y < box[3] || c.z > box[4] || c.z < box[5]) {
-            mode = 2;
+            // fly-away reset (gpu_Verlet.cu:338-352): stop the particle, undo the move
             vel = dm(0, 0, 0);
             vel12 = vel;
             om12bf = vel;
             ombf = vel;
             om = vel;
             c = c + dx * (-1);
+            to = c_old;
             if (a.n_reset) atomicAdd(a.n_reset, 1);
         }
         dst(a.v + 3 * P, vel);
@@ -176,29 +173,52 @@ __global__ void __launch_bounds__(RB) verlet_ref_kernel(VerletRefArgs a)
         dqst(a.q12 + 4 * P, qh);
         dqst(a.q + 4 * P, qq);
         dqst(a.qall + 4 * P, qa);
-        s_q[threadIdx.x] = qq;
-        s_c[threadIdx.x] = c_old;
-        s_dx[threadIdx.x] = dx;
+        // the matrix of v -> vector part of q (0, v) q*
+        const double ww = qq.w * qq.w, xx = qq.x * qq.x, yy = qq.y * qq.y, zz = qq.z * qq.z;
+        double* M = s_m[lane];
+        M[0] = (ww + xx) - (yy + zz);
+        M[4] = (ww + yy) - (xx + zz);
+        M[8] = (ww + zz) - (xx + yy);
+        M[1] = 2 * fma(qq.x, qq.y, -(qq.w * qq.z));
+        M[3] = 2 * fma(qq.x, qq.y, qq.w * qq.z);
+        M[2] = 2 * fma(qq.x, qq.z, qq.w * qq.y);
+        M[6] = 2 * fma(qq.x, qq.z, -(qq.w * qq.y));
+        M[5] = 2 * fma(qq.y, qq.z, -(qq.w * qq.x));
+        M[7] = 2 * fma(qq.y, qq.z, qq.w * qq.x);
+        s_c[lane] = c_old;
+        s_t[lane] = to;
     }
-    s_mode[threadIdx.x] = mode;
-    __syncthreads();
-    // vertices of this block's rows: rotate about the old centre, then translate (gpu_Verlet.cu:279-352)
+    s_on[lane] = on;
+    __syncwarp();
+    // vertices of the warp's rows: turned about the old centre, then moved (gpu_Verlet.cu:279-352)
     const int V = a.p.V;
-    const int p0 = blockIdx.x * RB;
-    const int rows = min(RB, a.N - p0);
-    for (int j = threadIdx.x; j < rows * V; j += RB) {
-        const int r = j / V;
-        const int md = s_mode[r];
-        if (!md) continue;
-        double* vp = a.verts + ((size_t)(p0 + r) * V + (j - r * V)) * 3;
-        const dq q = s_q[r];
-        const d3 c = s_c[r], dx = s_dx[r];
-        d3 v = dqtrip(q, dld(vp) - c, dqinv(q)) + c;
-        v = v + dx;
-        if (md == 2) v = v + dx * (-1);
-        dst(vp, v);
+    const int total = min(rows, a.N - p0) * V;
+    double* vp = a.verts + (size_t)p0 * V * 3;
+    constexpr int U = 4;  // vertices in flight per lane
+    for (int j0 = lane; j0 < total; j0 += U * VR) {
+        d3 v[U];
+        int r[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int j = j0 + k * VR;
+            r[k] = j < total ? j / V : 0;
+            if (j < total && s_on[r[k]]) v[k] = dld(vp + 3 * (size_t)j);
+            else r[k] = -1;
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            if (r[k] < 0) continue;
+            const d3 c = s_c[r[k]], t = s_t[r[k]];
+            const double* M = s_m[r[k]];
+            const d3 d = v[k] - c;
+            // the turned offset first: rounded at its own size, not at the coordinates'
+            const d3 o = dm(ddot(dld(M), d), ddot(dld(M + 3), d), ddot(dld(M + 6), d));
+            dst(vp + 3 * (size_t)(j0 + k * VR), o + t);
+        }
     }
 }
+
+constexpr int RB = 128;  // rows per block
 
 // ------------------------------------------------------------------ FP32 device-resident step
 
@@ -439,7 +459,12 @@ __global__ void __launch_bounds__(256) world_verts_kernel(mwd_state st)
 int launch_verlet_ref(const VerletRefArgs& a, cudaStream_t s)
 {
     if (a.N <= 0) return MWD_OK;
-    verlet_ref_kernel<<<(a.N + RB - 1) / RB, RB, 0, s>>>(a);
+    // whole rounds of one warp per scheduler (four per SM), with the fewest rows per warp that need no
+    // further round: a row's own arithmetic takes a warp as long for 1 row as for 32, its vertices do not
+    const int schedulers = 4 * num_sms();
+    const int rounds = (a.N + VR * schedulers - 1) / (VR * schedulers);
+    const int rows = (a.N + rounds * schedulers - 1) / (rounds * schedulers);
+    verlet_ref_kernel<<<(a.N + rows - 1) / rows, VR, 0, s>>>(a, rows);
     MWD_CUDA(cudaGetLastError());
     return MWD_OK;
 }
