@@ -306,6 +306,10 @@ __device__ __forceinline__ bool is_flat(f3 S1, f3 S2, f3 S3, f3 S4)
 // and the shifted bounds round by at most 6e-8 x more (1.4e-7 x < 2^-22 x in all), so outside that band
 // the float answer is the double one; inside it (and for x outside [1e-30, 1e37], NaN, or 0) the
 // reference's tests run.
+__device__ __noinline__ bool epa_stops_exactly(float x, float p)
+{
+    return x > p || ((double)x * 1.00001 > (double)p && (double)x * 0.99999 < (double)p);
+}
 __device__ __forceinline__ bool epa_stops(float x, float p)
 {
     if (x > 1e-30f && x < 1e37f) {
@@ -313,7 +317,7 @@ __device__ __forceinline__ bool epa_stops(float x, float p)
         if (p < hi - tol) return true;
         if (p > hi + tol) return false;
     }
-    return x > p || ((double)x * 1.00001 > (double)p && (double)x * 0.99999 < (double)p);
+    return epa_stops_exactly(x, p);
 }
 
 // ---------------------------------------------------------------- the reference's double results in FP32
@@ -602,6 +606,67 @@ __device__ __forceinline__ float4 face_plane(f3 a, f3 b, f3 c, bool& flip)
     return f4(n, ia > 0.f && ib > 0.f && ic > 0.f ? dist : 1e30f);
 }
 
+// edge j of a removed face: its vertices, and the code of the unordered pair
+__device__ __forceinline__ int edge_vertices(uint32_t t, int j, int& e0, int& e1)
+{
+    e0 = (int)((t >> (8 * j)) & 0xffu);
+    e1 = (int)((t >> (j == 2 ? 0 : 8 * j + 8)) & 0xffu);
+    return min(e0, e1) * VCAP + max(e0, e1);
+}
+
+// What an EPA seldom needs stays out of its loop, whose time on a short list is that of fetching its
+// instructions.
+
+// the horizon of more than ten removed faces (more edges than lanes), 32 edges at a time
+__device__ __noinline__ int horizon_many(WarpEpaMem& m, int edges)
+{
+    const int lane = threadIdx.x & 31;
+    int e0, e1, nnew = 0;
+    for (int c = lane; c < edges; c += 32) m.mark[edge_vertices(m.del[c / 3], c % 3, e0, e1)] = (uint16_t)c;
+    __syncwarp();
+    for (int c = lane; c < edges; c += 32) {
+        const int code = edge_vertices(m.del[c / 3], c % 3, e0, e1);
+        if (m.mark[code] != c) m.mark[code] = 0xffffu;
+    }
+    __syncwarp();
+    for (int base = 0; base < edges; base += 32) {
+        const int c = base + lane;
+        const bool keep = c < edges && m.mark[edge_vertices(m.del[c / 3], c % 3, e0, e1)] == c;
+        const unsigned b = __ballot_sync(0xffffffffu, keep);
+        const int q = nnew + __popc(b & ((1u << lane) - 1u));
+        if (keep && q < FCAP) m.edge[q] = (uint16_t)(e0 | (e1 << 8));
+        nnew += __popc(b);
+    }
+    return nnew;
+}
+
+// the removed faces out of the list in shared memory, the first one excepted; returns the new length
+__device__ __noinline__ int drop_removed(WarpEpaMem& m, int nt)
+{
+    const int lane = threadIdx.x & 31;
+    int kept = 0;
+    bool first = true;
+    for (int base = 0; base < nt; base += 32) {
+        const int f = base + lane;
+        const bool in = f < nt;
+        const float4 p = in ? m.fn[f] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const uint32_t t = in ? m.ft[f] : 0u;
+        const unsigned gone = __ballot_sync(0xffffffffu, in && !(t & FACE_LIVE));
+        const bool keep = in && ((t & FACE_LIVE) || (first && lane == __ffs(gone) - 1));
+        if (gone) first = false;
+        const unsigned b = __ballot_sync(0xffffffffu, keep);
+        const int o = kept + __popc(b & ((1u << lane) - 1u));  // at most f: nothing unread is overwritten
+        __syncwarp();
+        if (keep) {
+            m.fn[o] = p;
+            m.ft[o] = t;
+        }
+        kept += __popc(b);
+    }
+    __syncwarp();
+    return kept;
+}
+
 struct WarpEpaOut {
     float4 face;      // the final face's normal; w: depth
     uint32_t t;       // its vertices in the polytope
@@ -702,6 +767,7 @@ __device__ __forceinline__ void epa_warp(WarpEpaMem& m, const WarpHulls& h, f3 S
                     ft[s] &= ~FACE_LIVE;
                     fd[s] = 3e20f;
                     m.fn[32 * s + lane].w = 3e20f;
+                    m.ft[32 * s + lane] = ft[s];
                 }
                 ndel += __popc(b);
             }
@@ -715,19 +781,11 @@ __device__ __forceinline__ void epa_warp(WarpEpaMem& m, const WarpHulls& h, f3 S
         // comparing the lanes' pairs by exchanges took a quarter of the EPA's instructions.)
         int nnew = 0;
         const int edges = 3 * ndel;
-        auto edge_of = [&](int c, int& e0, int& e1) {
-            const int f = c < 32 ? lane_face : c / 3;
-            const int j = c < 32 ? lane_edge : c - 3 * f;
-            const uint32_t t = m.del[f];
-            e0 = (int)((t >> (8 * j)) & 0xffu);
-            e1 = (int)((t >> (j == 2 ? 0 : 8 * j + 8)) & 0xffu);
-            return min(e0, e1) * VCAP + max(e0, e1);
-        };
         if (edges <= 32) {
             const bool has = lane < edges;
             int e0 = 0, e1 = 0, code = 0;
             if (has) {
-                code = edge_of(lane, e0, e1);
+                code = edge_vertices(m.del[lane_face], lane_edge, e0, e1);
                 m.mark[code] = (uint16_t)lane;
             }
             __syncwarp();
@@ -738,46 +796,14 @@ __device__ __forceinline__ void epa_warp(WarpEpaMem& m, const WarpHulls& h, f3 S
             if (keep) m.edge[__popc(b & lt)] = (uint16_t)(e0 | (e1 << 8));
             nnew = __popc(b);
         } else {
-            int e0, e1;
-            for (int c = lane; c < edges; c += 32) m.mark[edge_of(c, e0, e1)] = (uint16_t)c;
-            __syncwarp();
-            for (int c = lane; c < edges; c += 32) {
-                const int code = edge_of(c, e0, e1);
-                if (m.mark[code] != c) m.mark[code] = 0xffffu;
-            }
-            __syncwarp();
-            for (int base = 0; base < edges; base += 32) {
-                const int c = base + lane;
-                const bool keep = c < edges && m.mark[edge_of(c, e0, e1)] == c;
-                const unsigned b = __ballot_sync(ALL, keep);
-                const int q = nnew + __popc(b & lt);
-                if (keep && q < FCAP) m.edge[q] = (uint16_t)(e0 | (e1 << 8));
-                nnew += __popc(b);
-            }
+            nnew = horizon_many(m, edges);
         }
         __syncwarp();
         if (nt + nnew > FCAP) {
             // the list is full (about one deep overlap in 120,000 of random hulls, some contacts of every
             // step of packed hulls or cubes): drop the removed faces, the first one excepted.  At most
             // 2 * 30 - 4 = 56 faces of a closed polytope are alive within the reference's iteration limit.
-            int kept = 0;
-            bool first = true;
-#pragma unroll
-            for (int s = 0; s < FACE_SLOTS; ++s) {
-                const bool in = 32 * s + lane < nt;
-                const unsigned gone = __ballot_sync(ALL, in && !(ft[s] & FACE_LIVE));
-                const bool keep = in && ((ft[s] & FACE_LIVE) || (first && lane == __ffs(gone) - 1));
-                if (gone) first = false;
-                const unsigned b = __ballot_sync(ALL, keep);
-                if (keep) {
-                    const int o = kept + __popc(b & lt);
-                    m.fn[o] = f4(fn[s], fd[s]);
-                    m.ft[o] = ft[s];
-                }
-                kept += __popc(b);
-            }
-            __syncwarp();
-            nt = kept;
+            nt = drop_removed(m, nt);
 #pragma unroll
             for (int s = 0; s < FACE_SLOTS; ++s) {
                 fd[s] = nan;
@@ -1457,7 +1483,7 @@ struct EpaDone {
 };
 
 // The forces of up to 32 finished records, one per lane
-__device__ __forceinline__ void epa_flush(const NarrowArgs& a, const EpaDone* done, int n)
+__device__ __noinline__ void epa_flush(const NarrowArgs& a, const EpaDone* done, int n)
 {
     const int lane = threadIdx.x & 31;
     __syncwarp();
@@ -1506,7 +1532,7 @@ __device__ __forceinline__ void epa_flush(const NarrowArgs& a, const EpaDone* do
 
 // BT threads per block, registers capped so that 640 threads per SM stay resident (5 blocks of 128)
 template <int BT>
-__global__ void __launch_bounds__(BT, 640 / BT) epa_pass_kernel(NarrowArgs a)
+__global__ void __launch_bounds__(BT, 640 / BT) epa_pass_kernel(const __grid_constant__ NarrowArgs a)
 {
     pdl_wait();
     pdl_launch_dependents();
