@@ -94,18 +94,27 @@ __device__ __forceinline__ d3 rotv(dq q, d3 r)
               2.0 * (x * y + w * z) * r.x + (1.0 - 2.0 * (x * x + z * z)) * r.y + 2.0 * (y * z - w * x) * r.z,
               2.0 * (x * z - w * y) * r.x + 2.0 * (y * z + w * x) * r.y + (1.0 - 2.0 * (x * x + y * y)) * r.z);
 }
-__device__ __forceinline__ dq rotv_rev(dq q, d3 r, d3 g)
+// The gradient on q of sum_k <g_k, R(q) r_k> from the sum of the outer products G = sum_k g_k r_k^T
+// (rows x, y, z): a third of the multiply-adds of the three vertices taken one by one
+struct Outer {
+    d3 x, y, z;
+};
+__device__ __forceinline__ void outer_add(Outer& G, d3 g, d3 r)
+{
+    G.x += r * g.x;
+    G.y += r * g.y;
+    G.z += r * g.z;
+}
+__device__ __forceinline__ dq rotv_rev(dq q, const Outer& G)
 {
     const double w = q.w, x = q.x, y = q.y, z = q.z;
+    const double a = G.z.y - G.y.z, b = G.x.z - G.z.x, c = G.y.x - G.x.y;  // antisymmetric part
+    const double d = G.x.y + G.y.x, e = G.x.z + G.z.x, f = G.y.z + G.z.y;  // symmetric part
     dq o;
-    o.w = g.x * (-2.0 * z * r.y + 2.0 * y * r.z) + g.y * (2.0 * z * r.x - 2.0 * x * r.z) +
-          g.z * (-2.0 * y * r.x + 2.0 * x * r.y);
-    o.x = g.x * (2.0 * y * r.y + 2.0 * z * r.z) + g.y * (2.0 * y * r.x - 4.0 * x * r.y - 2.0 * w * r.z) +
-          g.z * (2.0 * z * r.x + 2.0 * w * r.y - 4.0 * x * r.z);
-    o.y = g.x * (-4.0 * y * r.x + 2.0 * x * r.y + 2.0 * w * r.z) + g.y * (2.0 * x * r.x + 2.0 * z * r.z) +
-          g.z * (-2.0 * w * r.x + 2.0 * z * r.y - 4.0 * y * r.z);
-    o.z = g.x * (-4.0 * z * r.x - 2.0 * w * r.y + 2.0 * x * r.z) + g.y * (2.0 * w * r.x - 4.0 * z * r.y + 2.0 * y * r.z) +
-          g.z * (2.0 * x * r.x + 2.0 * y * r.y);
+    o.w = 2.0 * (x * a + y * b + z * c);
+    o.x = 2.0 * (w * a + y * d + z * e - 2.0 * x * (G.y.y + G.z.z));
+    o.y = 2.0 * (w * b + x * d + z * f - 2.0 * y * (G.x.x + G.z.z));
+    o.z = 2.0 * (w * c + x * e + y * f - 2.0 * z * (G.x.x + G.y.y));
     return o;
 }
 
@@ -145,13 +154,20 @@ __device__ __forceinline__ d3 rot_rev(d3 w, double s, const Rot& r, dq g)
 
 constexpr double kPi = 3.141592653589793;
 
+// a / b from y = 1 / b: the product corrected by its exact remainder (Markstein, IBM J. Res. Dev. 34, 1990)
+__device__ __forceinline__ double quotient(double a, double b, double y)
+{
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+
 // ------------------------------------------------------------------ pair map
 struct PairIn {
     d3 cA, cB, vA, vB, wA, wB;
     dq qA, qB;
     d3 rA[3], rB[3];  // body-frame support vertices
     double IsA, IsB;
-    double Kn, en, et, mu;
+    double Kn, en, et, mu, Len, Let;  // Len, Let: log en, log et
     double cps;  // contact point (cpA + cps cpB) / 2: -1 the reference's, +1 the midpoint
 };
 
@@ -162,6 +178,7 @@ struct PairTape {
     double d00, d01, d11, d20, d21, den, b0, b1, b2;
     d3 cpA, cpB, cp, dA, dB;
     double C, Len, Let, Xen, S, Gn, Gt, sgn;
+    double il, iden, iC, imu, iIsA, iIsB, iXen;  // reciprocals (an FP64 division is ten instructions)
     d3 n, rA, rB, u, un, ut;
     double uns;
     d3 Fn, Ft, Ff;
@@ -188,7 +205,8 @@ __device__ __forceinline__ void pair_fwd(const PairIn& p, PairTape& t, PairOut& 
     t.l = sqrt(dot3(t.m, t.m));
     t.ok = t.l > 0.0;
     if (!t.ok) return;
-    t.n0 = t.m * (1.0 / t.l);
+    t.il = 1.0 / t.l;
+    t.n0 = t.m * t.il;
     t.depth = dot3(t.n0, t.V[0]);
     t.Pr = t.n0 * t.depth;
     t.u1 = t.V[2] - t.V[0];
@@ -201,22 +219,28 @@ __device__ __forceinline__ void pair_fwd(const PairIn& p, PairTape& t, PairOut& 
     t.den = t.d00 * t.d11 - t.d01 * t.d01;
     t.ok = t.den > 0.0;
     if (!t.ok) return;
-    t.b1 = (t.d11 * t.d20 - t.d01 * t.d21) / t.den;
-    t.b2 = (t.d00 * t.d21 - t.d01 * t.d20) / t.den;
+    t.iden = 1.0 / t.den;
+    t.b1 = quotient(t.d11 * t.d20 - t.d01 * t.d21, t.den, t.iden);
+    t.b2 = quotient(t.d00 * t.d21 - t.d01 * t.d20, t.den, t.iden);
     t.b0 = 1.0 - t.b2 - t.b1;
     t.cpA = (t.a[0] * t.b0 + t.a[1] * t.b1) + t.a[2] * t.b2;
     t.cpB = (t.b[0] * t.b0 + t.b[1] * t.b1) + t.b[2] * t.b2;
     t.cp = (t.cpA + t.cpB * p.cps) * 0.5;
     t.dA = t.cp - p.cA;
     t.dB = t.cp - p.cB;
-    t.C = 1.0 / p.mu + dot3(t.dA, t.dA) / p.IsA + dot3(t.dB, t.dB) / p.IsB;
-    t.Len = log(p.en);
-    t.Let = log(p.et);
+    t.imu = 1.0 / p.mu;
+    t.iIsA = 1.0 / p.IsA;
+    t.iIsB = 1.0 / p.IsB;
+    t.C = t.imu + quotient(dot3(t.dA, t.dA), p.IsA, t.iIsA) + quotient(dot3(t.dB, t.dB), p.IsB, t.iIsB);
+    t.iC = 1.0 / t.C;
+    t.Len = p.Len;
+    t.Let = p.Let;
     t.Xen = t.Len * t.Len + kPi * kPi;
+    t.iXen = 1.0 / t.Xen;
     // Gn = -2 mu Len / tc with tc = sqrt(mu Xen / Kn), i.e. -2 Len sqrt(mu Kn / Xen) (.cu:676-690)
-    t.S = sqrt(p.mu * p.Kn / t.Xen);
+    t.S = sqrt(quotient(p.mu * p.Kn, t.Xen, t.iXen));
     t.Gn = -2.0 * t.Len * t.S;
-    t.Gt = -2.0 * t.Let / t.C;
+    t.Gt = quotient(-2.0 * t.Let, t.C, t.iC);
     t.sgn = dot3(p.cB - p.cA, t.n0) < 0.0 ? -1.0 : 1.0;
     t.n = t.n0 * t.sgn;
     t.rA = t.cpA - p.cA;
@@ -307,21 +331,22 @@ __device__ __forceinline__ void pair_rev(const PairIn& p, const PairTape& t, d3 
     // n = n0 sgn
     d3 gn0 = gn * t.sgn;
     // Gt = -2 Let / C
-    double gC = gGt * 2.0 * t.Let / (t.C * t.C);
-    const double gLet = gGt * (-2.0 / t.C);
+    double gC = -gGt * t.Gt * t.iC;
+    const double gLet = gGt * (-2.0 * t.iC);
     // Gn = -2 Len S, S = sqrt(mu Kn / Xen), Xen = Len^2 + pi^2
     const double gS = gGn * (-2.0 * t.Len);
     double gLen = gGn * (-2.0 * t.S);
-    g.mu += gS * t.S / (2.0 * p.mu);
-    g.Kn += gS * t.S / (2.0 * p.Kn);
-    const double gXen = -gS * t.S / (2.0 * t.Xen);
+    const double gS2 = 0.5 * gS * t.S;
+    g.mu += gS2 * t.imu;
+    g.Kn += gS2 / p.Kn;
+    const double gXen = -gS2 * t.iXen;
     gLen += gXen * 2.0 * t.Len;
     g.en += gLen / p.en;
     g.et += gLet / p.et;
     // C = 1/mu + dA.dA / IsA + dB.dB / IsB
-    g.mu += -gC / (p.mu * p.mu);
-    gdA += t.dA * (2.0 * gC / p.IsA);
-    gdB += t.dB * (2.0 * gC / p.IsB);
+    g.mu += -gC * t.imu * t.imu;
+    gdA += t.dA * (2.0 * gC * t.iIsA);
+    gdB += t.dB * (2.0 * gC * t.iIsB);
     // dA = cp - cA, dB = cp - cB, cp = (cpA + cps cpB) / 2
     const d3 gcp = gdA + gdB;
     g.cA -= gdA;
@@ -339,8 +364,8 @@ __device__ __forceinline__ void pair_rev(const PairIn& p, const PairTape& t, d3 
     }
     // w0 = 1 - w2 - w1, w1 = N1 / den, w2 = N2 / den
     const double gb1 = gbeta[1] - gbeta[0], gb2 = gbeta[2] - gbeta[0];
-    const double gN1 = gb1 / t.den, gN2 = gb2 / t.den;
-    const double gden = -(t.b1 * gb1 + t.b2 * gb2) / t.den;
+    const double gN1 = gb1 * t.iden, gN2 = gb2 * t.iden;
+    const double gden = -(t.b1 * gN1 + t.b2 * gN2);
     const double gd00 = gN2 * t.d21 + gden * t.d11;
     const double gd11 = gN1 * t.d20 + gden * t.d00;
     const double gd01 = -gN1 * t.d21 - gN2 * t.d20 - 2.0 * gden * t.d01;
@@ -359,7 +384,7 @@ __device__ __forceinline__ void pair_rev(const PairIn& p, const PairTape& t, d3 
     gn0 += t.V[0] * gdepth;
     gV[0] += t.n0 * gdepth;
     // n0 = m / l, m = e1 x e2
-    const d3 gm = (gn0 - t.n0 * dot3(t.n0, gn0)) * (1.0 / t.l);
+    const d3 gm = (gn0 - t.n0 * dot3(t.n0, gn0)) * t.il;
     ge1 += cross3(t.e2, gm);
     const d3 ge2 = cross3(gm, t.e1);
     // e1 = V1 - V0, e2 = V2 - V1
@@ -367,14 +392,17 @@ __device__ __forceinline__ void pair_rev(const PairIn& p, const PairTape& t, d3 
     gV[0] -= ge1;
     gV[2] += ge2;
     gV[1] -= ge2;
+    Outer GA = {zero3(), zero3(), zero3()}, GB = {zero3(), zero3(), zero3()};
     for (int k = 0; k < 3; ++k) {
         ga[k] += gV[k];
         gb[k] -= gV[k];
         g.cA += ga[k];
         g.cB += gb[k];
-        g.qA += rotv_rev(p.qA, p.rA[k], ga[k]);
-        g.qB += rotv_rev(p.qB, p.rB[k], gb[k]);
+        outer_add(GA, ga[k], p.rA[k]);
+        outer_add(GB, gb[k], p.rB[k]);
     }
+    g.qA = rotv_rev(p.qA, GA);
+    g.qB = rotv_rev(p.qB, GB);
 }
 
 // ------------------------------------------------------------------ row map (integrator)
@@ -527,6 +555,13 @@ __device__ __forceinline__ int step_of(const mwd_diff& d, int t)
     return t >= 0 ? t + (d.t_base ? *d.t_base : 0) : *d.t_dev;
 }
 
+// log en and log et of the particle law (lanes 0, 1) and the wall law (lanes 2, 3), one log per warp
+__device__ __forceinline__ double law_log(const mwd_diff& d)
+{
+    const int k = threadIdx.x & 3;
+    return log(d.law[4 * (k >> 1) + 1 + (k & 1)]);
+}
+
 __device__ __forceinline__ void load_pair_in(const mwd_diff& d, const double* x, const mwd_contact_rec& rc, PairIn& p,
                                              bool& wall)
 {
@@ -644,6 +679,8 @@ __device__ __forceinline__ void write_mirror(const mwd_state& m, int r, const do
 __global__ void diff_collect_kernel(mwd_diff d, const int2* __restrict__ pairs, const int64_t* __restrict__ n_pairs,
                                     const int32_t* __restrict__ collision, const int32_t* __restrict__ face_ids)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     const int t = *d.t_dev;
     if (t >= d.n_steps) return;
     const int64_t np = *n_pairs;
@@ -677,15 +714,23 @@ __global__ void diff_collect_kernel(mwd_diff d, const int2* __restrict__ pairs, 
 
 __global__ void diff_force_kernel(mwd_diff d, const double* __restrict__ x, int t_arg)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     const int t = step_of(d, t_arg);
     if (t >= d.n_steps) return;
     const int64_t cnt = log_count(d, t);
     const int64_t off = d.step_off[t];
+    if ((int64_t)blockIdx.x * blockDim.x >= cnt) return;
+    const double mine = law_log(d);
+    const double L[4] = {__shfl_sync(0xffffffffu, mine, 0), __shfl_sync(0xffffffffu, mine, 1),
+                         __shfl_sync(0xffffffffu, mine, 2), __shfl_sync(0xffffffffu, mine, 3)};
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x) {
         const mwd_contact_rec rc = d.rec[off + i];
         PairIn p;
         bool wall;
         load_pair_in(d, x, rc, p, wall);
+        p.Len = wall ? L[2] : L[0];
+        p.Let = wall ? L[3] : L[1];
         PairTape tp;
         PairOut o;
         pair_fwd(p, tp, o);
@@ -712,6 +757,8 @@ __global__ void __launch_bounds__(DIFF_RB) diff_integrate_kernel(mwd_diff d, con
                                                                  double* FT_store, mwd_state mirror, int has_mirror,
                                                                  int t_arg)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ double s_com[3][DIFF_RB / 32];
     __shared__ bool s_last;
     const int t = step_of(d, t_arg);
@@ -802,6 +849,8 @@ __global__ void __launch_bounds__(DIFF_RB) diff_integrate_kernel(mwd_diff d, con
 
 __global__ void diff_mirror_kernel(mwd_diff d, const double* __restrict__ x, mwd_state mirror)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= d.n) return;
     write_mirror(mirror, r, x + (size_t)MWD_DIFF_ROW * r);
@@ -813,6 +862,8 @@ __global__ void __launch_bounds__(DIFF_RB) adj_integrate_kernel(mwd_diff d, cons
                                                                 const double* __restrict__ lam, double* lam_prev,
                                                                 const double* __restrict__ com_grad, double* gFT)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = step_of(d, t_arg);
     if (r >= d.n || t >= d.n_steps) return;
@@ -862,10 +913,16 @@ __global__ void __launch_bounds__(DIFF_RB) adj_integrate_kernel(mwd_diff d, cons
 __global__ void adj_force_kernel(mwd_diff d, const double* __restrict__ x, int t_arg, const double* __restrict__ gFT,
                                  double* lam_prev, double* glaw)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     const int t = step_of(d, t_arg);
     if (t >= d.n_steps) return;
     const int64_t cnt = log_count(d, t);
     const int64_t off = d.step_off[t];
+    if ((int64_t)blockIdx.x * blockDim.x >= cnt) return;
+    const double mine = law_log(d);
+    const double L[4] = {__shfl_sync(0xffffffffu, mine, 0), __shfl_sync(0xffffffffu, mine, 1),
+                         __shfl_sync(0xffffffffu, mine, 2), __shfl_sync(0xffffffffu, mine, 3)};
     double gl[8];
     for (int k = 0; k < 8; ++k) gl[k] = 0.0;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -875,6 +932,8 @@ __global__ void adj_force_kernel(mwd_diff d, const double* __restrict__ x, int t
         PairIn p;
         bool wall;
         load_pair_in(d, x, rc, p, wall);
+        p.Len = wall ? L[2] : L[0];
+        p.Let = wall ? L[3] : L[1];
         PairTape tp;
         PairOut o;
         pair_fwd(p, tp, o);
@@ -949,9 +1008,8 @@ int mwd_diff_collect(const mwd_diff* d, const mwd_work* work, mwd_stream_t strea
     int64_t b = (work->pair_cap + 255) / 256;
     const int64_t cap = (int64_t)num_sms() * 2;
     if (b > cap) b = cap;
-    diff_collect_kernel<<<(int)b, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        *d, reinterpret_cast<const int2*>(work->pairs), work->n_pairs, work->collision, work->face_ids);
-    MWD_CUDA(cudaGetLastError());
+    MWD_CUDA(launch_pdl(diff_collect_kernel, (unsigned)b, 256, 0, reinterpret_cast<cudaStream_t>(stream), *d,
+                        reinterpret_cast<const int2*>(work->pairs), work->n_pairs, work->collision, work->face_ids));
     return MWD_OK;
 }
 
@@ -963,8 +1021,7 @@ int mwd_diff_force(const mwd_diff* d, const double* x, int32_t t, mwd_stream_t s
         return MWD_ERR_INVALID;
     }
     // the contact count lives on the device: one block per SM strides through the step's records
-    diff_force_kernel<<<num_sms(), 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(*d, x, t);
-    MWD_CUDA(cudaGetLastError());
+    MWD_CUDA(launch_pdl(diff_force_kernel, (unsigned)num_sms(), 128, 0, reinterpret_cast<cudaStream_t>(stream), *d, x, t));
     return MWD_OK;
 }
 
@@ -987,9 +1044,8 @@ int mwd_diff_integrate(const mwd_diff* d, const double* x, double* x_out, double
         m = *mirror;
     }
     const int blocks = (d->n + DIFF_RB - 1) / DIFF_RB;
-    diff_integrate_kernel<<<blocks, DIFF_RB, 0, reinterpret_cast<cudaStream_t>(stream)>>>(*d, x, x_out, FT_store, m,
-                                                                                        mirror ? 1 : 0, t);
-    MWD_CUDA(cudaGetLastError());
+    MWD_CUDA(launch_pdl(diff_integrate_kernel, (unsigned)blocks, DIFF_RB, 0, reinterpret_cast<cudaStream_t>(stream), *d, x,
+                        x_out, FT_store, m, mirror ? 1 : 0, t));
     if (mirror && m.xform && m.vert_owner) return launch_world_verts(m, reinterpret_cast<cudaStream_t>(stream));
     return MWD_OK;
 }
@@ -1004,8 +1060,8 @@ int mwd_diff_mirror(const mwd_diff* d, const double* x, mwd_state* mirror, mwd_s
         return MWD_ERR_INVALID;
     }
     if (d->n == 0) return MWD_OK;
-    diff_mirror_kernel<<<(d->n + 127) / 128, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(*d, x, *mirror);
-    MWD_CUDA(cudaGetLastError());
+    MWD_CUDA(launch_pdl(diff_mirror_kernel, (unsigned)((d->n + 127) / 128), 128, 0, reinterpret_cast<cudaStream_t>(stream),
+                        *d, x, *mirror));
     if (mirror->xform && mirror->vert_owner) return launch_world_verts(*mirror, reinterpret_cast<cudaStream_t>(stream));
     return MWD_OK;
 }
@@ -1020,10 +1076,9 @@ int mwd_diff_adjoint(const mwd_diff* d, const double* x, const double* FT, int32
     }
     if (d->n == 0) return MWD_OK;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    adj_integrate_kernel<<<(d->n + DIFF_RB - 1) / DIFF_RB, DIFF_RB, 0, s>>>(*d, x, FT, t, lam, lam_prev, com_grad, gFT);
-    MWD_CUDA(cudaGetLastError());
-    adj_force_kernel<<<num_sms(), 128, 0, s>>>(*d, x, t, gFT, lam_prev, glaw);
-    MWD_CUDA(cudaGetLastError());
+    MWD_CUDA(launch_pdl(adj_integrate_kernel, (unsigned)((d->n + DIFF_RB - 1) / DIFF_RB), DIFF_RB, 0, s, *d, x, FT, t, lam,
+                        lam_prev, com_grad, gFT));
+    MWD_CUDA(launch_pdl(adj_force_kernel, (unsigned)num_sms(), 128, 0, s, *d, x, t, gFT, lam_prev, glaw));
     return MWD_OK;
 }
 
