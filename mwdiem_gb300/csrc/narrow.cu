@@ -56,17 +56,6 @@ __device__ __forceinline__ unsigned fkey(float f)
     return b ^ ((unsigned)((int)b >> 31) | 0x80000000u);
 }
 
-// Group-wide (largest value, then smallest index) of the lanes' (v, i), v not NaN: the sequential
-// "v > best" scan's first-index result when each lane holds its own first-index best.
-template <int LPP>
-__device__ __forceinline__ int group_argmax(const Group<LPP>& g, float v, int i)
-{
-    if (LPP == 1) return i;  // one lane per pair: its own scan is the sequential one
-    const unsigned k = fkey(v);
-    const unsigned km = __reduce_max_sync(g.mask, k);
-    return (int)__reduce_min_sync(g.mask, k == km ? (unsigned)i : 0xffffffffu);
-}
-
 // Work queue of the EPA pass: a 64-bit counter after the EPA record count in the block epa_count points
 // to (MWD_EPA_COUNT_INTS ints, 8-byte aligned), ints [2..3].  Zeroed with the record count before
 // each narrow phase.
@@ -84,94 +73,59 @@ __device__ __forceinline__ int64_t claim(const Group<LPP>& g, unsigned long long
     return (int64_t)__shfl_sync(g.mask, base, (int)(threadIdx.x & 31) - g.lane);
 }
 
-// argmax of d.a over A and of (-d).b over B, first index on ties (.cu:55-101)
 // work counted per pair when the caller asks for it: vertex dot products, EPA faces, support queries
 struct Work3 {
     uint32_t dots, faces, queries;
 };
 
-template <int LPP>
-__device__ __forceinline__ void support(const Group<LPP>& g, const float4* hA, int nA, const float4* hB, int nB,
-                                        f3 d, f3& s, int& ia, int& ib, Work3& wk)
-{
-    wk.dots += (uint32_t)(nA + nB);
-    wk.queries += 1;
-    float bA = -1e30f, bB = -1e30f;
-    int iA = 0, iB = 0;
-    // unrolled so that several vertex loads are in flight (the scan order, and so the result, is
-    // unchanged)
-#pragma unroll 4
-    for (int i = g.lane; i < nA; i += LPP) {
-        float4 v = hA[i];
-        float t = d.x * v.x + d.y * v.y + d.z * v.z;
-        if (t > bA) { bA = t; iA = i; }
-    }
-    f3 nd = d * (-1.f);
-#pragma unroll 4
-    for (int j = g.lane; j < nB; j += LPP) {
-        float4 v = hB[j];
-        float t = nd.x * v.x + nd.y * v.y + nd.z * v.z;
-        if (t > bB) { bB = t; iB = j; }
-    }
-    iA = group_argmax<LPP>(g, bA, iA);
-    iB = group_argmax<LPP>(g, bB, iB);
-    ia = iA;
-    ib = iB;
-    float4 a = hA[iA], b = hB[iB];
-    s = mk3(a.x - b.x, a.y - b.y, a.z - b.z);
-}
-
-// The first two support queries of GJK, in directions d1 and d2 = -d1, in one pass over the hulls:
-// the same dot products, maxima and first-index ties as two calls of support() (the A side of d2
-// and the B side of d1 both use -d1 = d1 * -1, the B side of d2 uses d2 * -1 = d1), so the results
-// are those two calls'.  The second query's latency overlaps the first's; the caller counts it as
-// work only when GJK gets that far.
-template <int LPP>
-__device__ __forceinline__ void support_pair(const Group<LPP>& g, const float4* hA, int nA, const float4* hB, int nB,
-                                             f3 d1, f3& S1, int& a1, int& b1, f3& S2, int& a2, int& b2)
-{
-    const f3 n1 = d1 * (-1.f);
-    float tA = -1e30f, uA = -1e30f, tB = -1e30f, uB = -1e30f;
-    int itA = 0, iuA = 0, itB = 0, iuB = 0;
-#pragma unroll 4
-    for (int i = g.lane; i < nA; i += LPP) {
-        const float4 v = hA[i];
-        const float t = d1.x * v.x + d1.y * v.y + d1.z * v.z;
-        const float u = n1.x * v.x + n1.y * v.y + n1.z * v.z;
-        if (t > tA) { tA = t; itA = i; }
-        if (u > uA) { uA = u; iuA = i; }
-    }
-#pragma unroll 4
-    for (int j = g.lane; j < nB; j += LPP) {
-        const float4 v = hB[j];
-        const float t = d1.x * v.x + d1.y * v.y + d1.z * v.z;
-        const float u = n1.x * v.x + n1.y * v.y + n1.z * v.z;
-        if (t > tB) { tB = t; itB = j; }
-        if (u > uB) { uB = u; iuB = j; }
-    }
-    a1 = group_argmax<LPP>(g, tA, itA);  // support(d1): argmax d1.a, argmax (-d1).b
-    b1 = group_argmax<LPP>(g, uB, iuB);
-    a2 = group_argmax<LPP>(g, uA, iuA);  // support(d2): argmax (-d1).a, argmax d1.b
-    b2 = group_argmax<LPP>(g, tB, itB);
-    const float4 p1 = hA[a1], q1 = hB[b1], p2 = hA[a2], q2 = hB[b2];
-    S1 = mk3(p1.x - q1.x, p1.y - q1.y, p1.z - q1.z);
-    S2 = mk3(p2.x - q2.x, p2.y - q2.y, p2.z - q2.z);
-}
-
-// two hulls read in place (or staged) by a group of lanes
-template <int LPP>
-struct GroupHulls {
-    const Group<LPP>& g;
+// Two hulls read in place by one lane.  query: argmax of d.a over A and of (-d).b over B, first index on ties
+// (.cu:55-101); both: the queries in the directions d and -d in one pass over the hulls (the second one's
+// products are the first one's negated, exactly).
+struct LaneHulls {
     const float4 *hA, *hB;
     int nA, nB;
     __device__ __forceinline__ void query(f3 d, f3& s, int& ia, int& ib) const
     {
-        Work3 wk;
-        support<LPP>(g, hA, nA, hB, nB, d, s, ia, ib, wk);
+        float bA = -1e30f, bB = -1e30f;
+        ia = ib = 0;
+        // unrolled so that several vertex loads are in flight
+#pragma unroll 4
+        for (int i = 0; i < nA; ++i) {
+            const float4 v = hA[i];
+            const float t = d.x * v.x + d.y * v.y + d.z * v.z;
+            if (t > bA) { bA = t; ia = i; }
+        }
+        const f3 nd = d * (-1.f);
+#pragma unroll 4
+        for (int j = 0; j < nB; ++j) {
+            const float4 v = hB[j];
+            const float t = nd.x * v.x + nd.y * v.y + nd.z * v.z;
+            if (t > bB) { bB = t; ib = j; }
+        }
+        const float4 a = hA[ia], b = hB[ib];
+        s = mk3(a.x - b.x, a.y - b.y, a.z - b.z);
     }
     __device__ __forceinline__ void both(f3 d, f3& S1, int& a1, int& b1, f3& S2, int& a2, int& b2) const
     {
-        support_pair<LPP>(g, hA, nA, hB, nB, d, S1, a1, b1, S2, a2, b2);
+        float tA = -1e30f, uA = -1e30f, tB = -1e30f, uB = -1e30f;
+        a1 = b1 = a2 = b2 = 0;
+#pragma unroll 4
+        for (int i = 0; i < nA; ++i) {
+            const float4 v = hA[i];
+            const float t = d.x * v.x + d.y * v.y + d.z * v.z;
+            if (t > tA) { tA = t; a1 = i; }
+            if (-t > uA) { uA = -t; a2 = i; }
+        }
+#pragma unroll 4
+        for (int j = 0; j < nB; ++j) {
+            const float4 v = hB[j];
+            const float t = d.x * v.x + d.y * v.y + d.z * v.z;
+            if (t > tB) { tB = t; b2 = j; }
+            if (-t > uB) { uB = -t; b1 = j; }
+        }
+        const float4 p1 = hA[a1], q1 = hB[b1], p2 = hA[a2], q2 = hB[b2];
+        S1 = mk3(p1.x - q1.x, p1.y - q1.y, p1.z - q1.z);
+        S2 = mk3(p2.x - q2.x, p2.y - q2.y, p2.z - q2.z);
     }
 };
 
@@ -253,32 +207,28 @@ __device__ __forceinline__ int tri_outcome(f3 P1, f3 P2, f3 P3)
     return !beside && dot(P3, n) == 0.f ? 1 : -1;
 }
 
-// tet_test by a group of at least four lanes: lane f = 0, 1, 2 tests the face (P1,P2,P4), (P2,P3,P4),
-// (P3,P1,P4) -- tri_test's outcome and the side the origin lies on -- and ballots combine them.  (On every
-// lane in turn, the three faces are about 400 instructions, and GJK's slow pairs run 50 such tests.)
+// tet_test by each group of LPP >= 4 lanes of a full warp: lane f = 0, 1, 2 tests the face (P1,P2,P4),
+// (P2,P3,P4), (P3,P1,P4) -- tri_test's outcome and the side the origin lies on -- and ballots combine them.
+// (On every lane in turn, the three faces are about 400 instructions, and GJK's slow pairs run 50 such tests.)
 template <int LPP>
-__device__ __forceinline__ void tet_test_lanes(const Group<LPP>& g, f3 P1, f3 P2, f3 P3, f3 P4, int& coll, f3& d,
-                                               int& todel)
+__device__ __forceinline__ void tet_test_lanes(f3 P1, f3 P2, f3 P3, f3 P4, int& coll, f3& d, int& todel)
 {
     static_assert(LPP >= 4, "a lane per face");
-    const int f = g.lane & 3;
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, g0 = lane & ~(LPP - 1), f = lane & 3;
     const f3 a = f == 0 ? P1 : f == 1 ? P2 : P3;
     const f3 b = f == 0 ? P2 : f == 1 ? P3 : P1;
     const int c = tri_outcome(a, b, P4);
     const f3 n = cross(b - a, P4 - a);
-    const unsigned inside = g.ballot(c == 1) & 7u, zero = g.ballot(c == 0) & 7u;
-    const unsigned beyond = g.ballot(dot(n, P4) < 0.f) & 7u;
-    todel = 0;
-    coll = -1;
-    if (inside) { coll = 1; return; }
-    if (__popc(zero) >= 2) { coll = 0; return; }  // c1 + c2 + c3 > -2
-    if (!beyond) { coll = 1; return; }
-    const int first = __ffs(beyond) - 1;
+    const unsigned inside = (__ballot_sync(ALL, c == 1) >> g0) & 7u, zero = (__ballot_sync(ALL, c == 0) >> g0) & 7u;
+    const unsigned beyond = (__ballot_sync(ALL, dot(n, P4) < 0.f) >> g0) & 7u;
+    const int first = beyond ? __ffs(beyond) - 1 : 0;
+    // c1 + c2 + c3 > -2: two of them zero
+    coll = inside ? 1 : __popc(zero) >= 2 ? 0 : beyond ? -1 : 1;
     todel = first == 0 ? 3 : first;
-    const int src = (int)(threadIdx.x & 31) - g.lane + first;
-    d.x = __shfl_sync(g.mask, n.x, src);
-    d.y = __shfl_sync(g.mask, n.y, src);
-    d.z = __shfl_sync(g.mask, n.z, src);
+    d.x = __shfl_sync(ALL, n.x, g0 + first);
+    d.y = __shfl_sync(ALL, n.y, g0 + first);
+    d.z = __shfl_sync(ALL, n.z, g0 + first);
 }
 
 // (double)v < 1e-6 && (double)v > -1e-6 for a float v, without FP64: a float compares with the
@@ -1079,12 +1029,9 @@ __device__ __forceinline__ void accumulate(const NarrowArgs& a, const PairView& 
 // after 50 tetrahedron iterations.
 // h: the hulls, with the support queries of the group or warp that holds them
 template <int LPP, class Hulls>
-__device__ __forceinline__ int gjk_decide(const Group<LPP>& g, const Hulls& h, f3 cA, f3 cB, SimplexRec& rec, Work3& wk)
+__device__ __forceinline__ int gjk_decide(const Hulls& h, f3 cA, f3 cB, SimplexRec& rec, int& queries)
 {
-    auto counted = [&]() {
-        wk.dots += (uint32_t)(h.nA + h.nB);
-        wk.queries += 1;
-    };
+    auto counted = [&]() { ++queries; };
     f3 S1, S2, S3, S4, d3, d4;
     int a1, b1, a2, b2, a3, b3, a4 = 0, b4 = 0, todel = 0, coll = -1;
     f3 d1 = cB - cA;
@@ -1108,7 +1055,7 @@ __device__ __forceinline__ int gjk_decide(const Group<LPP>& g, const Hulls& h, f
         bool hit = false;
         if (S4.x == 0.f && S4.y == 0.f && S4.z == 0.f) hit = true;
         else {
-            if constexpr (LPP >= 4) tet_test_lanes<LPP>(g, S1, S2, S3, S4, coll, d4, todel);
+            if constexpr (LPP >= 4) tet_test_lanes<LPP>(S1, S2, S3, S4, coll, d4, todel);
             else tet_test(S1, S2, S3, S4, coll, d4, todel);
             if (coll == 0) return 0;
             if (coll == 1) hit = true;
@@ -1129,6 +1076,164 @@ __device__ __forceinline__ int gjk_decide(const Group<LPP>& g, const Hulls& h, f
     return -1;
 }
 
+// ------------------------------------------------------------------ GJK by lane groups in lockstep
+//
+// The groups of a warp (LPP = 4, 8, 16 or 32 lanes, a pair each) run GJK together: every exchange between
+// lanes names the whole warp, so one instruction serves all the pairs of the warp until the last of them
+// is decided.  (Groups that exchange under masks of their own run one after another from the first
+// exchange on: 13,000 candidates of a pour took 20 us with them.)
+
+// (largest v, then smallest i) over aligned runs of H lanes
+template <int H>
+__device__ __forceinline__ int run_argmax(float v, int i)
+{
+    const unsigned k = fkey(v);
+    unsigned m = k;
+#pragma unroll
+    for (int o = H / 2; o > 0; o /= 2) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    int w = k == m ? i : 0x7fffffff;
+#pragma unroll
+    for (int o = H / 2; o > 0; o /= 2) w = min(w, __shfl_xor_sync(0xffffffffu, w, o));
+    return w;
+}
+
+// the hulls of a group, read in place or staged: the lower half of its lanes scans A's vertices, the upper
+// half B's
+template <int LPP>
+struct LockHulls {
+    const float4 *hA, *hB;
+    int nA, nB;
+    // support() of the groups that are on
+    __device__ __forceinline__ void query(f3 d, bool on, f3& s, int& ia, int& ib) const
+    {
+        constexpr int H = LPP / 2;
+        const int lane = threadIdx.x & 31, g0 = lane & ~(LPP - 1);
+        const bool onB = (lane & H) != 0;
+        const float4* h = onB ? hB : hA;
+        const int n = !on ? 0 : onB ? nB : nA;
+        const f3 e = onB ? d * (-1.f) : d;
+        float best = -1e30f;
+        int at = 0;
+#pragma unroll 4
+        for (int i = lane & (H - 1); i < n; i += H) {
+            const float4 v = h[i];
+            const float t = e.x * v.x + e.y * v.y + e.z * v.z;
+            if (t > best) { best = t; at = i; }
+        }
+        at = run_argmax<H>(best, at);
+        const int wA = __shfl_sync(0xffffffffu, at, g0), wB = __shfl_sync(0xffffffffu, at, g0 + H);
+        if (on) {  // (a decided group keeps what it has)
+            ia = wA;
+            ib = wB;
+            const float4 a = hA[ia], b = hB[ib];
+            s = mk3(a.x - b.x, a.y - b.y, a.z - b.z);
+        }
+    }
+    // the queries in the directions d and -d: the second one's products are the first one's negated (exactly)
+    __device__ __forceinline__ void both(f3 d, bool on, f3& S1, int& a1, int& b1, f3& S2, int& a2, int& b2) const
+    {
+        constexpr int H = LPP / 2;
+        const int lane = threadIdx.x & 31, g0 = lane & ~(LPP - 1);
+        const bool onB = (lane & H) != 0;
+        const float4* h = onB ? hB : hA;
+        const int n = !on ? 0 : onB ? nB : nA;
+        const f3 e = onB ? d * (-1.f) : d;
+        float best = -1e30f, opp = -1e30f;
+        int at = 0, oat = 0;
+#pragma unroll 4
+        for (int i = lane & (H - 1); i < n; i += H) {
+            const float4 v = h[i];
+            const float t = e.x * v.x + e.y * v.y + e.z * v.z;
+            if (t > best) { best = t; at = i; }
+            if (-t > opp) { opp = -t; oat = i; }
+        }
+        at = run_argmax<H>(best, at);
+        oat = run_argmax<H>(opp, oat);
+        a1 = __shfl_sync(0xffffffffu, at, g0);
+        b1 = __shfl_sync(0xffffffffu, at, g0 + H);
+        a2 = __shfl_sync(0xffffffffu, oat, g0);
+        b2 = __shfl_sync(0xffffffffu, oat, g0 + H);
+        if (on) {
+            const float4 p1 = hA[a1], q1 = hB[b1], p2 = hA[a2], q2 = hB[b2];
+            S1 = mk3(p1.x - q1.x, p1.y - q1.y, p1.z - q1.z);
+            S2 = mk3(p2.x - q2.x, p2.y - q2.y, p2.z - q2.z);
+        }
+    }
+};
+
+// gjk_decide of every group that is on, by a full warp; queries: the group's support queries
+template <int LPP>
+__device__ __forceinline__ int gjk_lockstep(const LockHulls<LPP>& h, bool on, f3 cA, f3 cB, SimplexRec& rec, int& queries)
+{
+    constexpr unsigned ALL = 0xffffffffu;
+    f3 S1 = mk3(0.f, 0.f, 0.f), S2 = S1, S3 = S1, S4 = S1, d3 = S1, d4 = S1;
+    int a1, b1, a2, b2, a3 = 0, b3 = 0, a4 = 0, b4 = 0, coll = -1, out = 0;
+    queries = 0;
+    const f3 d1 = cB - cA;
+    const f3 d2 = d1 * (-1.f);
+    h.both(d1, on, S1, a1, b1, S2, a2, b2);
+    if (on) {
+        queries = 1;
+        on = !(dot(d1, S1) < 0.f);
+        if (on) {
+            queries = 2;
+            on = !(dot(d2, S2) < 0.f);
+        }
+        if (on) {
+            seg_test(S1, S2, coll, d3);
+            on = coll != 0;
+        }
+    }
+    if (__any_sync(ALL, on)) {
+        h.query(d3, on, S3, a3, b3);
+        if (on) {
+            ++queries;
+            on = !(dot(d3, S3) < 0.f);
+            if (on) {
+                tri_test(S1, S2, S3, coll, d4);
+                on = coll != 0;
+            }
+        }
+        for (int zz = 0; zz < 50 && __any_sync(ALL, on); ++zz) {
+            h.query(d4, on, S4, a4, b4);
+            bool hit = false;
+            if (on) {
+                ++queries;
+                on = !(dot(d4, S4) < 0.f);
+                hit = S4.x == 0.f && S4.y == 0.f && S4.z == 0.f;
+            }
+            f3 n;
+            int todel;
+            tet_test_lanes<LPP>(S1, S2, S3, S4, coll, n, todel);
+            if (on) {
+                hit = hit || coll == 1;
+                if (hit) out = 1;
+                on = !hit && coll != 0;
+            }
+            if (on) {
+                d4 = n;
+                if (todel == 1) { S1 = S2; a1 = a2; b1 = b2; S2 = S3; a2 = a3; b2 = b3; }
+                else if (todel == 2) {
+                    const f3 t = S1;
+                    const int ta = a1, tb = b1;
+                    S1 = S3; a1 = a3; b1 = b3;
+                    S2 = t; a2 = ta; b2 = tb;
+                }
+                S3 = S4;
+                a3 = a4;
+                b3 = b4;
+            }
+        }
+        if (on) out = -1;
+    }
+    if (out == 1) {
+        rec.S[0] = f4(S1, 0.f); rec.S[1] = f4(S2, 0.f); rec.S[2] = f4(S3, 0.f); rec.S[3] = f4(S4, 0.f);
+        rec.ia = (uint32_t)a1 | ((uint32_t)a2 << 8) | ((uint32_t)a3 << 16) | ((uint32_t)a4 << 24);
+        rec.ib = (uint32_t)b1 | ((uint32_t)b2 << 8) | ((uint32_t)b3 << 16) | ((uint32_t)b4 << 24);
+    }
+    return out;
+}
+
 // ------------------------------------------------------------------ single-pass narrow phase
 // GJK by the groups of a warp, each on its own pair, then EPA by the whole warp on one after another of
 // the pairs they found in contact; the lane that leads a pair's group evaluates its force.
@@ -1142,12 +1247,12 @@ __device__ __forceinline__ void narrow_pairs(const NarrowArgs& a, int64_t P, boo
     SimplexRec rec;
     int out = 0;  // 0 separated, 1 in contact, -1 undecided
     bool ok = false;
-    if (in) {
-        ok = load_pair<MODE>(a, P, p, hA, hB, g.lane, LPP);
-        g.sync();
-        if (ok) out = gjk_decide<LPP>(g, GroupHulls<LPP>{g, hA, hB, p.nA, p.nB}, p.cA, p.cB, rec, wk);
-    }
+    if (in) ok = load_pair<MODE>(a, P, p, hA, hB, g.lane, LPP);
     __syncwarp();
+    int queries;
+    out = gjk_lockstep<LPP>(LockHulls<LPP>{hA, hB, p.nA, p.nB}, ok, p.cA, p.cB, rec, queries);
+    wk.queries = (uint32_t)queries;
+    wk.dots = ok ? (uint32_t)queries * (uint32_t)(p.nA + p.nB) : 0u;
     EpaResult er;
     er.status = 0;
     for (unsigned hits = __ballot_sync(0xffffffffu, out == 1 && g.lane == 0); hits; hits &= hits - 1) {
@@ -1284,101 +1389,111 @@ __global__ void __launch_bounds__(NARROW_THREADS) narrow_kernel(NarrowArgs a)
 // stopped -- CorrectFlat, EPA, force -- for the listed pairs only, a warp each.
 // The operation sequence per pair is the single-pass kernel's.
 
-// GJK on pair P by the group (a full warp holds the hulls in registers); lane 0 records the outcome
-// (status, contact flag, and for a pair in contact its simplex in the EPA list)
-template <int LPP>
-__device__ __forceinline__ void gjk_pair(const NarrowArgs& a, const Group<LPP>& g, int64_t P)
+// The outcome of GJK on pair P: its contact flag, and for a pair in contact its simplex in the EPA list
+__device__ __forceinline__ void gjk_outcome(const NarrowArgs& a, int64_t P, bool ok, int out, SimplexRec& rec, int queries,
+                                            int verts)
 {
-    const double4* pos = reinterpret_cast<const double4*>(a.st.pos);
-    const int2* pairs = reinterpret_cast<const int2*>(a.pairs);
-    const float4* wv = reinterpret_cast<const float4*>(a.st.world_verts);
-    SimplexRec* recs = reinterpret_cast<SimplexRec*>(a.epa_rec);
-    const int2 pr = pairs[P];
-    const double4 pa = pos[pr.x], pb = pos[pr.y];
-    const f3 cA = mk3((float)pa.x, (float)pa.y, (float)pa.z);
-    const f3 cB = mk3((float)pb.x, (float)pb.y, (float)pb.z);
-    const int oa = a.st.vert_off[pr.x], ob = a.st.vert_off[pr.y];
-    const int nA = a.st.vert_off[pr.x + 1] - oa, nB = a.st.vert_off[pr.y + 1] - ob;
-    Work3 wk = {0u, 0u, 0u};
-    SimplexRec rec;
-    int out = 0;
-    const bool ok = nA <= a.hull_cap && nB <= a.hull_cap;
-    if (ok) {
-        if constexpr (LPP == 32) {
-            WarpHulls h;
-            h.load(wv + oa, nA, wv + ob, nB);
-            out = gjk_decide<LPP>(g, h, cA, cB, rec, wk);
+    if (!ok) {
+        set_status(a.status, MWD_ST_BAD_SHAPE);
+        if (a.collision) a.collision[P] = -1;
+    } else if (out == 1) {
+        const int slot = atomicAdd(a.epa_count, 1);
+        if (slot < a.epa_cap) {
+            rec.P = P;
+            reinterpret_cast<SimplexRec*>(a.epa_rec)[slot] = rec;
         } else {
-            out = gjk_decide<LPP>(g, GroupHulls<LPP>{g, wv + oa, wv + ob, nA, nB}, cA, cB, rec, wk);
+            set_status(a.status, MWD_ST_PAIR_OVERFLOW);
         }
-    }
-    if (g.lane == 0) {
-        if (!ok) {
-            set_status(a.status, MWD_ST_BAD_SHAPE);
-            if (a.collision) a.collision[P] = -1;
-        } else if (out == 1) {
-            const int slot = atomicAdd(a.epa_count, 1);
-            if (slot < a.epa_cap) {
-                rec.P = P;
-                recs[slot] = rec;
-            } else {
-                set_status(a.status, MWD_ST_PAIR_OVERFLOW);
-            }
-            if (a.collision) a.collision[P] = 1;
-        } else {
-            // undecided pairs add zero force in the reference (.cu:1304-1319): nothing to add
-            if (out == -1) set_status(a.status, MWD_ST_GJK_NOCONV);
-            if (a.collision) a.collision[P] = out;
-        }
-        if (a.work_counters) {
-            atomicAdd(a.work_counters + 0, (unsigned long long)wk.dots);
-            atomicAdd(a.work_counters + 2, (unsigned long long)wk.queries);
-        }
-    }
-    g.sync();
-}
-
-// GJK on the candidates [base, hi) (LPP at most) by one group.  pre_culled: the broad phase already dropped
-// the pairs whose spheres are apart, and there is one candidate, which runs GJK; otherwise the candidates
-// are sphere-tested at once (one per lane) and the survivors run GJK one after another.
-template <int LPP>
-__device__ __forceinline__ void gjk_candidates(const NarrowArgs& a, const Group<LPP>& g, int64_t base, int64_t hi)
-{
-    unsigned msk;
-    if (a.pre_culled) {
-        msk = 1u;
+        if (a.collision) a.collision[P] = 1;
     } else {
-        const double4* pos = reinterpret_cast<const double4*>(a.st.pos);
-        const int2* pairs = reinterpret_cast<const int2*>(a.pairs);
-        const int64_t Pl = base + g.lane;
-        bool live = false;
-        if (Pl < hi) {
-            const int2 pr = pairs[Pl];
-            live = !spheres_apart(pos[pr.x], pos[pr.y]);
-            if (!live && a.collision) a.collision[Pl] = 0;
-        }
-        msk = g.ballot(live);
+        // undecided pairs add zero force in the reference (.cu:1304-1319): nothing to add
+        if (out == -1) set_status(a.status, MWD_ST_GJK_NOCONV);
+        if (a.collision) a.collision[P] = out;
     }
-    while (msk) {
-        const int l = __ffs(msk) - 1;
-        msk &= msk - 1;
-        gjk_pair<LPP>(a, g, base + l);
+    if (a.work_counters) {
+        atomicAdd(a.work_counters + 0, (unsigned long long)queries * (unsigned long long)verts);
+        atomicAdd(a.work_counters + 2, (unsigned long long)queries);
     }
 }
 
+// a pair's hulls and centres in the tables
+struct TablePair {
+    const float4 *hA, *hB;
+    int nA, nB;
+    f3 cA, cB;
+    bool ok;
+    __device__ __forceinline__ void load(const NarrowArgs& a, int64_t P)
+    {
+        const double4* pos = reinterpret_cast<const double4*>(a.st.pos);
+        const float4* wv = reinterpret_cast<const float4*>(a.st.world_verts);
+        const int2 pr = reinterpret_cast<const int2*>(a.pairs)[P];
+        const double4 pa = pos[pr.x], pb = pos[pr.y];
+        cA = mk3((float)pa.x, (float)pa.y, (float)pa.z);
+        cB = mk3((float)pb.x, (float)pb.y, (float)pb.z);
+        const int oa = a.st.vert_off[pr.x], ob = a.st.vert_off[pr.y];
+        nA = a.st.vert_off[pr.x + 1] - oa;
+        nB = a.st.vert_off[pr.y + 1] - ob;
+        hA = wv + oa;
+        hB = wv + ob;
+        ok = nA <= a.hull_cap && nB <= a.hull_cap;
+    }
+};
+
+// GJK on pair P (if any: on) by each group: one lane, a group of a warp in lockstep, or a warp, which holds
+// the hulls in registers
+template <int LPP>
+__device__ __forceinline__ void gjk_pair(const NarrowArgs& a, int64_t P, bool on)
+{
+    TablePair p;
+    p.hA = p.hB = nullptr;
+    p.nA = p.nB = 0;
+    p.cA = p.cB = mk3(0.f, 0.f, 0.f);
+    p.ok = false;
+    if (on) p.load(a, P);
+    SimplexRec rec;
+    int out = 0, queries = 0;
+    if constexpr (LPP == 32) {
+        if (p.ok) {
+            WarpHulls h;
+            h.load(p.hA, p.nA, p.hB, p.nB);
+            out = gjk_decide<32>(h, p.cA, p.cB, rec, queries);
+        }
+    } else if constexpr (LPP == 1) {
+        if (p.ok) out = gjk_decide<1>(LaneHulls{p.hA, p.hB, p.nA, p.nB}, p.cA, p.cB, rec, queries);
+    } else {
+        out = gjk_lockstep<LPP>(LockHulls<LPP>{p.hA, p.hB, p.nA, p.nB}, p.ok, p.cA, p.cB, rec, queries);
+    }
+    if (on && (threadIdx.x & (LPP - 1)) == 0) gjk_outcome(a, P, p.ok, out, rec, queries, p.nA + p.nB);
+    if (LPP > 1) __syncwarp();
+}
+
+// The pair list over the grid's warps, 32 / LPP pairs each at a time.  Where the broad phase has not dropped
+// the pairs whose spheres are apart (a.pre_culled), they are tested here first, a lane per candidate:
+// 32 candidates per warp when there are that many, else as many as the warp has groups.
 template <int LPP, int BT>
 __device__ __forceinline__ void gjk_stride(const NarrowArgs& a, int64_t n)
 {
-    constexpr int GPB = BT / LPP;
-    const int grp = threadIdx.x / LPP;
-    Group<LPP> g;
-    g.lane = threadIdx.x % LPP;
-    g.mask = LPP == 32 ? 0xffffffffu : (((1u << LPP) - 1u) << ((threadIdx.x & 31) / LPP * LPP));
-    // candidates a group takes at a time: one when they are pre-culled or no more than the groups
-    const int chunk = a.pre_culled || n <= (int64_t)gridDim.x * GPB ? 1 : LPP;
-    const int64_t stride = (int64_t)gridDim.x * GPB * chunk;
-    for (int64_t base = ((int64_t)blockIdx.x * GPB + grp) * chunk; base < n; base += stride)
-        gjk_candidates<LPP>(a, g, base, base + chunk < n ? base + chunk : n);
+    constexpr int G = 32 / LPP;
+    const int lane = threadIdx.x & 31, grp = lane / LPP;
+    const int64_t warps = (int64_t)gridDim.x * (BT / 32);
+    const int chunk = !a.pre_culled && n > warps * G ? 32 : G;
+    for (int64_t base = ((int64_t)blockIdx.x * (BT / 32) + threadIdx.x / 32) * chunk; base < n; base += warps * chunk) {
+        bool live = lane < chunk && base + lane < n;
+        if (live && !a.pre_culled) {
+            const double4* pos = reinterpret_cast<const double4*>(a.st.pos);
+            const int2 pr = reinterpret_cast<const int2*>(a.pairs)[base + lane];
+            live = !spheres_apart(pos[pr.x], pos[pr.y]);
+            if (!live && a.collision) a.collision[base + lane] = 0;
+        }
+        unsigned m = __ballot_sync(0xffffffffu, live);
+        while (m) {
+            // the next G survivors, one per group
+            unsigned mine = m;
+            for (int k = 0; k < grp; ++k) mine &= mine - 1;
+            gjk_pair<LPP>(a, base + (mine ? __ffs(mine) - 1 : 0), mine != 0);
+            for (int k = 0; k < G; ++k) m &= m - 1;
+        }
+    }
 }
 
 // BT threads per block (64, 128 or 256: the autotuner's block-size knob), registers capped so that
