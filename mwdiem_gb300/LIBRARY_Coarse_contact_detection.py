@@ -21,12 +21,11 @@ from ._lib import check, lib
 
 
 def _run_pairs(call, cap):
-    n_out = torch.zeros(1, dtype=torch.int64, device="cuda")
+    n_out = torch.empty(1, dtype=torch.int64, device="cuda")  # always written by the call
     while True:
         pairs = torch.empty((max(cap, 1), 2), dtype=torch.int32, device="cuda")
         call(pairs, cap, n_out)
-        torch.cuda.current_stream().synchronize()
-        n = int(n_out.item())
+        n = int(n_out.item())  # waits for the call
         if n < cap or cap == 0 and n == 0:
             return pairs[:n]
         if n == cap:

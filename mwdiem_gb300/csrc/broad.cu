@@ -1021,7 +1021,7 @@ __global__ void keys_kernel(int N, const double* com, double csx, double csy, do
 
 __global__ void minmax_kernel(const int64_t* keys, int lo, int hi, unsigned long long* mm)
 {
-    // mm[0] = min, mm[1] = max of keys in [lo, hi), as order-preserving unsigned values
+    // mm[0] = min, mm[1] = ~max of keys in [lo, hi), as order-preserving unsigned values (both ~0 before)
     const int i = lo + blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long v_min = ~0ull, v_max = 0ull;
     if (i < hi) {
@@ -1036,9 +1036,12 @@ __global__ void minmax_kernel(const int64_t* keys, int lo, int hi, unsigned long
     }
     if ((threadIdx.x & 31) == 0 && i - (int)(threadIdx.x & 31) < hi) {
         atomicMin(mm, v_min);
-        atomicMax(mm + 1, v_max);
+        atomicMin(mm + 1, ~v_max);
     }
 }
+
+// a scene from the launch's arguments: no copy from host memory that would have to outlive the call
+__global__ void put_scene_kernel(mwd_scene* dst, const __grid_constant__ mwd_scene sc) { *dst = sc; }
 
 inline unsigned blocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
@@ -1192,9 +1195,17 @@ int launch_keys(int N, const double* com, double csx, double csy, double csz, in
     return MWD_OK;
 }
 
+int launch_put_scene(mwd_scene* dst, const mwd_scene& sc, cudaStream_t s)
+{
+    put_scene_kernel<<<1, 1, 0, s>>>(dst, sc);
+    MWD_CUDA(cudaGetLastError());
+    return MWD_OK;
+}
+
 int launch_minmax(const int64_t* keys, int lo, int hi, unsigned long long* mm, cudaStream_t s)
 {
     if (hi <= lo) return MWD_OK;
+    MWD_CUDA(cudaMemsetAsync(mm, 0xff, 2 * sizeof(*mm), s));
     minmax_kernel<<<blocks(hi - lo, 256), 256, 0, s>>>(keys, lo, hi, mm);
     MWD_CUDA(cudaGetLastError());
     return MWD_OK;

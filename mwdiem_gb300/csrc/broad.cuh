@@ -57,6 +57,8 @@ int broad_sparse(int64_t rows, int64_t total_cells, int64_t tile_sum_ints, int m
 void broad_table_ints(int64_t rows, int64_t total_cells, int sparse, int64_t* count_ints, int64_t* start_ints);
 int launch_keys(int N, const double* com, double csx, double csy, double csz, int64_t nx, int64_t ny, int64_t* keys,
                 cudaStream_t s);
+int launch_put_scene(mwd_scene* dst, const mwd_scene& sc, cudaStream_t s);
+// mm[0] = min, mm[1] = ~max of the keys, sign bit flipped
 int launch_minmax(const int64_t* keys, int lo, int hi, unsigned long long* mm, cudaStream_t s);
 int launch_wall_pairs(int n_wall, int n_lo, int n_hi, const double* com, const double* wn, const double* wc,
                       double range, int32_t* flags, int32_t* offs, int32_t* tmp, int32_t* pairs, int64_t cap,

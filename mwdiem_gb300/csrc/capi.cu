@@ -420,14 +420,13 @@ int mwd_linked_cell_hash(int32_t n_lo, int32_t n_hi, const int64_t* keys, int64_
     void* base;
     int rc = scratch(4096, &base);
     if (rc) return rc;
-    unsigned long long init[2] = {~0ull, 0ull}, mm[2];
-    MWD_CUDA(cudaMemcpyAsync(base, init, sizeof(init), cudaMemcpyHostToDevice, s));
+    unsigned long long mm[2];
     rc = launch_minmax(keys, n_lo, n_hi, reinterpret_cast<unsigned long long*>(base), s);
     if (rc) return rc;
     MWD_CUDA(cudaMemcpyAsync(mm, base, sizeof(mm), cudaMemcpyDeviceToHost, s));
     MWD_CUDA(cudaStreamSynchronize(s));
     const int64_t kmin = (int64_t)(mm[0] ^ 0x8000000000000000ull);
-    const int64_t kmax = (int64_t)(mm[1] ^ 0x8000000000000000ull);
+    const int64_t kmax = (int64_t)(~mm[1] ^ 0x8000000000000000ull);
     const int64_t R = kmax - kmin + 1;
     const int64_t rows = n_hi - n_lo;
     const int64_t m = (R > rows ? R : rows) + 1;
@@ -460,7 +459,8 @@ int mwd_linked_cell_hash(int32_t n_lo, int32_t n_hi, const int64_t* keys, int64_
     sc.key_min = kmin;
     sc.n_keys = R;
     sc.cell_base = 0;
-    MWD_CUDA(cudaMemcpyAsync(b + o_scene, &sc, sizeof(sc), cudaMemcpyHostToDevice, s));
+    rc = launch_put_scene(reinterpret_cast<mwd_scene*>(b + o_scene), sc, s);
+    if (rc) return rc;
     MWD_CUDA(cudaMemsetAsync(b + o_tmp, 0, o_count - o_tmp + count_ints * sizeof(int32_t), s));
     int32_t* tile_sums = reinterpret_cast<int32_t*>(b + o_tmp) + scan_tile_sums_offset(m);
     BroadArgs a = {};
@@ -485,7 +485,7 @@ int mwd_linked_cell_hash(int32_t n_lo, int32_t n_hi, const int64_t* keys, int64_
     a.sparse = sparse;
     rc = launch_broad(a, s);
     if (rc) return rc;
-    // the host copy of the scene must outlive the async copy
+    // the scratch is free again when the call returns, for calls on other streams too
     MWD_CUDA(cudaStreamSynchronize(s));
     return MWD_OK;
 }
