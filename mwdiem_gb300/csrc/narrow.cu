@@ -900,9 +900,35 @@ struct PairView {
     int wall;
 };
 
-template <int MODE>
-__device__ __forceinline__ bool load_pair(const NarrowArgs& a, int64_t P, PairView& p, float4* hA, float4* hB,
-                                          int lane, int lpp, bool stage = true)
+// Both hulls of a pair into the group's staging area, 32 vertices of each at a time, all their loads in
+// flight at once (a vertex per lane and round trip, the drop-in kernel waited for nine of them in a row:
+// 122k candidate pairs 122 us).  at(v, i): vertex i of hull v.
+template <int LPP, class At>
+__device__ __forceinline__ void stage_hulls(float4* hA, int nA, float4* hB, int nB, int lane, At&& at)
+{
+    constexpr int U = LPP < 32 ? 32 / LPP : 2;
+    const int most = max(nA, nB);
+    for (int base = lane; base < most; base += U * LPP) {
+        float4 x[U], y[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = base + u * LPP;
+            x[u] = y[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < nA) x[u] = at(0, i);
+            if (i < nB) y[u] = at(1, i);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = base + u * LPP;
+            if (i < nA) hA[i] = x[u];
+            if (i < nB) hB[i] = y[u];
+        }
+    }
+}
+
+// LPP: lanes of the group that stages the hulls (0: not staged)
+template <int MODE, int LPP>
+__device__ __forceinline__ bool load_pair(const NarrowArgs& a, int64_t P, PairView& p, float4* hA, float4* hB, int lane)
 {
     if (MODE == 0) {
         const float* c;
@@ -925,8 +951,11 @@ __device__ __forceinline__ bool load_pair(const NarrowArgs& a, int64_t P, PairVi
         if (p.nA < 0 || p.nB < 0 || p.nA > a.hull_cap || p.nB > a.hull_cap) return false;
         const float* va = a.A_verts + P * a.V * 3;
         const float* vb = a.B_verts + P * a.V * 3;
-        for (int i = lane; i < p.nA; i += lpp) hA[i] = make_float4(va[3 * i], va[3 * i + 1], va[3 * i + 2], 0.f);
-        for (int i = lane; i < p.nB; i += lpp) hB[i] = make_float4(vb[3 * i], vb[3 * i + 1], vb[3 * i + 2], 0.f);
+        if constexpr (LPP > 0)
+            stage_hulls<LPP>(hA, p.nA, hB, p.nB, lane, [&](int v, int i) {
+                const float* x = (v ? vb : va) + 3 * i;
+                return make_float4(x[0], x[1], x[2], 0.f);
+            });
     } else {
         int2 pr = reinterpret_cast<const int2*>(a.pairs)[P];
         p.idA = pr.x;
@@ -950,10 +979,9 @@ __device__ __forceinline__ bool load_pair(const NarrowArgs& a, int64_t P, PairVi
         p.nA = a.st.vert_off[p.idA + 1] - oa;
         p.nB = a.st.vert_off[p.idB + 1] - ob;
         if (p.nA > a.hull_cap || p.nB > a.hull_cap) return false;
-        if (stage) {
+        if constexpr (LPP > 0) {
             const float4* wv = reinterpret_cast<const float4*>(a.st.world_verts);
-            for (int i = lane; i < p.nA; i += lpp) hA[i] = wv[oa + i];
-            for (int i = lane; i < p.nB; i += lpp) hB[i] = wv[ob + i];
+            stage_hulls<LPP>(hA, p.nA, hB, p.nB, lane, [&](int v, int i) { return wv[(v ? ob : oa) + i]; });
         }
     }
     p.dtn = sqrtf(p.dt.x * p.dt.x + p.dt.y * p.dt.y + p.dt.z * p.dt.z);
@@ -1310,7 +1338,7 @@ __device__ __forceinline__ void narrow_pairs(const NarrowArgs& a, int64_t P, boo
     GjkState gs;
     int out = 0;  // 0 separated, 1 in contact, -1 undecided
     bool ok = false;
-    if (in) ok = load_pair<MODE>(a, P, p, hA, hB, g.lane, LPP);
+    if (in) ok = load_pair<MODE, LPP>(a, P, p, hA, hB, g.lane);
     __syncwarp();
     int queries;
     out = gjk_lockstep<LPP>(LockHulls<LPP>{hA, hB, p.nA, p.nB}, ok, p.cA, p.cB, gs, queries);
@@ -1698,7 +1726,7 @@ __device__ __noinline__ void epa_flush(const NarrowArgs& a, const EpaDone* done,
         const int64_t i = (int64_t)__float_as_uint(e.c.w);
         const int64_t P = reinterpret_cast<const SimplexRec*>(a.epa_rec)[i].P;
         PairView p;
-        load_pair<1>(a, P, p, nullptr, nullptr, 0, 1, false);
+        load_pair<1, 0>(a, P, p, nullptr, nullptr, 0);
         const float4* wv = reinterpret_cast<const float4*>(a.st.world_verts);
         EpaResult er;
         er.depth = e.nd.w;
