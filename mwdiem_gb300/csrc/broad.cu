@@ -422,6 +422,15 @@ __device__ __forceinline__ int2 cell_range(const BroadArgs& a, int g)
     return make_int2(st[c], st[c + 1]);
 }
 
+// position in the sorted list of the first row in cell g or a later one (g up to total_cells)
+__device__ __forceinline__ int list_start(const BroadArgs& a, int64_t g)
+{
+    if (!a.sparse) return a.cell_start[g];
+    const int word = (int)(g >> 5);
+    if (word >= a.n_words) return occ_start(a)[a.cell_start[a.n_words]];
+    return occ_start(a)[a.cell_start[word] + __popc(occ_copy(a)[word] & ((1u << (g & 31)) - 1u))];
+}
+
 // rows in the sorted list (those with a cell)
 __device__ __forceinline__ int n_sorted_rows(const BroadArgs& a)
 {
@@ -738,14 +747,6 @@ __global__ void __launch_bounds__(PLACE_THREADS) place_kernel(BroadArgs a)
 
 // walls of one scene staged as floats (centre + radius, normal) by the append kernel
 constexpr int WALL_STAGE = 16;
-struct WallStage {
-    const float4* c;  // (nw,) centre, bounding radius
-    const float4* n;  // (nw,) normal, and n . c in float
-    const float2* m;  // (nw,) |n|_1, and |c|_1 |n|_1 + range: the parts of the margin fixed per wall
-    int scene;        // the scene they belong to (-1: nothing staged)
-    int nw;
-};
-
 // the reference's forward stencil in linear keys, o = 0..6: +1, +nx, +nx*ny, +nx*ny+1, +nx*ny+1+nx,
 // +nx*ny+nx, +nx+1 (LIBRARY_Coarse_contact_detection.py:96-129), from bit masks (no local array)
 __device__ __forceinline__ int64_t forward_offset(int o, int64_t nx, int64_t nxy)
@@ -753,74 +754,112 @@ __device__ __forceinline__ int64_t forward_offset(int o, int64_t nx, int64_t nxy
     return (((0x3c >> o) & 1) ? nxy : 0) + (((0x72 >> o) & 1) ? nx : 0) + ((0x59 >> o) & 1);
 }
 
-// every candidate of the row at sorted position t (row r, cell g), passed to sink(A, B).
-// ws: optional float copies of the row's scene walls for the wall-distance test.
-// part: -1 the whole walk; 0 the walls and the later members of the row's own cell; 1..7 the
-// members of forward neighbour cell part - 1 (the eight parts together are the whole walk).
-// what: WALK_WALLS, WALK_CELLS or both (walls first).
-constexpr int WALK_WALLS = 1, WALK_CELLS = 2;
-template <class Sink>
-__device__ __forceinline__ void walk_pairs(const BroadArgs& a, int t, int r, int g, const mwd_scene& sc, int scene,
-                                           const WallStage* ws, Sink&& sink, int part = -1,
-                                           int what = WALK_WALLS | WALK_CELLS)
+// The walls of the scene of the block's first row (sorted position t0), as floats, staged by the first warp
+// alone: its lane 0 finds the scene, its lanes copy one wall each; the other warps go on to their cells, and
+// every thread tests the walls after a block barrier.
+struct WallStageMem {
+    float4 c[WALL_STAGE], n[WALL_STAGE];
+    float2 m[WALL_STAGE];
+    int scene, nw;
+};
+__device__ __forceinline__ void stage_walls(const BroadArgs& a, WallStageMem& s, int t0, int n_sorted)
 {
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    int sc0 = -1, nw = 0;
+    if (lane == 0 && a.walls && a.sorted_pos && t0 < n_sorted) {
+        sc0 = scene_of(a, a.sorted[t0]);
+        const mwd_scene& sc = a.scenes[sc0];
+        nw = sc.wall_end - sc.row_begin;
+        if (nw > WALL_STAGE) sc0 = -1;
+    }
+    sc0 = __shfl_sync(0xffffffffu, sc0, 0);
+    nw = __shfl_sync(0xffffffffu, nw, 0);
+    if (sc0 >= 0 && lane < nw) {
+        const mwd_scene& sc = a.scenes[sc0];
+        const int w = sc.row_begin + lane;
+        const dpos c = reinterpret_cast<const dpos*>(a.pos)[w];
+        const dpos n = reinterpret_cast<const dpos*>(a.wall_normal)[w];
+        const float4 cf = make_float4((float)c.x, (float)c.y, (float)c.z, (float)c.w);
+        const float4 nf = make_float4((float)n.x, (float)n.y, (float)n.z, 0.f);
+        const float n1 = fabsf(nf.x) + fabsf(nf.y) + fabsf(nf.z);
+        s.c[lane] = cf;
+        s.n[lane] = make_float4(nf.x, nf.y, nf.z, nf.x * cf.x + nf.y * cf.y + nf.z * cf.z);
+        s.m[lane] = make_float2(n1, (fabsf(cf.x) + fabsf(cf.y) + fabsf(cf.z)) * n1 + (float)sc.wall_range);
+    }
+    if (lane == 0) {
+        s.scene = sc0;
+        s.nw = nw;
+    }
+}
+
+// The wall candidates of row r (MWDiem.py:808-811): pair [particle, wall] when |n . (p - c)| < wall_range in
+// FP64; walls first, first + step, ... of its scene.  me: its centre and radius.
+template <class Sink>
+__device__ __forceinline__ void walk_walls(const BroadArgs& a, int r, const mwd_scene& sc, int scene, float4 me,
+                                           const WallStageMem& ws, int first, int step, Sink&& sink)
+{
+    if (!a.walls) return;
     const bool cull = a.cull && a.sorted_pos;
-    const float4 me = a.sorted_pos ? a.sorted_pos[t] : make_float4(0.f, 0.f, 0.f, 0.f);
-    // wall candidates (MWDiem.py:808-811): pair [particle, wall] when |n . (p - c)| < wall_range (FP64)
-    if (a.walls && part <= 0 && (what & WALK_WALLS)) {
-        if (ws && ws->scene == scene && a.sorted_pos) {
-            // FP32 test with a margin above its rounding error: s = n . p - n . c with the inputs rounded
-            // to float, three products, three sums and n . c rounded once at staging is within
-            // 6 u |n|_1 (|p|_1 + |c|_1) of the exact value (u = 2^-24); the margin, 1e-6 (~16.8 u) times
-            // that sum plus the range, covers it with room.  Inside the margin band the FP64 test decides.
-            const float range = (float)sc.wall_range;
-            const float me1 = fabsf(me.x) + fabsf(me.y) + fabsf(me.z);
-            for (int k = 0; k < ws->nw; ++k) {
-                const float4 c = ws->c[k], nr = ws->n[k];
-                const float2 wm = ws->m[k];
-                const float sf = (nr.x * me.x + nr.y * me.y + nr.z * me.z) - nr.w;
-                const float mg = 1e-6f * (me1 * wm.x + wm.y);
-                bool in;
-                if (fabsf(sf) < range - mg) in = true;
-                else if (fabsf(sf) > range + mg) in = false;
-                else {
-                    const int w = sc.row_begin + k;
-                    const dpos p = reinterpret_cast<const dpos*>(a.pos)[r];
-                    const dpos wc = reinterpret_cast<const dpos*>(a.pos)[w];
-                    const dpos wn = reinterpret_cast<const dpos*>(a.wall_normal)[w];
-                    const double s = wn.x * (p.x - wc.x) + wn.y * (p.y - wc.y) + wn.z * (p.z - wc.z);
-                    in = fabs(s) < sc.wall_range;
-                }
-                // optional exact-outcome filter: pairs the reference's GJK rejects at its first test
-                if (in && !(cull && spheres_apart_f(me, c))) sink(r, sc.row_begin + k);
+    if (ws.scene == scene && a.sorted_pos) {
+        // FP32 test with a margin above its rounding error: s = n . p - n . c with the inputs rounded
+        // to float, three products, three sums and n . c rounded once at staging is within
+        // 6 u |n|_1 (|p|_1 + |c|_1) of the exact value (u = 2^-24); the margin, 1e-6 (~16.8 u) times
+        // that sum plus the range, covers it with room.  Inside the margin band the FP64 test decides.
+        const float range = (float)sc.wall_range;
+        const float me1 = fabsf(me.x) + fabsf(me.y) + fabsf(me.z);
+        for (int k = first; k < ws.nw; k += step) {
+            const float4 c = ws.c[k], nr = ws.n[k];
+            const float2 wm = ws.m[k];
+            const float sf = (nr.x * me.x + nr.y * me.y + nr.z * me.z) - nr.w;
+            const float mg = 1e-6f * (me1 * wm.x + wm.y);
+            bool in;
+            if (fabsf(sf) < range - mg) in = true;
+            else if (fabsf(sf) > range + mg) in = false;
+            else {
+                const int w = sc.row_begin + k;
+                const dpos p = reinterpret_cast<const dpos*>(a.pos)[r];
+                const dpos wc = reinterpret_cast<const dpos*>(a.pos)[w];
+                const dpos wn = reinterpret_cast<const dpos*>(a.wall_normal)[w];
+                const double s = wn.x * (p.x - wc.x) + wn.y * (p.y - wc.y) + wn.z * (p.z - wc.z);
+                in = fabs(s) < sc.wall_range;
             }
-        } else {
-            const dpos p = reinterpret_cast<const dpos*>(a.pos)[r];
-            for (int k = sc.row_begin; k < sc.wall_end; ++k) {
-                const dpos wc = reinterpret_cast<const dpos*>(a.pos)[k];
-                const dpos wn = reinterpret_cast<const dpos*>(a.wall_normal)[k];
-                double s = wn.x * (p.x - wc.x) + wn.y * (p.y - wc.y) + wn.z * (p.z - wc.z);
-                if (!(fabs(s) < sc.wall_range)) continue;
-                if (cull) {
-                    const float4 pb = make_float4((float)wc.x, (float)wc.y, (float)wc.z, (float)wc.w);
-                    if (spheres_apart_f(me, pb)) continue;
-                }
-                sink(r, k);
+            // optional exact-outcome filter: pairs the reference's GJK rejects at its first test
+            if (in && !(cull && spheres_apart_f(me, c))) sink(r, sc.row_begin + k);
+        }
+    } else {
+        const dpos p = reinterpret_cast<const dpos*>(a.pos)[r];
+        for (int k = sc.row_begin + first; k < sc.wall_end; k += step) {
+            const dpos wc = reinterpret_cast<const dpos*>(a.pos)[k];
+            const dpos wn = reinterpret_cast<const dpos*>(a.wall_normal)[k];
+            double s = wn.x * (p.x - wc.x) + wn.y * (p.y - wc.y) + wn.z * (p.z - wc.z);
+            if (!(fabs(s) < sc.wall_range)) continue;
+            if (cull) {
+                const float4 pb = make_float4((float)wc.x, (float)wc.y, (float)wc.z, (float)wc.w);
+                if (spheres_apart_f(me, pb)) continue;
             }
+            sink(r, k);
         }
     }
-    if (!(what & WALK_CELLS)) return;
+}
+
+// The cell candidates of the row at sorted position t (row r, cell g) in the reference's order: the later
+// members of its cell in set order, then those of the 7 forward neighbours.  part: -1 all of them; 0 the
+// row's own cell; 1..7 forward neighbour part - 1.
+template <class Sink>
+__device__ __forceinline__ void walk_cells(const BroadArgs& a, int t, int r, int g, const mwd_scene& sc, float4 me, int part,
+                                           Sink&& sink)
+{
+    const bool cull = a.cull && a.sorted_pos;
     auto put = [&](int B, int j) {
         if (cull && spheres_apart_f(me, a.sorted_pos[j])) return;
         sink(r, B);
     };
-    // later members of the same cell, in set order
     if (part <= 0) {
         const int ce = cell_range(a, g).y;
         for (int j = t + 1; j < ce; ++j) put(a.sorted[j], j);
     }
     if (part == 0) return;
-    // forward neighbours
     const int64_t local = (int64_t)g - sc.cell_base;
     const int64_t nx = sc.nx, nxy = sc.nx * sc.ny;
     if (part > 0) {
@@ -846,111 +885,148 @@ __device__ __forceinline__ void walk_pairs(const BroadArgs& a, int t, int r, int
         for (int j = rs[o]; j < re[o]; ++j) put(a.sorted[j], j);
 }
 
-// EMIT false: the candidates of each row, and (scan_tmp, zeroed by assign_kernel) of each tile of the
-// scan that follows; EMIT true: the pairs themselves, at the offsets that the scan left in pair_count
+// The same candidates in any order: a cell and the next one are neighbours in the sorted list too, so the row's
+// own cell and the seven forward ones are four ranges of it (the offsets 0 and 1, nx and nx + 1, nx ny and
+// nx ny + 1, nx ny + nx and nx ny + nx + 1).  part: -1 all four; 0..3 one of them.
+template <class Sink>
+__device__ __forceinline__ void walk_ranges(const BroadArgs& a, int t, int r, int g, const mwd_scene& sc, float4 me, int part,
+                                            Sink&& sink)
+{
+    const bool cull = a.cull && a.sorted_pos;
+    const int64_t local = (int64_t)g - sc.cell_base;
+    const int64_t nx = sc.nx, nxy = sc.nx * sc.ny;
+    auto range = [&](int k) {
+        const int64_t l2 = local + ((k & 1) ? nx : 0) + ((k & 2) ? nxy : 0);
+        if (l2 < 0 || l2 >= sc.n_keys) return make_int2(0, 0);
+        const int64_t hi = l2 + 2 < sc.n_keys ? l2 + 2 : sc.n_keys;
+        int2 se = make_int2(k == 0 ? t + 1 : list_start(a, sc.cell_base + l2), list_start(a, sc.cell_base + hi));
+        return se;
+    };
+    auto walk = [&](int2 se) {
+        for (int j = se.x; j < se.y; ++j) {
+            if (cull && spheres_apart_f(me, a.sorted_pos[j])) continue;
+            sink(r, a.sorted[j]);
+        }
+    };
+    if (part >= 0) {
+        walk(range(part));
+        return;
+    }
+    int2 se[4];  // loaded first (independent loads), then walked
+#pragma unroll
+    for (int k = 0; k < 4; ++k) se[k] = range(k);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) walk(se[k]);
+}
+
+constexpr int APPEND_THREADS = 128;
+constexpr int APPEND_KEEP = 8;  // pairs a thread keeps from its walk; threads with more walk again
+
+// Threads per row of the pair kernels while the rows alone leave the GPU short of threads (a step of tens of
+// thousands of rows is bound by the chain of dependent loads per thread); with many rows one thread per row
+// does less redundant work.
+constexpr int ORDERED_PARTS = 8;  // walls and own cell, and each forward neighbour cell
+constexpr int APPEND_PARTS = 4;   // each range of walk_ranges, and every fourth wall
+
+// The list in cell order, each row's walls first.  EMIT false: the candidates of each row, and (scan_tmp,
+// zeroed by assign_kernel) of each tile of the scan that follows; EMIT true: the pairs themselves, at the
+// offsets that the scan left in pair_count.  A row's threads (1 or 8) count their shares and add them up in
+// order.  (5,003 packed hulls: 6.7 and 7.9 us; 11.7 and 16.5 with one thread per row and FP64 wall tests.)
 template <bool EMIT>
-__global__ void pairs_kernel(BroadArgs a)
+__global__ void __launch_bounds__(APPEND_THREADS) pairs_kernel(BroadArgs a)
 {
     pdl_wait();
     pdl_launch_dependents();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = t < n_sorted_rows(a);
+    __shared__ int2 keep[EMIT ? APPEND_KEEP : 1][APPEND_THREADS];
+    __shared__ WallStageMem ws;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool split = a.walk_parts > 1;
+    const int t = split ? tid / ORDERED_PARTS : tid;
+    const int part = split ? tid % ORDERED_PARTS : -1;
+    const int n_sorted = n_sorted_rows(a);
+    stage_walls(a, ws, (int)(blockIdx.x * blockDim.x) / (split ? ORDERED_PARTS : 1), n_sorted);
+    const bool live = t < n_sorted;
     const int r = live ? a.sorted[t] : 0;
     const int g = !live ? 0 : a.sorted_cell ? a.sorted_cell[t] : a.cell_of[r];
     const int scene = live ? scene_of(a, r) : 0;
     const mwd_scene& sc = a.scenes[scene];
-    if (EMIT) {
+    const float4 me = live && a.sorted_pos ? a.sorted_pos[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    auto walk = [&](auto&& sink) {
         if (!live) return;
-        int64_t out = a.pair_count[t];
+        if (part <= 0) walk_walls(a, r, sc, scene, me, ws, 0, 1, sink);
+        walk_cells(a, t, r, g, sc, me, part, sink);
+    };
+    int c = 0;
+    walk([&](int A, int B) {
+        if (EMIT && c < APPEND_KEEP) keep[c][threadIdx.x] = make_int2(A, B);
+        ++c;
+    });
+    int inc = c;  // candidates of the row up to this thread's share
+    if (split) {
+#pragma unroll
+        for (int o = 1; o < ORDERED_PARTS; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, inc, o, ORDERED_PARTS);
+            if ((tid & (ORDERED_PARTS - 1)) >= o) inc += y;
+        }
+    }
+    if (EMIT) {
+        if (!live || c == 0) return;
+        const int64_t out = (int64_t)a.pair_count[t] + inc - c;
         const int64_t cap = a.pair_cap;
         int2* pairs = reinterpret_cast<int2*>(a.pairs);
-        walk_pairs(a, t, r, g, sc, scene, nullptr, [&](int A, int B) {
-            if (out < cap) pairs[out] = make_int2(A, B);
-            ++out;
-        });
+        const int kept = c < APPEND_KEEP ? c : APPEND_KEEP;
+        for (int i = 0; i < kept; ++i)
+            if (out + i < cap) pairs[out + i] = keep[i][threadIdx.x];
+        if (c > APPEND_KEEP) {
+            int i = 0;
+            walk([&](int A, int B) {
+                if (i >= APPEND_KEEP && out + i < cap) pairs[out + i] = make_int2(A, B);
+                ++i;
+            });
+        }
     } else {
-        int c = 0;
-        if (live) walk_pairs(a, t, r, g, sc, scene, nullptr, [&](int, int) { ++c; });
-        if (t < a.row_hi - a.row_lo) a.pair_count[t] = c;
+        if (t < a.row_hi - a.row_lo && (!split || part == ORDERED_PARTS - 1)) a.pair_count[t] = inc;
         const int sum = __reduce_add_sync(0xffffffffu, c);
         if ((threadIdx.x & 31) == 0 && sum) atomicAdd(a.scan_tmp + t / SCAN_TILE, sum);
     }
 }
 
-constexpr int APPEND_THREADS = 128;
-constexpr int APPEND_KEEP = 8;   // pairs a thread keeps from its walk; threads with more walk again
-constexpr int APPEND_PARTS = 8;  // threads per row: walls + own cell, and each forward neighbour cell
-
-// one walk (the first APPEND_KEEP pairs kept in shared memory), reserve (one atomic per warp on
-// n_pairs, zeroed by assign_kernel), write.  With walk_parts = APPEND_PARTS each row's walk is split
-// over that many threads (its own cell and walls, and one per forward neighbour), so the chain of
-// dependent loads per thread is short (a 20k-row step: 72.9 -> 68.7 us); with many rows one thread
-// per row does less redundant work (2M rows: 1.33 -> 0.99 ms).  The list order is arbitrary anyway
-// in this mode.
+// one walk (the first APPEND_KEEP pairs kept in shared memory), reserve (one atomic per warp on n_pairs, zeroed
+// by assign_kernel), write.  With walk_parts = APPEND_PARTS each row's walk is split over that many threads.
+// The list order is arbitrary in this mode.  (The four ranges against eight cells: 30,011 packed hulls 14.5 ->
+// 9.7 us, a pour of 20,000 8.7 -> 6.8, 256 scenes of 2.0M rows 93 -> 87.)
 __global__ void __launch_bounds__(APPEND_THREADS) pairs_append_kernel(BroadArgs a)
 {
     pdl_wait();
     pdl_launch_dependents();
     __shared__ int2 keep[APPEND_KEEP][APPEND_THREADS];
-    __shared__ float4 s_wc[WALL_STAGE], s_wn[WALL_STAGE];
-    __shared__ float2 s_wm[WALL_STAGE];
-    __shared__ int s_scene, s_nw;
+    __shared__ WallStageMem ws;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int t = a.walk_parts > 1 ? tid / APPEND_PARTS : tid;
-    const int part = a.walk_parts > 1 ? tid % APPEND_PARTS : -1;
+    const bool split = a.walk_parts > 1;
+    const int t = split ? tid / APPEND_PARTS : tid;
+    const int part = split ? tid % APPEND_PARTS : -1;
     const int n_sorted = n_sorted_rows(a);
     const bool live = t < n_sorted;
-    // the walls of the scene of the block's first row, as floats, staged by the first warp alone
-    // (its lane 0 finds the scene, its lanes copy one wall each); the other warps walk the cells
-    // meanwhile, and every thread tests the walls after one block barrier
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        int sc0 = -1, nw = 0;
-        const int t0 = blockIdx.x * blockDim.x / (a.walk_parts > 1 ? APPEND_PARTS : 1);
-        if (lane == 0 && a.walls && a.sorted_pos && t0 < n_sorted) {
-            sc0 = scene_of(a, a.sorted[t0]);
-            const mwd_scene& sc = a.scenes[sc0];
-            nw = sc.wall_end - sc.row_begin;
-            if (nw > WALL_STAGE) sc0 = -1;
-        }
-        sc0 = __shfl_sync(0xffffffffu, sc0, 0);
-        nw = sc0 >= 0 ? __shfl_sync(0xffffffffu, nw, 0) : 0;
-        if (lane < nw) {
-            const mwd_scene& sc = a.scenes[sc0];
-            const int w = sc.row_begin + lane;
-            const dpos c = reinterpret_cast<const dpos*>(a.pos)[w];
-            const dpos n = reinterpret_cast<const dpos*>(a.wall_normal)[w];
-            const float4 cf = make_float4((float)c.x, (float)c.y, (float)c.z, (float)c.w);
-            const float4 nf = make_float4((float)n.x, (float)n.y, (float)n.z, 0.f);
-            const float n1 = fabsf(nf.x) + fabsf(nf.y) + fabsf(nf.z);
-            s_wc[lane] = cf;
-            s_wn[lane] = make_float4(nf.x, nf.y, nf.z, nf.x * cf.x + nf.y * cf.y + nf.z * cf.z);
-            s_wm[lane] = make_float2(n1, (fabsf(cf.x) + fabsf(cf.y) + fabsf(cf.z)) * n1 + (float)sc.wall_range);
-        }
-        if (lane == 0) {
-            s_scene = sc0;
-            s_nw = nw;
-        }
-    }
-    const WallStage ws = {s_wc, s_wn, s_wm, -1, 0};  // scene and count read after the barrier
+    stage_walls(a, ws, (int)(blockIdx.x * blockDim.x) / (split ? APPEND_PARTS : 1), n_sorted);
     int r = 0, g = 0, c = 0, scene = 0;
     const mwd_scene* sc = nullptr;
+    float4 me = make_float4(0.f, 0.f, 0.f, 0.f);
     auto keep_pair = [&](int A, int B) {
         if (c < APPEND_KEEP) keep[c][threadIdx.x] = make_int2(A, B);
         ++c;
     };
+    auto walls = [&](auto&& sink) { walk_walls(a, r, *sc, scene, me, ws, split ? part : 0, split ? APPEND_PARTS : 1, sink); };
     if (live) {
         r = a.sorted[t];
         g = a.sorted_cell ? a.sorted_cell[t] : a.cell_of[r];
+        if (a.sorted_pos) me = a.sorted_pos[t];
         scene = scene_of(a, r);
         sc = &a.scenes[scene];
-        walk_pairs(a, t, r, g, *sc, scene, &ws, keep_pair, part, WALK_CELLS);
+        walk_ranges(a, t, r, g, *sc, me, part, keep_pair);
     }
     __syncthreads();
-    WallStage wst = ws;
-    wst.scene = s_scene;
-    wst.nw = s_nw;
-    if (live) walk_pairs(a, t, r, g, *sc, scene, &wst, keep_pair, part, WALK_WALLS);
+    if (live) walls(keep_pair);
     const int lane = threadIdx.x & 31;
     int inc = c;
 #pragma unroll
@@ -976,8 +1052,8 @@ __global__ void __launch_bounds__(APPEND_THREADS) pairs_append_kernel(BroadArgs 
             if (i >= APPEND_KEEP && out + i < cap) pairs[out + i] = make_int2(A, B);
             ++i;
         };
-        walk_pairs(a, t, r, g, *sc, scene, &wst, write_rest, part, WALK_CELLS);
-        walk_pairs(a, t, r, g, *sc, scene, &wst, write_rest, part, WALK_WALLS);
+        walk_ranges(a, t, r, g, *sc, me, part, write_rest);
+        walls(write_rest);
     }
 }
 
@@ -1166,23 +1242,22 @@ int launch_broad(const BroadArgs& a_in, cudaStream_t s)
     else
         MWD_CUDA(launch_pdl(place_kernel<false>, blocks(rows, PLACE_THREADS), PLACE_THREADS, 0, s, a));
     // rows that have a cell are at most `rows`; threads past cell_start[total] exit
+    BroadArgs b = a;
+    const bool split = rows * ORDERED_PARTS <= 4 * (int64_t)num_sms() * 2048;
     if (a.append) {
-        // split each row's walk over APPEND_PARTS threads while the rows alone leave the GPU short of
-        // threads (a latency-bound step); with many rows one thread per row does less redundant work
-        BroadArgs b = a;
-        const int64_t resident = (int64_t)num_sms() * 2048;
-        b.walk_parts = rows * APPEND_PARTS <= 4 * resident ? APPEND_PARTS : 1;
+        b.walk_parts = split ? APPEND_PARTS : 1;
         MWD_CUDA(launch_pdl(pairs_append_kernel, blocks(rows * b.walk_parts, APPEND_THREADS), APPEND_THREADS, 0, s,
                             b));
-        MWD_CUDA(cudaGetLastError());
         return MWD_OK;
     }
-    MWD_CUDA(launch_pdl(pairs_kernel<false>, blocks(rows, T), T, 0, s, a));
+    b.walk_parts = split ? ORDERED_PARTS : 1;
+    const unsigned grid = blocks(rows * b.walk_parts, APPEND_THREADS);
+    MWD_CUDA(launch_pdl(pairs_kernel<false>, grid, APPEND_THREADS, 0, s, b));
     const int nb = (int)((rows + SCAN_TILE - 1) / SCAN_TILE);
     MWD_CUDA(launch_pdl(scan_final_kernel<SCAN_SUMS>, nb, SCAN_THREADS, 0, s, (const int32_t*)a.pair_count, rows,
                         (const int32_t*)a.scan_tmp, a.pair_count, nb, a.n_pairs, a.pair_cap, a.status,
                         (uint32_t)MWD_ST_PAIR_OVERFLOW, aligned16(a.pair_count, a.pair_count), (int32_t*)nullptr));
-    MWD_CUDA(launch_pdl(pairs_kernel<true>, blocks(rows, T), T, 0, s, a));
+    MWD_CUDA(launch_pdl(pairs_kernel<true>, grid, APPEND_THREADS, 0, s, b));
     return MWD_OK;
 }
 

@@ -34,7 +34,7 @@ struct BroadArgs {
     int64_t pair_cap;
     int32_t* tile_sums;          // per-scan-tile cell counts, zero on entry, added to by assign_kernel, read by
                                  // the cell scan (no reduce pass) and zeroed by place_kernel
-    int32_t walk_parts;          // append mode: threads per row (1, or 8: walls + own cell, 7 neighbours)
+    int32_t walk_parts;          // threads per row of the pair kernels: 1, or several (launch_broad sets it)
     // occupancy-compressed cell table (sparse = 1; needs tile_sums): a bit per cell of the dense
     // table, the cells' ranks among the occupied ones, and counts and starts per occupied cell, all
     // carved out of cell_count and cell_start (launch_broad sets these)
