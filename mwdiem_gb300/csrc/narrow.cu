@@ -450,11 +450,12 @@ __device__ __forceinline__ void epa_contact(f3 Va, f3 Vb, f3 Vc, int pa, int pb,
 //
 // One pair per warp, laid out for the length of an iteration's dependent chain, which sets the time of
 // a step with a few thousand contacts (its longest EPA runs 25 iterations): each lane keeps its
-// hull vertices and its faces of the append-only list (face f in lane f % 32, slot f / 32) in
-// registers, so a support query, the minimum search and the visibility test read no memory; the new
-// faces are computed in the lanes that will hold them.  Shared memory holds what is looked up by index:
-// the polytope's vertices and a copy of the faces.  The forces wait until the warp has up to 32 of them,
-// one per lane.
+// hull vertices and the distances and vertex numbers of its faces of the append-only list (face f in lane
+// f % 32, slot f / 32) in registers, so a support query and the minimum search read no memory; the new
+// faces are computed in the lanes that will hold them.  Shared memory holds the polytope's vertices and the
+// faces' normals (in registers too, 2M random pairs took 4% longer; with nothing of the faces in
+// registers 1% less, but short lists 2-4% longer).  The forces wait until the warp has up to 32 of them, one
+// per lane.
 //
 // Against groups of 8, 16 or 32 lanes with the polytope in shared memory, which it replaces: an iteration
 // alone on its scheduler 3,300 cycles (of about 560 instructions, mostly waiting for their fetch);
@@ -663,13 +664,11 @@ __device__ __forceinline__ void epa_warp(WarpEpaMem& m, const WarpHulls& h, f3 S
         m.pab[0] = (uint16_t)(a1 | (b1 << 8)); m.pab[1] = (uint16_t)(a2 | (b2 << 8));
         m.pab[2] = (uint16_t)(a3 | (b3 << 8)); m.pab[3] = (uint16_t)(a4 | (b4 << 8));
     }
-    // this lane's faces: normal, distance (NaN: no face), first vertex, vertex numbers
-    f3 fn[FACE_SLOTS], f0[FACE_SLOTS];
+    // this lane's faces: distance (NaN: no face), vertex numbers
     float fd[FACE_SLOTS];
     uint32_t ft[FACE_SLOTS];
 #pragma unroll
     for (int s = 0; s < FACE_SLOTS; ++s) {
-        fn[s] = f0[s] = mk3(0.f, 0.f, 0.f);
         fd[s] = nan;
         ft[s] = 0;
     }
@@ -681,9 +680,7 @@ __device__ __forceinline__ void epa_warp(WarpEpaMem& m, const WarpHulls& h, f3 S
         const uint32_t e = lane == 0 ? 0x020100u : lane == 1 ? 0x030201u : lane == 2 ? 0x030002u : 0x030100u;
         bool flip;
         const float4 p = face_plane(a, b, c, flip);
-        fn[0] = xyz(p);
         fd[0] = p.w;
-        f0[0] = a;
         ft[0] = (flip ? (e & 0xffu) | ((e >> 8) & 0xff00u) | ((e & 0xff00u) << 8) : e) | FACE_LIVE;
         m.fn[lane] = p;
         m.ft[lane] = ft[0];
@@ -726,12 +723,13 @@ __device__ __forceinline__ void epa_warp(WarpEpaMem& m, const WarpHulls& h, f3 S
             m.pab[nv] = (uint16_t)(sa | (sb << 8));
         }
         nv++;
+        __syncwarp();  // every lane has read the chosen face
         // faces that the new vertex sees are removed, collected in index order
         int ndel = 0;
 #pragma unroll
         for (int s = 0; s < FACE_SLOTS; ++s) {
             if (32 * s < nt) {
-                const bool dead = (ft[s] & FACE_LIVE) && dot(sp - f0[s], fn[s]) >= 0.f;
+                const bool dead = (ft[s] & FACE_LIVE) && dot(sp - xyz(m.pv[ft_v(ft[s], 0)]), xyz(m.fn[32 * s + lane])) >= 0.f;
                 const unsigned b = __ballot_sync(ALL, dead);
                 if (dead) {
                     m.del[ndel + __popc(b & lt)] = ft[s];
@@ -782,9 +780,7 @@ __device__ __forceinline__ void epa_warp(WarpEpaMem& m, const WarpHulls& h, f3 S
                 if (32 * s + lane < nt) {
                     const float4 p = m.fn[32 * s + lane];
                     ft[s] = m.ft[32 * s + lane];
-                    fn[s] = xyz(p);
                     fd[s] = p.w;
-                    f0[s] = xyz(m.pv[ft_v(ft[s], 0)]);
                 }
             }
             __syncwarp();
@@ -812,13 +808,7 @@ __device__ __forceinline__ void epa_warp(WarpEpaMem& m, const WarpHulls& h, f3 S
             for (int s = 0; s < FACE_SLOTS; ++s) {
                 if (s != s0 && s != s0 + 1) continue;
                 const bool here = (pos >> 5) == s;  // selects, so that the arrays stay in registers
-                fn[s].x = here ? p.x : fn[s].x;
-                fn[s].y = here ? p.y : fn[s].y;
-                fn[s].z = here ? p.z : fn[s].z;
                 fd[s] = here ? p.w : fd[s];
-                f0[s].x = here ? a.x : f0[s].x;
-                f0[s].y = here ? a.y : f0[s].y;
-                f0[s].z = here ? a.z : f0[s].z;
                 ft[s] = here ? t : ft[s];
             }
         }
