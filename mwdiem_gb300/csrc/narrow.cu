@@ -38,14 +38,12 @@ template <int LPP>
 struct Group {
     int lane;
     unsigned mask;
-    __device__ __forceinline__ void sync() const { __syncwarp(mask); }
     __device__ __forceinline__ unsigned ballot(bool p) const
     {
         unsigned b = __ballot_sync(mask, p);
         if (LPP < 32) b = (b & mask) >> (__ffs(mask) - 1);
         return b;
     }
-    __device__ __forceinline__ unsigned lt_mask() const { return (1u << lane) - 1u; }
 };
 
 // Order-preserving key of a float (-0 and +0 share the key of +0, as they compare equal): the
@@ -64,13 +62,12 @@ __device__ __forceinline__ unsigned long long* epa_queue(const NarrowArgs& a)
     return reinterpret_cast<unsigned long long*>(a.epa_count + 2);
 }
 
-// The next `amount` items of a queue for the calling group: its first lane takes them with one atomic.
-template <int LPP>
-__device__ __forceinline__ int64_t claim(const Group<LPP>& g, unsigned long long* next, int64_t amount)
+// The next `amount` items of a queue for the calling warp: its first lane takes them with one atomic.
+__device__ __forceinline__ int64_t claim(unsigned long long* next, int64_t amount)
 {
     unsigned long long base = 0;
-    if (g.lane == 0) base = atomicAdd(next, (unsigned long long)amount);
-    return (int64_t)__shfl_sync(g.mask, base, (int)(threadIdx.x & 31) - g.lane);
+    if ((threadIdx.x & 31) == 0) base = atomicAdd(next, (unsigned long long)amount);
+    return (int64_t)__shfl_sync(0xffffffffu, base, 0);
 }
 
 // work counted per pair when the caller asks for it: vertex dot products, EPA faces, support queries
@@ -1787,9 +1784,6 @@ __global__ void __launch_bounds__(BT, 640 / BT) epa_pass_kernel(const __grid_con
     EpaDone* done = reinterpret_cast<EpaDone*>(reinterpret_cast<WarpEpaMem*>(smem) + W) + 32 * warp;
     const float4* wv = reinterpret_cast<const float4*>(a.st.world_verts);
     const SimplexRec* recs = reinterpret_cast<const SimplexRec*>(a.epa_rec);
-    Group<32> g;
-    g.lane = lane;
-    g.mask = 0xffffffffu;
     const int cnt = *a.epa_count;
     const int m = (int64_t)cnt < a.epa_cap ? cnt : (int)a.epa_cap;
     // Persistent over a work queue (guided self-scheduling): every warp first takes a fixed share of
@@ -1813,7 +1807,7 @@ __global__ void __launch_bounds__(BT, 640 / BT) epa_pass_kernel(const __grid_con
             if (fixed >= m) break;
             int size = (m - fixed - seen) / (EPA_GUIDE * G);
             if (size < EPA_CLAIM) size = EPA_CLAIM;
-            const int64_t b = (int64_t)fixed + claim<32>(g, next, size);
+            const int64_t b = (int64_t)fixed + claim(next, size);
             if (b >= m) break;
             i = (int)b;
             step = 1;
@@ -1864,9 +1858,6 @@ int launch_epa_bt(const NarrowArgs& a, cudaStream_t s)
     MWD_CUDA(launch_pdl(epa_pass_kernel<BT>, (unsigned)(num_sms() * per_sm), BT, shm, s, a));
     return MWD_OK;
 }
-
-// threads per block of a block-size code of the lanes word (0: 128, 1: 64, 2: 256)
-inline int block_threads(int code) { return code == 1 ? 64 : code == 2 ? 256 : 128; }
 
 template <int LPP, int BT>
 int launch_gjk_bt(const NarrowArgs& a, cudaStream_t s)
