@@ -56,9 +56,9 @@ class host_prints_to_stderr:
 METRIC = "particle-steps/s"
 WINDOW_STEPS = 500  # the pour configuration runs 500 steps
 # DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) of one GJK-pass and one EPA-pass
-# launch of this step, from one capture of the eager first step: 5.185 MB + 0.169 MB (the writes stay
+# launch of this step, from one capture of the eager first step: 5.209 MB + 0.186 MB (the writes stay
 # in L2).  ncu cannot run inside this timing, so the figure is carried here.
-NARROW_DRAM_BYTES_PER_LAUNCH = 5.184512e6 + 0.169472e6
+NARROW_DRAM_BYTES_PER_LAUNCH = 5.209088e6 + 0.186112e6
 # broad phase 4 (assign, cell scan, place, append) + GJK pass + EPA pass + integrator rows + vertices
 KERNELS_PER_STEP = 8
 
