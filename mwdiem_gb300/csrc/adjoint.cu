@@ -154,11 +154,21 @@ __device__ __forceinline__ d3 rot_rev(d3 w, double s, const Rot& r, dq g)
 
 constexpr double kPi = 3.141592653589793;
 
-// a / b from y = 1 / b: the product corrected by its exact remainder (Markstein, IBM J. Res. Dev. 34, 1990)
+// 2^-400 <= |v| < 2^400, from the exponent bits (a comparison in FP64 would be an FP64 instruction)
+__device__ __forceinline__ bool mid_range(double v)
+{
+    return ((unsigned)__double2hiint(v) >> 20 & 0x7ffu) - 623u < 800u;
+}
+
+// a / b from y = 1 / b: the product corrected by its exact remainder (Markstein, IBM J. Res. Dev. 34, 1990).
+// The correction needs b and the quotient in mid range: an infinite or zero b or an infinite a would turn
+// into NaN (a frictionless law has C = 1 / mu + ... infinite and Gt = -2 Let / C = 0; et = 0 has Gt infinite
+// and the slip test caps it; an infinite inertia drops out of C).  Everything else is divided.
 __device__ __forceinline__ double quotient(double a, double b, double y)
 {
     const double q = a * y;
-    return fma(fma(-b, q, a), y, q);
+    if (mid_range(b) && mid_range(q)) return fma(fma(-b, q, a), y, q);
+    return a / b;
 }
 
 // ------------------------------------------------------------------ pair map

@@ -173,3 +173,47 @@ def test_fp64_forces_agree_with_fp32_narrow_phase():
     W = eng.n_walls
     rel = (f32[W:] - f64[W:]).norm(dim=1) / (f64[W:].norm(dim=1) + 1.0)
     assert float(rel.median()) < 1e-4 and float(rel.max()) < 1e-2, rel
+
+
+# (row, column) of the law, and the value: a frictionless law, et at its ends
+EXTREME_LAWS = {"mu": {(0, 3): 0.0, (1, 3): 0.0}, "mu_pairs": {(0, 3): 0.0}, "mu_wall": {(1, 3): 0.0},
+                "et_one": {(0, 2): 1.0, (1, 2): 1.0}, "et": {(0, 2): 0.0}, "inertia": {}}
+
+
+@pytest.mark.parametrize("which", sorted(EXTREME_LAWS))
+def test_extreme_laws_match_torch_restatement(which):
+    """mu = 0 (1 / mu and C infinite, Gt 0), et = 0 between particles (Gt infinite, capped by the slip; not at a
+    wall, where a slip along an axis has a zero component: 0 * infinity), an infinite inertia size of some rows
+    (their terms of C 0): the state and, where the restatement has one, the gradient on it."""
+    from mwdiem_gb300.diff import rollout
+    steps = 20
+    eng, x0 = make_engine(steps=steps, K=7)
+    W = eng.n_walls
+    law0 = eng.default_law()
+    for k, v in EXTREME_LAWS[which].items():
+        law0[k] = v
+    if which == "inertia":
+        eng.inertia[:W + 4, 3] = float("inf")
+    wx = torch.from_numpy(np.random.default_rng(1).normal(size=(eng.n, 32))).cuda() * 1e-2
+    X = x0.clone().requires_grad_(True)
+    com, xT = rollout(eng, X, law0, steps)
+    (com.sum() + (xT * wx).sum()).backward()
+    logs = logs_of(eng, steps)
+    Xr = x0.clone().requires_grad_(True)
+    com_r, xT_r = diff_ref.rollout(Xr, law0, logs, diff_ref.engine_consts(eng), steps)
+    (com_r.sum() + (xT_r * wx).sum()).backward()
+    assert sum(len(l) for l in logs) > 8 * steps and eng.status_word() & 0x380 == 0
+    assert diff_ref.check_finite(com, xT, com_r, xT_r)
+    assert (com - com_r).abs().max() <= 1e-11 * (1 + com_r.abs().max())
+    err = (xT - xT_r).abs().max(0).values / (1 + xT_r.abs().max(0).values)
+    assert err.max() <= 1e-9, err
+    gx, gxr = X.grad[W:, :30], Xr.grad[W:, :30]
+    if which == "et":  # 0 * log(0) in C's gradient: NaN in both
+        assert not diff_ref.check_finite(gxr)
+        return
+    assert diff_ref.check_finite(gx, gxr)
+    # 1e-8 of the column's largest entry, as above, and for columns that nearly cancel the rounding of some
+    # thousand float64 operations on terms of the largest entry's size (1e4 * 1.1e-16)
+    col = gxr.abs().max(0).values
+    err = (gx - gxr).abs().max(0).values
+    assert (err <= 1e-8 * col + 1e-12 * col.max()).all(), (err, col)
