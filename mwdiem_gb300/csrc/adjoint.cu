@@ -48,6 +48,16 @@ __device__ __forceinline__ d3 cross3(d3 a, d3 b)
 {
     return D3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
 }
+// the same, rounded product by product: terms that cancel give 0 (fused, the rounding of one product stays)
+__device__ __forceinline__ double dot3_rn(d3 a, d3 b)
+{
+    return __dadd_rn(__dadd_rn(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)), __dmul_rn(a.z, b.z));
+}
+__device__ __forceinline__ d3 cross3_rn(d3 a, d3 b)
+{
+    return D3(__dsub_rn(__dmul_rn(a.y, b.z), __dmul_rn(a.z, b.y)), __dsub_rn(__dmul_rn(a.z, b.x), __dmul_rn(a.x, b.z)),
+              __dsub_rn(__dmul_rn(a.x, b.y), __dmul_rn(a.y, b.x)));
+}
 __device__ __forceinline__ d3 had(d3 a, d3 b) { return D3(a.x * b.x, a.y * b.y, a.z * b.z); }
 __device__ __forceinline__ d3 zero3() { return D3(0.0, 0.0, 0.0); }
 
@@ -211,7 +221,7 @@ __device__ __forceinline__ void pair_fwd(const PairIn& p, PairTape& t, PairOut& 
     }
     t.e1 = t.V[1] - t.V[0];
     t.e2 = t.V[2] - t.V[1];
-    t.m = cross3(t.e1, t.e2);
+    t.m = cross3_rn(t.e1, t.e2);  // 0 for three points on a line: a face without a normal
     t.l = sqrt(dot3(t.m, t.m));
     t.ok = t.l > 0.0;
     if (!t.ok) return;
@@ -251,7 +261,7 @@ __device__ __forceinline__ void pair_fwd(const PairIn& p, PairTape& t, PairOut& 
     t.S = sqrt(quotient(p.mu * p.Kn, t.Xen, t.iXen));
     t.Gn = -2.0 * t.Len * t.S;
     t.Gt = quotient(-2.0 * t.Let, t.C, t.iC);
-    t.sgn = dot3(p.cB - p.cA, t.n0) < 0.0 ? -1.0 : 1.0;
+    t.sgn = dot3_rn(p.cB - p.cA, t.n0) < 0.0 ? -1.0 : 1.0;  // + where the centres lie across the normal
     t.n = t.n0 * t.sgn;
     t.rA = t.cpA - p.cA;
     t.rB = t.cpB - p.cB;

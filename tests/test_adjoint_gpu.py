@@ -217,3 +217,47 @@ def test_extreme_laws_match_torch_restatement(which):
     col = gxr.abs().max(0).values
     err = (gx - gxr).abs().max(0).values
     assert (err <= 1e-8 * col + 1e-12 * col.max()).all(), (err, col)
+
+
+def logged_contact(offset, corner, fa, fb, edge=0.0246):
+    """Force and status of one logged contact of two equal cubes, `offset` apart, the first centred at `corner`;
+    fa, fb: the signs of the three vertices of A and of B."""
+    import ctypes as C
+    import dataclasses
+
+    from mwdiem_gb300 import scene, shapes
+    from mwdiem_gb300._lib import check, lib
+    from mwdiem_gb300.diff import DiffEngine
+    body = scene.body_from_shape(shapes.cube(edge))
+    spec = dataclasses.replace(scene.packed_scene(n=2, seed=0), bodies=[body, body], velocities=np.zeros((2, 3)),
+                               centres=np.array([corner, np.add(corner, offset)]))
+    eng = DiffEngine(spec, 1, ckpt_every=1)
+    x0, W = eng.initial_state(), eng.n_walls
+    off = eng.sim.t["vert_off"].cpu().numpy()
+    signs = np.sign(eng.sim.t["body_verts"].cpu().numpy()[off[W]:off[W] + 8, :3]).astype(int).tolist()
+    eng.rec[0] = torch.tensor([W, W + 1] + [signs.index(list(s)) for s in fa + fb], dtype=torch.int32)
+    eng.step_count[0] = 1
+    eng.law.copy_(eng.default_law())
+    check(lib().mwd_diff_force(C.byref(eng.d), x0.data_ptr(), 0, None))
+    torch.cuda.synchronize()
+    return eng.F[W:, :3].cpu().numpy(), int(eng.status.item())
+
+
+@pytest.mark.parametrize("c", [0.015, 0.017, 0.0193, 0.02, 0.0211])
+def test_face_of_three_points_on_a_line_is_refused(c):
+    # cubes apart along their diagonal: the three differences of corners lie on that line, whatever their rounding
+    hi, lo = (1, 1, 1), (-1, -1, -1)
+    F, status = logged_contact((c, c, c), (0.1, 0.1, 0.1), [hi, lo, lo], [lo, hi, lo])
+    assert status & 128 and not F.any()
+
+
+@pytest.mark.parametrize("c", [0.011, 0.013, 0.0153, 0.017, 0.0191, 0.021])
+def test_normal_keeps_its_side_where_the_centres_lie_across_it(c):
+    # a face with the normal (1, -1, 0) / sqrt(2) and centres (c, c, 0) apart: their product is exactly 0
+    A = [(-1, -1, -1), (-1, -1, 1), (1, 1, 1)]
+    F, status = logged_contact((c, c, 0.0), (0.1, 0.1, 0.1), A, [(-1, 1, -1)] * 3)
+    # V1 - V0 along z, V2 - V1 along (1, 1, 0): n0 = (-1, 1, 0) / sqrt(2), depth n0 . V0 = -edge / sqrt(2);
+    # F = -Kn depth n0 on A
+    want = 1e5 * 0.0246 / np.sqrt(2.0) * np.array([-1.0, 1.0, 0.0]) / np.sqrt(2.0)
+    assert status == 0
+    assert np.abs(F - np.stack([want, -want])).max() <= 1e-6 * np.abs(want).max()
