@@ -363,10 +363,12 @@ __device__ __forceinline__ int pyset_warp_place(int k, int rank, unsigned h)
     return __shfl_sync(0xffffffffu, listed, rank < 0 ? 0 : rank);
 }
 
-// cells of up to 4 members are ordered by one thread, up to 18 by a warp of its block; larger cells go to a list
-// handled by one warp each with the table in shared memory
+// cells of up to 4 members are ordered by one thread, up to 18 by a warp of its block, up to 32 by one thread with
+// the table in local memory; larger cells go to a list handled by one warp per block with the table in shared memory
 constexpr int SMALL_CELL = 4;
 constexpr int WARP_CELL = 18;
+constexpr int LOCAL_CELL = 32;
+constexpr int LOCAL_TAB = 128;   // table size CPython reaches for <= 76 members
 constexpr int BIG_TAB = 512;     // table size CPython reaches for <= 306 members
 constexpr int BIG_CELL = 306;
 
@@ -582,6 +584,23 @@ __device__ __forceinline__ void order_small_cell(const BroadArgs& a, int g, int 
     }
 }
 
+// The same for a cell of 19 to 32 members: one thread replays the set inserts, its table in local memory, beside the
+// other threads' cells.  (One after another by the block's first warp, 2,000 rows in cells of 20 took the drop-in
+// broad phase 753 us instead of 143, 40,000 rows 1,864 instead of 221, 200,000 rows 2,546 instead of 312.)
+__device__ __noinline__ void order_local_cell(const int32_t* ids, int k, int base, int32_t* out)
+{
+    int m[LOCAL_CELL], o[LOCAL_CELL], tab[LOCAL_TAB], tmp[LOCAL_TAB];
+    unsigned char used[LOCAL_TAB], used2[LOCAL_TAB];
+    for (int j = 0; j < k; ++j) {
+        const int v = __ldcg(ids + j);
+        int i = j;
+        for (; i > 0 && m[i - 1] > v; --i) m[i] = m[i - 1];
+        m[i] = v;
+    }
+    pyset_order<LOCAL_TAB>(m, k, o, tab, used, tmp, used2, base);
+    for (int j = 0; j < k; ++j) out[j] = o[j];
+}
+
 // a cell of 5 to 18 members for a warp of its block: k members from sorted position s, cell g, base the
 // first row of their scene
 struct WarpCell {
@@ -701,6 +720,9 @@ __global__ void __launch_bounds__(PLACE_THREADS) place_kernel(BroadArgs a)
                         order_small_cell(a, g, s, k, base);
                     } else if (k <= WARP_CELL) {
                         s_mid[atomicAdd(&s_nm, 1)] = {g, s, k, base};
+                    } else if (k <= LOCAL_CELL) {
+                        order_local_cell(a.scatter_out + s, k, base, a.sorted + s);
+                        for (int j = 0; j < k && a.sorted_pos; ++j) place(a, s + j, a.sorted[s + j], g);
                     } else s_crowd[atomicAdd(&s_nc, 1)] = g;
                 }
             }

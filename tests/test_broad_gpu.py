@@ -151,3 +151,28 @@ def test_scan_tile_edges(n):
     wn, wc = np.array([[0.0, 0.6, 0.8]]), np.zeros((1, 3))
     wall = CCD.wall_pairs(com, wn, wc, 1, 1, n + 1, 14.4).cpu().numpy()
     assert np.array_equal(wall, oracle.wall_pairs(1, 1, n + 1, com, wn, wc, 14.4))
+
+
+@pytest.mark.parametrize("size", [19, 20, 32])
+def test_cells_past_the_warp_limit_are_ordered_side_by_side(size):
+    # 40,000 rows in cells of 18 members (a warp each) and of a few more: with the cells of a block one after
+    # another the call took 8 times as long, side by side 1.4 times
+    import torch
+
+    from mwdiem_gb300 import LIBRARY_Coarse_contact_detection as CCD
+
+    def fastest(members, n=40_000):
+        rng = np.random.default_rng(members)
+        cell = np.repeat(np.arange(n // members) * 97, members)
+        keys = torch.from_numpy(cell[rng.permutation(len(cell))].astype(np.int64)).cuda()
+        best = np.inf
+        for _ in range(12):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            CCD.linked_cell_pairs(keys, 0, len(cell), 11, 11, cap=members * len(cell))
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    assert fastest(size) < 3 * fastest(18)
