@@ -979,6 +979,18 @@ __global__ void __launch_bounds__(APPEND_THREADS) pairs_kernel(BroadArgs a)
         if (part <= 0) walk_walls(a, r, sc, scene, me, ws, 0, 1, sink);
         walk_cells(a, t, r, g, sc, me, part, sink);
     };
+    if (EMIT && !split) {
+        // the row's offset is the thread's own: written as they come (kept first, with a second walk past
+        // APPEND_KEEP of them, the drop-in call on 2M rows took 144 us here instead of 84)
+        int64_t out = live ? (int64_t)a.pair_count[t] : 0;
+        const int64_t cap = a.pair_cap;
+        int2* pairs = reinterpret_cast<int2*>(a.pairs);
+        walk([&](int A, int B) {
+            if (out < cap) pairs[out] = make_int2(A, B);
+            ++out;
+        });
+        return;
+    }
     int c = 0;
     walk([&](int A, int B) {
         if (EMIT && c < APPEND_KEEP) keep[c][threadIdx.x] = make_int2(A, B);
