@@ -505,10 +505,12 @@ __global__ void assign_kernel(BroadArgs a)
         return;
     }
     atomicAdd(a.cell_count + g, 1);
-    // one atomic per tile per warp (consecutive rows mostly share a tile)
-    const int tile = g / SCAN_TILE;
-    const unsigned peers = __match_any_sync(__activemask(), tile);
-    if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(a.tile_sums + tile, __popc(peers));
+    if (a.tile_sums) {
+        // one atomic per tile per warp (consecutive rows mostly share a tile)
+        const int tile = g / SCAN_TILE;
+        const unsigned peers = __match_any_sync(__activemask(), tile);
+        if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(a.tile_sums + tile, __popc(peers));
+    }
 }
 
 // sparse table: rows per occupied cell (by rank), with per-tile totals for the scan that follows
@@ -660,7 +662,7 @@ __global__ void __launch_bounds__(PLACE_THREADS) place_kernel(BroadArgs a)
     __shared__ WarpCell s_mid[PLACE_THREADS];
     __shared__ int s_nc, s_nm;
     if (threadIdx.x == 0) s_nc = s_nm = 0;
-    {  // read by the cell scan, which has finished: zero for the next broad phase
+    if (a.tile_sums) {  // read by the cell scan, which has finished: zero for the next broad phase
         int32_t* ts = a.sparse ? occ_tile_sums(a) : a.tile_sums;
         const int64_t nb = a.sparse ? (a.compact_len + SCAN_TILE - 1) / SCAN_TILE
                                     : (a.total_cells + SCAN_TILE - 1) / SCAN_TILE;
@@ -1234,8 +1236,8 @@ int launch_broad(const BroadArgs& a_in, cudaStream_t s)
         MWD_CUDA(cudaMemsetAsync(a.n_pairs, 0, sizeof(int64_t), s));
         return MWD_OK;
     }
-    if (!a.tile_sums) return MWD_ERR_INVALID;
     if (a.sparse) {
+        if (!a.tile_sums) return MWD_ERR_INVALID;
         const SparseLayout L = sparse_layout(rows, a.total_cells);
         a.n_words = (int32_t)L.n_words;
         a.words_pad = (int32_t)L.words_pad;
@@ -1259,6 +1261,15 @@ int launch_broad(const BroadArgs& a_in, cudaStream_t s)
                             (int64_t)a.compact_len, (const int32_t*)(a.tile_sums + nbw + 1), start, nbc,
                             (int64_t*)nullptr, (int64_t)INT64_MAX, (uint32_t*)nullptr, 0u, aligned16(cnt, start),
                             (int32_t*)nullptr));
+    } else if (!a.tile_sums) {
+        // rows in any order of cells: up to 32 atomics per warp on a few hundred tile counts cost more than a
+        // pass over the counts (the drop-in call, keys drawn at random: 400,000 rows 91 us in assign_kernel
+        // with them, 5.6 and a pass of 3.5 without; 2,000,000 rows 166, and 18 and 4.2).  The first half of
+        // scan_tmp stays zero for pairs_kernel.
+        const int64_t m = (a.total_cells > rows ? a.total_cells : rows) + 1;
+        const int rc = launch_scan(a.cell_count, a.total_cells, a.cell_start, a.scan_tmp + scan_tile_sums_offset(m),
+                                   nullptr, INT64_MAX, nullptr, 0, s);
+        if (rc) return rc;
     } else {
         // the tile totals were added up by assign_kernel: only the final pass of the scan remains (each
         // block adds up the totals of the tiles before it; turning them into prefixes in a separate

@@ -33,7 +33,8 @@ struct BroadArgs {
     int64_t total_cells;
     int64_t pair_cap;
     int32_t* tile_sums;          // per-scan-tile cell counts, zero on entry, added to by assign_kernel, read by
-                                 // the cell scan (no reduce pass) and zeroed by place_kernel
+                                 // the cell scan (no reduce pass) and zeroed by place_kernel; NULL (dense table
+                                 // only): the scan adds the counts up itself
     int32_t walk_parts;          // threads per row of the pair kernels: 1, or several (launch_broad sets it)
     // occupancy-compressed cell table (sparse = 1; needs tile_sums): a bit per cell of the dense
     // table, the cells' ranks among the occupied ones, and counts and starts per occupied cell, all

@@ -462,7 +462,8 @@ int mwd_linked_cell_hash(int32_t n_lo, int32_t n_hi, const int64_t* keys, int64_
     rc = launch_put_scene(reinterpret_cast<mwd_scene*>(b + o_scene), sc, s);
     if (rc) return rc;
     MWD_CUDA(cudaMemsetAsync(b + o_tmp, 0, o_count - o_tmp + count_ints * sizeof(int32_t), s));
-    int32_t* tile_sums = reinterpret_cast<int32_t*>(b + o_tmp) + scan_tile_sums_offset(m);
+    // the compressed table needs the per-tile counts; the dense one does without (rows in any order)
+    int32_t* tile_sums = sparse ? reinterpret_cast<int32_t*>(b + o_tmp) + scan_tile_sums_offset(m) : nullptr;
     BroadArgs a = {};
     a.row_lo = n_lo;
     a.row_hi = n_hi;
