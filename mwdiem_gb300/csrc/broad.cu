@@ -363,12 +363,20 @@ __device__ __forceinline__ int pyset_warp_place(int k, int rank, unsigned h)
     return __shfl_sync(0xffffffffu, listed, rank < 0 ? 0 : rank);
 }
 
-// cells of up to 4 members are ordered by one thread, up to 18 by a warp of its block, up to 32 by one thread with
-// the table in local memory; larger cells go to a list handled by one warp per block with the table in shared memory
+// cells of up to 4 members are ordered by one thread, up to 18 by a warp of its block (or by a thread where the block
+// has many), up to 32 by one thread with the table in local memory; larger cells go to a list handled by one warp per
+// block with the table in shared memory
 constexpr int SMALL_CELL = 4;
 constexpr int WARP_CELL = 18;
 constexpr int LOCAL_CELL = 32;
 constexpr int LOCAL_TAB = 128;   // table size CPython reaches for <= 76 members
+// Cells (those past WARP_CELL count four times) that the warps of a block take one after another; a block with more
+// gives each a thread.  A warp takes about 2 us per cell, a thread 20 to 25 for one and for 32 side by side.  Rows in
+// the order of their cells leave a block some ten of them; in random order the blocks that run last complete most
+// cells.  (Rows in random order, 20,000 in cells of 12 members: 38 us by warps alone, 21 with this line; packed beds,
+// 5,003 to 150,000 rows: 15 to 27 us with either, 25 to 56 by threads alone.  16 costs the beds up to 15 us, 48 costs
+// 5,000 random rows in cells of 12 members 7.)
+constexpr int MID_BY_WARP = 32;
 constexpr int BIG_TAB = 512;     // table size CPython reaches for <= 306 members
 constexpr int BIG_CELL = 306;
 
@@ -586,10 +594,15 @@ __device__ __forceinline__ void order_small_cell(const BroadArgs& a, int g, int 
     }
 }
 
-// The same for a cell of 19 to 32 members: one thread replays the set inserts, its table in local memory, beside the
-// other threads' cells.  (One after another by the block's first warp, 2,000 rows in cells of 20 took the drop-in
-// broad phase 753 us instead of 143, 40,000 rows 1,864 instead of 221, 200,000 rows 2,546 instead of 312.)
-__device__ __noinline__ void order_local_cell(const int32_t* ids, int k, int base, int32_t* out)
+// a cell of 5 to 32 members: k members from sorted position s, cell g, base the first row of their scene
+struct MidCell {
+    int g, s, k, base;
+};
+
+// Such a cell by one thread that replays the set inserts, its table in local memory, beside the other threads'
+// cells.  (Cells of 20 one after another by the block's first warp: the drop-in broad phase of 2,000 rows took 753 us
+// instead of 143, of 40,000 rows 1,864 instead of 221, of 200,000 rows 2,546 instead of 312.)
+__device__ __noinline__ void order_local(const int32_t* ids, int k, int base, int32_t* out)
 {
     int m[LOCAL_CELL], o[LOCAL_CELL], tab[LOCAL_TAB], tmp[LOCAL_TAB];
     unsigned char used[LOCAL_TAB], used2[LOCAL_TAB];
@@ -602,22 +615,22 @@ __device__ __noinline__ void order_local_cell(const int32_t* ids, int k, int bas
     pyset_order<LOCAL_TAB>(m, k, o, tab, used, tmp, used2, base);
     for (int j = 0; j < k; ++j) out[j] = o[j];
 }
+__device__ __forceinline__ void order_local_cell(const BroadArgs& a, const MidCell& c)
+{
+    order_local(a.scatter_out + c.s, c.k, c.base, a.sorted + c.s);
+    if (!a.sorted_pos) return;
+    for (int j = 0; j < c.k; ++j) place(a, c.s + j, a.sorted[c.s + j], c.g);
+}
 
-// a cell of 5 to 18 members for a warp of its block: k members from sorted position s, cell g, base the
-// first row of their scene
-struct WarpCell {
-    int g, s, k, base;
-};
-
-// the same for such cells, one after another by a full warp with one member per lane: list[i] for
+// Cells of 5 to 18 members, one after another by a full warp with one member per lane: list[i] for
 // i = first, first + step, ... < n.  The next cell's members are loaded while the present one is ordered.
-__device__ __forceinline__ void order_warp_cells(const BroadArgs& a, const WarpCell* list, int first, int step, int n)
+__device__ __forceinline__ void order_warp_cells(const BroadArgs& a, const MidCell* list, int first, int step, int n)
 {
     const int lane = threadIdx.x & 31;
     auto member = [&](int i) { return i < n && lane < list[i].k ? __ldcg(a.scatter_out + list[i].s + lane) : 0x7fffffff; };
     int next = member(first);
     for (int i = first; i < n; i += step) {
-        const WarpCell c = list[i];
+        const MidCell c = list[i];
         const int v = next;
         double4 p = make_double4(0.0, 0.0, 0.0, 0.0);
         if (lane < c.k && a.sorted_pos) p = reinterpret_cast<const double4*>(a.pos)[v];
@@ -642,8 +655,8 @@ __device__ __forceinline__ void order_warp_cells(const BroadArgs& a, const WarpC
 // themselves into scatter_out, and then add 1 << 16 to the same word with an acquire-release atomic:
 // each member's add releases its write, and the member whose add finds k - 1 earlier ones (acquiring
 // all of them) sets the count back to zero and orders the cell: in its own thread up to SMALL_CELL
-// members, by a warp of its block up to WARP_CELL, else by the block's first warp with the tables in
-// shared memory.  (On beds of 5,003 and 30,011 packed hulls, cells of up to 18 members, the pass takes 14
+// members, by a warp or a thread of its block up to LOCAL_CELL, else by the block's first warp with the
+// tables in shared memory.  (On beds of 5,003 and 30,011 packed hulls, cells of up to 18 members, the pass takes 14
 // and 16.5 us; with one thread ordering up to 32 members, its table in local memory, it took 24 and 29.)
 // (With PAIRS, of a two-member cell the first member to arrive leaves its id in the count word by an
 // atomic exchange and the second, finding it there, places both.)  Cells beyond BIG_CELL members are written in ascending ids, beyond
@@ -659,9 +672,9 @@ __global__ void __launch_bounds__(PLACE_THREADS) place_kernel(BroadArgs a)
     pdl_wait();
     pdl_launch_dependents();
     __shared__ int s_crowd[PLACE_THREADS];
-    __shared__ WarpCell s_mid[PLACE_THREADS];
-    __shared__ int s_nc, s_nm;
-    if (threadIdx.x == 0) s_nc = s_nm = 0;
+    __shared__ MidCell s_mid[PLACE_THREADS];  // at most one per thread: 5..18 members from the front, 19..32 from the end
+    __shared__ int s_nc, s_nm, s_nl;
+    if (threadIdx.x == 0) s_nc = s_nm = s_nl = 0;
     if (a.tile_sums) {  // read by the cell scan, which has finished: zero for the next broad phase
         int32_t* ts = a.sparse ? occ_tile_sums(a) : a.tile_sums;
         const int64_t nb = a.sparse ? (a.compact_len + SCAN_TILE - 1) / SCAN_TILE
@@ -723,15 +736,25 @@ __global__ void __launch_bounds__(PLACE_THREADS) place_kernel(BroadArgs a)
                     } else if (k <= WARP_CELL) {
                         s_mid[atomicAdd(&s_nm, 1)] = {g, s, k, base};
                     } else if (k <= LOCAL_CELL) {
-                        order_local_cell(a.scatter_out + s, k, base, a.sorted + s);
-                        for (int j = 0; j < k && a.sorted_pos; ++j) place(a, s + j, a.sorted[s + j], g);
+                        s_mid[PLACE_THREADS - 1 - atomicAdd(&s_nl, 1)] = {g, s, k, base};
                     } else s_crowd[atomicAdd(&s_nc, 1)] = g;
                 }
             }
         }
     }
     __syncthreads();
-    order_warp_cells(a, s_mid, threadIdx.x / 32, PLACE_THREADS / 32, s_nm);
+    {
+        const int nm = s_nm, nl = s_nl, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+        if (nm + 4 * nl > MID_BY_WARP) {
+            const int i = lane * (PLACE_THREADS / 32) + warp;  // one per thread, spread over the warps
+            if (i < nm + nl) order_local_cell(a, s_mid[i < nm ? i : PLACE_THREADS - 1 - (i - nm)]);
+        } else {
+            const int W = PLACE_THREADS / 32 - (nl > 0);  // the last warp's lanes take the larger ones
+            if (warp < W) order_warp_cells(a, s_mid, warp, W, nm);
+            else if (lane < nl) order_local_cell(a, s_mid[PLACE_THREADS - 1 - lane]);
+        }
+        __syncwarp();
+    }
     const int nc = s_nc;
     if (nc == 0 || threadIdx.x >= 32) return;
     // the block's crowded cells, one at a time by its first warp: members ranked by id in parallel,

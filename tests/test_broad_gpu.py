@@ -176,3 +176,18 @@ def test_cells_past_the_warp_limit_are_ordered_side_by_side(size):
         return best
 
     assert fastest(size) < 3 * fastest(18)
+
+
+@pytest.mark.parametrize("order", ["cells", "random"])
+@pytest.mark.parametrize("sizes", [(5,), (18,), (12, 25), (4, 19), (18, 32), (7, 9, 33, 2)])
+def test_cells_in_set_order_by_warps_and_by_threads(sizes, order):
+    # rows in the order of their cells (some ten cells of a block, by its warps) and at random (the last blocks
+    # complete most, by threads), cells past the warp's limit among them
+    from mwdiem_gb300 import LIBRARY_Coarse_contact_detection as CCD
+    cell = np.concatenate([np.full(k, 50 * i) for i, k in enumerate(sizes * (6000 // sum(sizes)))])
+    if order == "random":
+        cell = cell[np.random.default_rng(len(sizes)).permutation(len(cell))]
+    n = len(cell)
+    ref = oracle.linked_cell_hash(0, n, cell.astype(np.int64), 11, 11)
+    got = CCD.Linked_cell_hash(None, 11, 11, 0, n, [], cell.astype(np.int64))
+    assert len(got) == len(ref) and pairset(got) == pairset(ref)
