@@ -1311,14 +1311,17 @@ int launch_broad(const BroadArgs& a_in, cudaStream_t s)
         MWD_CUDA(launch_pdl(place_kernel<false>, blocks(rows, PLACE_THREADS), PLACE_THREADS, 0, s, a));
     // rows that have a cell are at most `rows`; threads past cell_start[total] exit
     BroadArgs b = a;
-    const bool split = rows * ORDERED_PARTS <= 4 * (int64_t)num_sms() * 2048;
+    // Several threads per row up to one wave of resident threads.  (Four waves, as the eight-way append once
+    // had it, the ordered list's two passes took the drop-in call on 100,000 rows 39 us instead of 16, a packed bed
+    // of 150,000 rows 79 instead of 39 and its append pass 27 instead of 18; at 30,011 rows 30 and 33, 11 and 17.)
+    const int64_t wave = (int64_t)num_sms() * 2048;
     if (a.append) {
-        b.walk_parts = split ? APPEND_PARTS : 1;
+        b.walk_parts = rows * APPEND_PARTS <= wave ? APPEND_PARTS : 1;
         MWD_CUDA(launch_pdl(pairs_append_kernel, blocks(rows * b.walk_parts, APPEND_THREADS), APPEND_THREADS, 0, s,
                             b));
         return MWD_OK;
     }
-    b.walk_parts = split ? ORDERED_PARTS : 1;
+    b.walk_parts = rows * ORDERED_PARTS <= wave ? ORDERED_PARTS : 1;
     const unsigned grid = blocks(rows * b.walk_parts, APPEND_THREADS);
     MWD_CUDA(launch_pdl(pairs_kernel<false>, grid, APPEND_THREADS, 0, s, b));
     const int nb = (int)((rows + SCAN_TILE - 1) / SCAN_TILE);

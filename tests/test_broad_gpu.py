@@ -191,3 +191,17 @@ def test_cells_in_set_order_by_warps_and_by_threads(sizes, order):
     ref = oracle.linked_cell_hash(0, n, cell.astype(np.int64), 11, 11)
     got = CCD.Linked_cell_hash(None, 11, 11, 0, n, [], cell.astype(np.int64))
     assert len(got) == len(ref) and pairset(got) == pairset(ref)
+
+
+@pytest.mark.parametrize("past", [0, 1])
+def test_ordered_list_on_both_sides_of_the_thread_split(past):
+    # eight threads per row up to one wave of resident threads, one beyond; some rows with more candidates than
+    # a thread keeps from its walk
+    from mwdiem_gb300 import LIBRARY_Coarse_contact_detection as CCD
+    from mwdiem_gb300._lib import lib
+    n = lib().mwd_num_sms() * 2048 // 8 + past
+    side = round((n / 3) ** (1 / 3))
+    keys = np.random.default_rng(n).integers(0, side ** 3, size=n).astype(np.int64)
+    ref = oracle.linked_cell_hash(0, n, keys, side, side)
+    got = CCD.Linked_cell_hash(None, side, side, 0, n, [], keys)
+    assert len(got) == len(ref) and pairset(got) == pairset(ref)
