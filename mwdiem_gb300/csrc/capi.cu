@@ -563,7 +563,8 @@ static int narrow_force(const mwd_state* st, const mwd_scene* scenes_dev, mwd_wo
     int rc = gjk_one ? MWD_OK : check_lanes(lanes & 0xff, &lp);
     if (rc) return rc;
     if (gjk_one) lp = 1;
-    const int elp = (lanes >> 8) & 0xff;
+    // what the two-pass narrow phase takes: its lanes and the passes' block-size codes
+    const int word = lp | (lanes & (0xff << 8 | 3 << MWD_LANES_GJK_BLOCK_SHIFT | 3 << MWD_LANES_EPA_BLOCK_SHIFT));
     NarrowArgs a = {};
     a.st = *st;
     a.scenes = scenes_dev;
@@ -605,11 +606,11 @@ static int narrow_force(const mwd_state* st, const mwd_scene* scenes_dev, mwd_wo
             d.force = st->force;
             d.torque = st->torque;
             a.det_out = d.out;
-            rc = launch_narrow_two_pass(a, lp | (elp << 8), reinterpret_cast<cudaStream_t>(stream));
+            rc = launch_narrow_two_pass(a, word, reinterpret_cast<cudaStream_t>(stream));
             if (rc) return rc;
             return launch_det_reduce(d, reinterpret_cast<cudaStream_t>(stream));
         }
-        return launch_narrow_two_pass(a, lp | (elp << 8), reinterpret_cast<cudaStream_t>(stream));
+        return launch_narrow_two_pass(a, word, reinterpret_cast<cudaStream_t>(stream));
     }
     if (work->deterministic || work->hist_keys) {
         set_error("deterministic accumulation and persistent history need the two-pass narrow phase (work->epa_rec)");

@@ -101,3 +101,18 @@ def test_cell_table_sizes():
     rows = (5_005 + 1 + 3) // 4 * 4
     assert (c.value, s.value) == (pad + rows, 2 * pad + rows + 1)
     assert c.value + s.value < 0.15 * (2 * 5_400_000 + 1)
+
+
+def test_block_size_codes_reach_the_narrow_phase():
+    # the two-pass narrow phase refuses block-size code 3 of either pass before any device call
+    import ctypes
+    from mwdiem_gb300 import _lib, autotune
+    buf = ctypes.create_string_buffer(4096)
+    st, w = _lib.State(), _lib.Work()
+    st.max_verts = 8
+    w.epa_rec = w.epa_count = ctypes.addressof(buf)
+    w.epa_cap = 1
+    for shift in (autotune.GJK_BLOCK_SHIFT, autotune.EPA_BLOCK_SHIFT):
+        rc = _lib.lib().mwd_narrow_force(ctypes.byref(st), ctypes.addressof(buf), ctypes.byref(w), 8 | 3 << shift, None)
+        assert rc == _lib.MWD_ERR_INVALID
+        assert b"block-size code" in _lib.lib().mwd_last_error()

@@ -40,6 +40,31 @@ def test_pairs_vs_oracle(two_pass, lanes):
     assert bits_equal(F, o["force"]) and bits_equal(T, o["torque"])
 
 
+@pytest.mark.parametrize("lanes", [16 | (32 << 8), 32] + [g | (32 << 8) | (b << 20) | (e << 22)
+                                                          for g, b, e in ((1, 1, 2), (4, 2, 1), (8, 1, 1), (8, 2, 2),
+                                                                          (16, 2, 0), (32, 0, 1))])
+def test_lane_and_block_sizes_vs_oracle(lanes):
+    # every lane count of the GJK pass beyond a warp per pair, and the block sizes of both passes
+    test_pairs_vs_oracle(True, lanes)
+
+
+@pytest.mark.parametrize("past", [0, 1])
+@pytest.mark.parametrize("lanes,warps", [(1 | (32 << 8), 28), (8 | (32 << 8), 24), (16 | (32 << 8), 24)])
+def test_lists_at_the_warp_count_vs_oracle(lanes, warps, past):
+    # a warp per pair up to the warps of the GJK pass's grid (28 per SM with one lane per pair, 24 with groups, at
+    # 128 threads per block), the lanes' own form one pair beyond
+    from mwdiem_gb300._lib import lib
+    from mwdiem_gb300.pairbench import PairScene
+    n = lib().mwd_num_sms() * warps + past
+    ps = PairScene(n, seed=5, pool=96, lanes=lanes)
+    ps.narrow()
+    torch.cuda.synchronize()
+    o = oracle.contact(ps.gather(np.arange(n)), ps.params, 2 * n, "f32")
+    assert np.array_equal(ps.w["collision"].cpu().numpy(), o["collision"])
+    assert bits_equal(ps.t["force"][:, :3].cpu().numpy(), o["force"])
+    assert bits_equal(ps.t["torque"][:, :3].cpu().numpy(), o["torque"])
+
+
 def test_pairs_large_properties():
     from mwdiem_gb300.pairbench import PairScene
     n = 1 << 20
