@@ -574,6 +574,12 @@ def parse_lanes(text):
     return w
 
 
+def pair_candidates():
+    """The lanes words pairs_rate times first: one per distinct kernel (the EPA bits of a word have no effect)."""
+    from mwdiem_gb300 import autotune
+    return autotune.DEFAULT_CANDIDATES
+
+
 def pairs_rate(n_pairs, lanes, reps=5, with_cpu=True, fixed=None):
     """GJK/EPA pairs/s of the device-step narrow phase on independent random pairs (hulls of 8-64
     vertices, radius U[0.8,1.2], centre distance U[0.5,2.2] (rA+rB)/2; inputs ~10 GB, far above L2)."""
@@ -585,42 +591,30 @@ def pairs_rate(n_pairs, lanes, reps=5, with_cpu=True, fixed=None):
     from mwdiem_gb300 import autotune
     ps = PairScene(n_pairs, seed=1, lanes=lanes)
     stream = torch.cuda.current_stream()
-    sweep = {}
-    cands = tuple(parse_lanes(t) for t in ("gjk8/epa8", "gjk8/epa16", "gjk4/epa16", "gjk4/epa16g", "gjk4/epa8g",
-                                           "gjk8/epa16g", "gjk1/epa16", "gjk1/epa16g", "gjk1/epa8g", "gjk1/epa32g"))
-    if fixed is not None:
-        cands = (parse_lanes(fixed),)
-    for cand in cands:
-        ps.lanes = cand
+
+    def timed(word, reps):
+        """Median ms of `reps` launches, one after another, after one untimed launch."""
+        ps.lanes = word
         ps.narrow()
-        torch.cuda.synchronize()
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record(stream)
-        for _ in range(reps):
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(reps + 1)]
+        ev[0].record(stream)
+        for e in ev[1:]:
             ps.narrow()
-        e1.record(stream)
+            e.record(stream)
         torch.cuda.synchronize()
-        sweep[autotune.describe(cand)] = e0.elapsed_time(e1) / reps
+        return sorted(x.elapsed_time(y) for x, y in zip(ev, ev[1:]))[reps // 2]
+
+    words = pair_candidates() if fixed is None else (parse_lanes(fixed),)
+    sweep = {w: timed(w, reps) for w in words}
     if fixed is None:
         # block sizes of the two passes at the fastest lane setting
         top = min(sweep, key=sweep.get)
-        top_word = [c for c in cands if autotune.describe(c) == top][0]
-        extra = tuple(c for c in autotune.block_candidates(top_word) if c not in cands)
-        cands = cands + extra
-        for cand in extra:
-            ps.lanes = cand
-            ps.narrow()
-            torch.cuda.synchronize()
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record(stream)
-            for _ in range(reps):
-                ps.narrow()
-            e1.record(stream)
-            torch.cuda.synchronize()
-            sweep[autotune.describe(cand)] = e0.elapsed_time(e1) / reps
+        sweep.update({w: timed(w, reps) for w in autotune.block_candidates(top) if w not in sweep})
     best = min(sweep, key=sweep.get)
-    ms = sweep[best]
-    ps.lanes = [c for c in cands if autotune.describe(c) == best][0]
+    # timed anew: the smallest of the sweep's figures is also the luckiest
+    ms = timed(best, 2 * reps + 1)
+    sweep = {autotune.describe(w): v for w, v in sweep.items()}
+    best = autotune.describe(best)
     ps.narrow(count_work=True)
     torch.cuda.synchronize()
     dots, faces, queries = (int(x) for x in ps.w["counters"].cpu().numpy())

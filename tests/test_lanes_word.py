@@ -37,3 +37,14 @@ def test_header_bit_positions():
     assert int(defs["MWD_LANES_GJK_BLOCK_SHIFT"]) == autotune.GJK_BLOCK_SHIFT
     assert int(defs["MWD_LANES_EPA_BLOCK_SHIFT"]) == autotune.EPA_BLOCK_SHIFT
     assert 1 << int(defs["MWD_LANES_EPA_IN_PLACE"]) == autotune.EPA_IN_PLACE
+
+
+def test_every_timed_setting_is_a_kernel_of_its_own():
+    # the EPA-lane and in-place bits have no effect: words that differ in them alone are one kernel, and the
+    # smallest of their times would be that of the luckiest run
+    import bench
+    from mwdiem_gb300 import autotune
+    for words in (bench.pair_candidates(), autotune.DEFAULT_CANDIDATES,
+                  *(autotune.block_candidates(w) for w in autotune.DEFAULT_CANDIDATES)):
+        kernels = [w & ~(0xff << 8 | autotune.EPA_IN_PLACE) for w in words]
+        assert len(set(kernels)) == len(kernels)
