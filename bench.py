@@ -9,8 +9,8 @@ every timed step; each step is timed with CUDA events on the stream it runs on a
 summed.  `e2e` is the same step through the public host-buffer API (state copied from pinned host
 memory to the device and back every step).  `roofline` covers the kernel that dominates the step.
 `--impl reference` times the reference's own CPU path (oracle/stepper.py: its kernels compiled
-for the host from their source when that build is available, else the oracle's restatement) on
-this machine's host cores, on the same scene.  Under torchrun every rank runs an independent
+for the host from their source) on this machine's host cores, on the same scene; without that
+build it prints an `unavailable` line.  Under torchrun every rank runs an independent
 replica (the scene does not shard; no collective on the data path).
 """
 from __future__ import annotations
@@ -976,10 +976,16 @@ def fd_check(steps=50):
 
 
 def reference_arm(args):
-    """The reference's CPU path on this host, same scene, same metric."""
+    """The reference's CPU path on this host, same scene, same metric; where its kernels are not built here the
+    arm is unavailable (the oracle's restatement of them is not the reference)."""
     spec = build_scene(SCENE["seed"])
     s, kind = ref_kind(spec, None)
-    cores = (os.cpu_count() or 1) if kind == "reference" else 1
+    if kind != "reference":
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's own kernels are not built on this host "
+                                                              "(no source checkout): only the oracle's restatement is"}),
+              flush=True)
+        return 0
+    cores = os.cpu_count() or 1
     with host_prints_to_stderr():
         for _ in range(max(0, args.warmup)):
             s.step()
