@@ -80,9 +80,10 @@ def describe(lanes):
 
 
 def tune_lanes(sim, candidates=DEFAULT_CANDIDATES, steps=5, blocks=True, flush=None):
-    """Time the scene with each lanes-per-pair setting of the GJK pass on a copy of its state, then the block sizes of the two passes at the fastest setting; set the fastest
-    on `sim`, and return {setting: ms per step}.  The state of `sim` is restored afterwards.  `flush`:
-    time every step with L2 overwritten first (time_steps)."""
+    """Time the scene with each lanes-per-pair setting of the GJK pass on a copy of its state, then the block
+    sizes of the two passes at the fastest setting; set the fastest on `sim`, and return {setting: ms per
+    step}.  The state of `sim` is restored afterwards.  `flush`: time every step with L2 overwritten first
+    (time_steps)."""
     saved = {k: v.clone() for k, v in sim.t.items()}
     res = {}
 

@@ -123,7 +123,8 @@ __global__ void __launch_bounds__(VR) verlet_ref_kernel(VerletRefArgs a, int row
         dq qq = dqld(a.q + 4 * P), qh = dqld(a.q12 + 4 * P);
         d3 dxa = dld(a.dxall + 3 * P);
 
-        // F / m, each quotient corrected by its exact remainder (extreme operands divide)
+        // F / m, each quotient corrected by its exact remainder (Markstein, IBM J. Res. Dev. 34, 1990; extreme
+        // operands divide)
         const double im = 1 / m;
         const bool plain = fabs(m) > 1e-150 && fabs(m) < 1e150;
         auto over_m = [&](double x) {

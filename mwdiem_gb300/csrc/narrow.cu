@@ -12,11 +12,11 @@
 //  * a GJK support query is a strided scan of the float4 hull vertices (staged in shared memory, or read
 //    in place from the L1-cached vertex table) by the group's lanes, then a group argmax on (value
 //    desc, index asc), which reproduces the reference's strict-'>' first-index tie break;
-//  * the simplex logic runs redundantly (identically) on every lane of the group, so control flow
-//    stays group-uniform;
-//  * EPA keeps an append-only face list of MWD_EPA_FACE_CAP faces, four in each lane's registers, like
-//    the reference's T[50]/n[50]/dist[50] (which overflow past 50 faces); when it is full the removed
-//    faces are dropped from it; the face scan, the visibility test, the horizon edge count (the
+//  * the simplex logic runs identically on every lane of the group, so control flow stays group-uniform;
+//    the three faces of a tetrahedron test have a lane each (tet_test_lanes), ballots combine them;
+//  * EPA keeps an append-only face list of MWD_EPA_FACE_CAP faces, four to a lane (distances and vertex
+//    numbers in its registers, normals in shared memory), like the reference's T[50]/n[50]/dist[50] (which
+//    overflow past 50 faces); when it is full the removed faces are dropped from it; the face scan, the visibility test, the horizon edge count (the
 //    reference's 50x50 delpair matrix, replaced by marks per vertex pair) and the new faces are computed
 //    lane-parallel, with ballots to keep the reference's face order;
 //  * force/torque are accumulated with float atomics (skipped for wall rows in table mode, whose
@@ -454,11 +454,11 @@ __device__ __forceinline__ void epa_contact(f3 Va, f3 Vb, f3 Vc, int pa, int pb,
 // registers 1% less, but short lists 2-4% longer).  The forces wait until the warp has up to 32 of them, one
 // per lane.
 //
-// Against groups of 8, 16 or 32 lanes with the polytope in shared memory, which it replaces: an iteration
-// alone on its scheduler 3,300 cycles (of about 560 instructions, mostly waiting for their fetch);
-// the pass on 3,001 random pairs 122 -> 50 us (8 lanes before), on four steps of 5,003 packed hulls
-// 122 -> 56 us each (8 lanes and the rerun of the overflowing pairs), on 30,011 packed hulls 83 -> 70 us
-// (32 lanes), on 2M random pairs 9.05 -> 7.6 ms (16 lanes), where it issues on 71% of the cycles.
+// An iteration alone on its scheduler takes about 1.2 us (some 560 instructions, partly waiting for their
+// fetch).  Against groups of 8, 16 or 32 lanes with the polytope in shared memory, which it replaces: the pass
+// on 3,001 random pairs 122 -> 50 us (8 lanes before), on four steps of 5,003 packed hulls 122 -> 56 us each
+// (8 lanes and the rerun of the overflowing pairs), on 30,011 packed hulls 83 -> 70 us (32 lanes), on 2M random
+// pairs 9.05 -> 7.6 ms (16 lanes), where it issues on 74% of the cycles.
 
 // the two hulls over a warp: lanes 0-15 hold A's vertices, lanes 16-31 B's, `per` consecutive ones each
 // (NaN past the end: such a product never wins)
@@ -1632,7 +1632,8 @@ __global__ void __launch_bounds__(BT, (LPP == 1 ? 896 : 768) / BT) gjk_pass_kern
     pdl_launch_dependents();
     const int64_t m = *a.n_pairs_dev;
     const int64_t n = m < a.pair_cap ? m : a.pair_cap;
-    // as many warps as pairs: a warp for each, whatever LPP
+    // as many warps as pairs: a warp for each, whatever LPP (both passes on 4,200 random pairs 59 us and on 5,000,
+    // past the line of one lane per pair, 87; groups of eight 64 and 67)
     if (LPP < 32 && n <= (int64_t)gridDim.x * (BT / 32)) gjk_stride<32, BT>(a, n);
     else gjk_stride<LPP, BT>(a, n);
 }

@@ -19,6 +19,17 @@ def reference(x, p):
     return (x > p) | ((xd * 1.00001 > pd) & (xd * 0.99999 < pd))
 
 
+def test_epa_stops_decides_almost_always():
+    # the undecided band is 4.8e-7 of x wide: p within a factor of two of x lies in it once in some millions
+    rng = np.random.default_rng(1)
+    x = rng.uniform(0.5, 1.0, 200_000).astype(f32)
+    got, decided = epa_stops(x, (x * rng.uniform(0.5, 2.0, x.size)).astype(f32))
+    assert decided.mean() > 0.999 and got.any() and not got.all()
+    # and a p within 2e-5 of x, as near the end of a search, 97 times in 100
+    near = (x.astype(np.float64) * (1 + rng.normal(scale=2e-5, size=x.size))).astype(f32)
+    assert epa_stops(x, near)[1].mean() > 0.97
+
+
 def test_epa_stops_is_the_references_double_test():
     rng = np.random.default_rng(0)
     x = (rng.uniform(0.5, 1.0, 400_000) * 2.0 ** rng.integers(-110, 120, 400_000)).astype(f32)
