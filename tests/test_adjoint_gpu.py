@@ -219,28 +219,41 @@ def test_extreme_laws_match_torch_restatement(which):
     assert (err <= 1e-8 * col + 1e-12 * col.max()).all(), (err, col)
 
 
-def logged_contact(offset, corner, fa, fb, edge=0.0246):
-    """Force and status of one logged contact of two equal cubes, `offset` apart, the first centred at `corner`;
-    fa, fb: the signs of the three vertices of A and of B."""
-    import ctypes as C
-    import dataclasses
+class LoggedContacts:
+    """Force and status of single logged contacts of two equal cubes, the first centred at `corner`, the second
+    `offset` away; fa, fb: the signs of the three vertices of A and of B."""
 
-    from mwdiem_gb300 import scene, shapes
-    from mwdiem_gb300._lib import check, lib
-    from mwdiem_gb300.diff import DiffEngine
-    body = scene.body_from_shape(shapes.cube(edge))
-    spec = dataclasses.replace(scene.packed_scene(n=2, seed=0), bodies=[body, body], velocities=np.zeros((2, 3)),
-                               centres=np.array([corner, np.add(corner, offset)]))
-    eng = DiffEngine(spec, 1, ckpt_every=1)
-    x0, W = eng.initial_state(), eng.n_walls
-    off = eng.sim.t["vert_off"].cpu().numpy()
-    signs = np.sign(eng.sim.t["body_verts"].cpu().numpy()[off[W]:off[W] + 8, :3]).astype(int).tolist()
-    eng.rec[0] = torch.tensor([W, W + 1] + [signs.index(list(s)) for s in fa + fb], dtype=torch.int32)
-    eng.step_count[0] = 1
-    eng.law.copy_(eng.default_law())
-    check(lib().mwd_diff_force(C.byref(eng.d), x0.data_ptr(), 0, None))
-    torch.cuda.synchronize()
-    return eng.F[W:, :3].cpu().numpy(), int(eng.status.item())
+    def __init__(self, offset, corner, edge):
+        import dataclasses
+
+        from mwdiem_gb300 import scene, shapes
+        from mwdiem_gb300.diff import DiffEngine
+        body = scene.body_from_shape(shapes.cube(edge))
+        spec = dataclasses.replace(scene.packed_scene(n=2, seed=0), bodies=[body, body], velocities=np.zeros((2, 3)),
+                                   centres=np.array([corner, np.add(corner, offset)]))
+        self.eng = DiffEngine(spec, 1, ckpt_every=1)
+        self.x0, W = self.eng.initial_state(), self.eng.n_walls
+        off = self.eng.sim.t["vert_off"].cpu().numpy()
+        self.verts = self.eng.sim.t["body_verts"].cpu().numpy()[off[W]:off[W] + 8, :3]
+        self.signs = np.sign(self.verts).astype(int).tolist()
+        self.eng.law.copy_(self.eng.default_law())
+        self.eng.step_count[0] = 1
+
+    def __call__(self, fa, fb):
+        import ctypes as C
+
+        from mwdiem_gb300._lib import check, lib
+        eng, W = self.eng, self.eng.n_walls
+        eng.rec[0] = torch.tensor([W, W + 1] + [self.signs.index(list(s)) for s in fa + fb], dtype=torch.int32)
+        for buf in (eng.F, eng.T, eng.status):
+            buf.zero_()
+        check(lib().mwd_diff_force(C.byref(eng.d), self.x0.data_ptr(), 0, None))
+        torch.cuda.synchronize()
+        return eng.F[W:, :3].cpu().numpy(), int(eng.status.item())
+
+
+def logged_contact(offset, corner, fa, fb, edge=0.0246):
+    return LoggedContacts(offset, corner, edge)(fa, fb)
 
 
 @pytest.mark.parametrize("c", [0.015, 0.017, 0.0193, 0.02, 0.0211])
@@ -261,3 +274,34 @@ def test_normal_keeps_its_side_where_the_centres_lie_across_it(c):
     want = 1e5 * 0.0246 / np.sqrt(2.0) * np.array([-1.0, 1.0, 0.0]) / np.sqrt(2.0)
     assert status == 0
     assert np.abs(F - np.stack([want, -want])).max() <= 1e-6 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("edge,corner,offset", [(1.0, (0.55, 1.1, 1.75), (1.161, 0.0, -0.1)),
+                                                (0.9, (0.55, 1.1, 1.75), (0.091, 0.55, 0.3)),
+                                                (0.7, (2.1, 2.3, 2.7), (0.403, -0.55, -0.1))])
+def test_face_decisions_on_the_brink_are_those_of_rounded_products(edge, corner, offset):
+    # faces whose area test comes down to rounding (the differences of corners lie on a line but for the last
+    # bits): refused or not as the products rounded one by one say, here in Python floats
+    contacts = LoggedContacts(offset, corner, edge)
+    cA, cB = np.array(corner), np.add(corner, offset)
+    rng = np.random.default_rng(2)
+
+    def decide(A, B):
+        V = [[float(cA[i]) + float(a[i]) - (float(cB[i]) + float(b[i])) for i in range(3)] for a, b in zip(A, B)]
+        e1, e2, u1 = [[V[j][i] - V[k][i] for i in range(3)] for j, k in ((1, 0), (2, 1), (2, 0))]
+        dot = lambda a, b: a[0] * b[0] + a[1] * b[1] + a[2] * b[2]
+        m = [e1[1] * e2[2] - e1[2] * e2[1], e1[2] * e2[0] - e1[0] * e2[2], e1[0] * e2[1] - e1[1] * e2[0]]
+        den = dot(e1, e1) * dot(u1, u1) - dot(e1, u1) * dot(e1, u1)
+        return any(m), den, dot(e1, e1) * dot(u1, u1)
+
+    near, refused = 0, 0
+    for _ in range(1500):
+        i, j = rng.integers(8, size=3), rng.integers(8, size=3)
+        normal, den, scale = decide(contacts.verts[i], contacts.verts[j])
+        if not normal or abs(den) > 1e-13 * scale:
+            continue
+        near += 1
+        _, status = contacts([contacts.signs[k] for k in i], [contacts.signs[k] for k in j])
+        assert bool(status & 128) == (not den > 0.0), (i, j, den)
+        refused += not den > 0.0
+    assert near > 30 and 20 < refused < near
