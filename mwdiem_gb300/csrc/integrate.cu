@@ -108,8 +108,8 @@ constexpr int VR = 32;
 __global__ void __launch_bounds__(VR) verlet_ref_kernel(VerletRefArgs a, int rows)
 {
     __shared__ double s_m[VR][9];  // turn about the old centre
-    __shared__ d3 s_c[VR], s_t[VR];  // old centre, and where it goes
-    __shared__ bool s_on[VR];
+    __shared__ d3 s_c[VR], s_t[VR];  // old centre, and where it goes (a reset row: its undone shift)
+    __shared__ int s_mode[VR];       // 0 inactive, 1 active, 2 active with a fly-away reset
     const int lane = threadIdx.x;
     const int p0 = blockIdx.x * rows;
     const int P = p0 + lane;
@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(VR) verlet_ref_kernel(VerletRefArgs a, int row
         const d3 c_old = c;
         c = c + dx;
         d3 to = c;
+        int mode = 1;
         const double* box = a.p.box;
         if (c.x > box[0] || c.x < box[1] || c.y > box[2] || c.y < box[3] || c.z > box[4] || c.z < box[5]) {
             // fly-away reset (gpu_Verlet.cu:338-352): stop the particle, undo the move
@@ -161,7 +162,8 @@ __global__ void __launch_bounds__(VR) verlet_ref_kernel(VerletRefArgs a, int row
             ombf = vel;
             om = vel;
             c = c + dx * (-1);
-            to = c_old;
+            to = dx;
+            mode = 2;
             if (a.n_reset) atomicAdd(a.n_reset, 1);
         }
         dst(a.v + 3 * P, vel);
@@ -188,8 +190,10 @@ __global__ void __launch_bounds__(VR) verlet_ref_kernel(VerletRefArgs a, int row
         M[7] = 2 * fma(qq.y, qq.z, qq.w * qq.x);
         s_c[lane] = c_old;
         s_t[lane] = to;
+        s_mode[lane] = mode;
+    } else {
+        s_mode[lane] = 0;
     }
-    s_on[lane] = on;
     __syncwarp();
     // vertices of the warp's rows: turned about the old centre, then moved (gpu_Verlet.cu:279-352)
     const int V = a.p.V;
@@ -203,7 +207,7 @@ __global__ void __launch_bounds__(VR) verlet_ref_kernel(VerletRefArgs a, int row
         for (int k = 0; k < U; ++k) {
             const int j = j0 + k * VR;
             r[k] = j < total ? j / V : 0;
-            if (j < total && s_on[r[k]]) v[k] = dld(vp + 3 * (size_t)j);
+            if (j < total && s_mode[r[k]]) v[k] = dld(vp + 3 * (size_t)j);
             else r[k] = -1;
         }
 #pragma unroll
@@ -214,7 +218,10 @@ __global__ void __launch_bounds__(VR) verlet_ref_kernel(VerletRefArgs a, int row
             const d3 d = v[k] - c;
             // the turned offset first: rounded at its own size, not at the coordinates'
             const d3 o = dm(ddot(dld(M), d), ddot(dld(M + 3), d), ddot(dld(M + 6), d));
-            dst(vp + 3 * (size_t)(j0 + k * VR), o + t);
+            // a reset undoes the vertices' shift as it does the centre's (:338-352), with the same rounding
+            d3 w = o + t;
+            if (s_mode[r[k]] == 2) w = ((o + c) + t) + t * (-1);
+            dst(vp + 3 * (size_t)(j0 + k * VR), w);
         }
     }
 }

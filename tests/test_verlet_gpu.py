@@ -63,3 +63,26 @@ def test_verlet_device_tensors():
     assert int(nres.item()) == r == 1
     for k in ("com", "verts", "q", "v"):
         assert np.abs(d[k].cpu().numpy() - a[k]).max() <= 1e-12 * np.abs(a[k]).max()
+
+
+@pytest.mark.parametrize("speed", [1e4, 1e9, 1e15, 1e200, np.inf])
+def test_fly_away_vertices_are_shifted_and_shifted_back(speed):
+    # the vertices of a reset row are moved by dx and back, as its centre is: the digits that dx costs them are
+    # gone (all for 1e15 and beyond), an infinite dx leaves NaN
+    N, V, W, dt = 40, 12, 3, 1e-3
+    st, box = make_verlet_state(N, V, seed=8, W=W)
+    st["v12"][W + 2:W + 12] = np.array([0.3, -1.0, 0.5]) * speed if np.isfinite(speed) else np.inf
+    a = {k: v.copy() for k, v in st.items()}
+    b = {k: v.copy() for k, v in st.items()}
+    with np.errstate(all="ignore"):
+        oracle.verlet_f64(a, dt, box, W, N - 2)
+    gpu_step(b, dt, box, W, N, V)
+    assert np.all(b["v"][W + 2:W + 12] == 0)
+    # two units in the last place of the farthest point of the way, beside the integrator's 1e-12
+    tol = 1e-12 * np.abs(st["verts"]).max() + (2 * np.spacing(speed * dt) if np.isfinite(speed) else 0.0)
+    for k in ("com", "verts"):
+        assert np.array_equal(np.isnan(a[k]), np.isnan(b[k])), k
+        ok = ~np.isnan(a[k])
+        assert np.abs(a[k][ok] - b[k][ok]).max() <= tol, k
+    rest = np.r_[W:W + 1, W + 12:N - 2]
+    assert np.abs(a["verts"][rest] - b["verts"][rest]).max() <= 1e-12 * np.abs(st["verts"]).max()
